@@ -32,6 +32,7 @@ struct swm_index {
     int device;
     uint32_t k;
     uint64_t n, n_seeds, n_words2, n_words3, ref_length;
+    void *arena;           // the arrays below of a built index in one allocation (null: one each)
     uint32_t *d_count;     // 4^k
     uint32_t *d_off;       // 4^k + 1 start offsets (mapper_mpe.c:250-255)
     uint32_t *d_pos;       // n_seeds (+8): positions, bucket order (.positions)

@@ -1,18 +1,16 @@
 // swm_index.cu -- GPU k-mer index build, index files, device scan.
 //
 // Index build (serial_index.c:157-445, rebuilt for the GPU):
-//   kb_encode   32 bases per thread -> lo/hi bit planes, N mask, 2-bit seed
-//               words (get_seed, serial_index.c:157-232)
+//   kb_encode   32 bases per thread -> lo/hi bit planes and N mask (get_seed,
+//               serial_index.c:157-232)
 //   kb_count    one thread per sampled position p = 4t: k-mer and N test
-//               from the packed words, atomic count (chromo_hash_index,
+//               from the planes, atomic count (chromo_hash_index,
 //               serial_index.c:253-269)
 //   scan        start offsets (store_positions, serial_index.c:337-340)
-//   kb_scatter  atomic slot per sampled position, key = position << 16 | lseed
-//               (serial_index.c:343-352 without the serial order)
-//   kb_sort_*   per-bucket sort of the keys: positions are unique, so sorting
-//               each bucket restores the ascending order the reference's
-//               serial scatter produces
-//   kb_split    the sorted keys into the resident index: positions (u32) and
+//   kb_radix    the sampled positions ordered by k-mer: a stable radix sort
+//               keeps each bucket in position order, the order the
+//               reference's serial scatter produces (serial_index.c:343-352);
+//               its last pass writes the resident index, positions (u32) and
 //               flank codes (u16), the layout of .positions / .pos_lseeds
 #include <errno.h>
 #include <fcntl.h>
@@ -154,16 +152,32 @@ __global__ void k_scan_down(const uint32_t *__restrict__ in, const uint32_t *d_n
     if (base >= n) return;
     const uint64_t i0 = base + (uint64_t)threadIdx.x * SCAN_V;
     uint32_t v[SCAN_V];
+    const bool whole = i0 + SCAN_V <= n && (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+    if (whole) {
+        const uint4 a = reinterpret_cast<const uint4 *>(in + i0)[0], b = reinterpret_cast<const uint4 *>(in + i0)[1];
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
 #pragma unroll
-    for (int j = 0; j < SCAN_V; j++) v[j] = (i0 + j < n) ? in[i0 + j] : 0u;
+        for (int j = 0; j < SCAN_V; j++) v[j] = (i0 + j < n) ? in[i0 + j] : 0u;
+    }
     uint32_t s = 0;
 #pragma unroll
     for (int j = 0; j < SCAN_V; j++) s += v[j];
     uint32_t ex = block_excl_scan(s, nullptr) + part[blockIdx.x];
 #pragma unroll
-    for (int j = 0; j < SCAN_V; j++) {
-        if (i0 + j < n) out[i0 + j] = ex;
-        ex += v[j];
+    for (int j = 0; j < SCAN_V; j++) { // each becomes its exclusive prefix
+        const uint32_t x = v[j];
+        v[j] = ex;
+        ex += x;
+    }
+    if (whole) {
+        reinterpret_cast<uint4 *>(out + i0)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<uint4 *>(out + i0)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < SCAN_V; j++)
+            if (i0 + j < n) out[i0 + j] = v[j];
     }
 }
 
@@ -180,208 +194,301 @@ int swm_exclusive_scan(const uint32_t *d_in, uint32_t *d_out, const uint32_t *d_
 
 // ------------------------------------------------------------ index build
 
-__global__ void kb_encode(const uint8_t *__restrict__ seq, uint64_t n, uint32_t *__restrict__ b2,
-                          uint32_t *__restrict__ b3, uint32_t *__restrict__ s2) {
-    __shared__ uint8_t tab[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        int u = i & 0xdf; // toupper for letters (serial_index.c:152)
-        tab[i] = u == 'A' ? 0 : u == 'C' ? 1 : u == 'G' ? 2 : u == 'T' ? 3 : 4;
+// Four sequence bytes -> 4 lo bits, 4 hi bits, 4 "not A/C/G/T" bits, base j at
+// bit j. Lower case counts as upper case (serial_index.c:152); the code
+// ((c >> 1) ^ (c >> 2)) & 3 maps A C G T to 0 1 2 3, anything else encodes as 0.
+// The letter of each byte's code (one byte permute) tells whether the byte was
+// one of the four; almost always all are.
+__device__ __forceinline__ void encode4(uint32_t w, uint32_t &lo, uint32_t &hi, uint32_t &nm) {
+    w &= 0xdfdfdfdfu;
+    uint32_t c = ((w >> 1) ^ (w >> 2)) & 0x03030303u;
+    const uint32_t y = (c | (c >> 4)) & 0x00ff00ffu; // codes as permute selectors, a nibble each
+    const uint32_t x = __byte_perm(0x54474341u, 0u, y | (y >> 8)) ^ w;
+    nm = 0;
+    if (x) {
+        uint32_t bad = x | (x >> 4);
+        bad |= bad >> 2;
+        bad = (bad | (bad >> 1)) & 0x01010101u; // bytes that differ
+        c &= ~(bad * 3u);
+        nm = (bad * 0x10204080u) >> 28;
     }
-    __syncthreads();
+    lo = ((c & 0x01010101u) * 0x10204080u) >> 28;
+    hi = (((c >> 1) & 0x01010101u) * 0x10204080u) >> 28;
+}
+
+__global__ void kb_encode(const uint8_t *__restrict__ seq, uint64_t n, uint32_t *__restrict__ b2,
+                          uint32_t *__restrict__ b3) {
     const uint64_t W = (n + 31) / 32;
     for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < W; w += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t p0 = w * 32;
         const uint32_t cnt = (n - p0 >= 32) ? 32u : (uint32_t)(n - p0);
-        uint8_t bytes[32];
+        uint32_t q[8];
         if (cnt == 32 && (((uintptr_t)(seq + p0)) & 15) == 0) {
             const uint4 *v = reinterpret_cast<const uint4 *>(seq + p0);
-            uint4 a = v[0], b = v[1];
-            memcpy(bytes, &a, 16);
-            memcpy(bytes + 16, &b, 16);
-        } else {
-            for (uint32_t j = 0; j < cnt; j++) bytes[j] = seq[p0 + j];
-        }
-        uint32_t lo = 0, hi = 0, nm = 0, sa = 0, sb = 0;
+            const uint4 a = __ldcs(v), b = __ldcs(v + 1);
+            q[0] = a.x; q[1] = a.y; q[2] = a.z; q[3] = a.w;
+            q[4] = b.x; q[5] = b.y; q[6] = b.z; q[7] = b.w;
+        } else { // unaligned sequence, or the last partial word
 #pragma unroll
-        for (uint32_t j = 0; j < 32; j++) {
-            if (j < cnt) {
-                uint32_t c = tab[bytes[j]];
-                if (c == 4) {
-                    nm |= 1u << j;
-                } else {
-                    lo |= (c & 1u) << j;
-                    hi |= (c >> 1) << j;
-                    if (j < 16) sa |= c << (2 * j);
-                    else sb |= c << (2 * (j - 16));
-                }
+            for (uint32_t j = 0; j < 8; j++) {
+                q[j] = 0;
+#pragma unroll
+                for (uint32_t i = 0; i < 4; i++)
+                    if (4 * j + i < cnt) q[j] |= (uint32_t)seq[p0 + 4 * j + i] << (8 * i);
             }
         }
-        b2[2 * w] = lo;
-        b2[2 * w + 1] = hi;
+        uint32_t lo = 0, hi = 0, nm = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; j++) {
+            uint32_t l, h, m;
+            encode4(q[j], l, h, m);
+            lo |= l << (4 * j);
+            hi |= h << (4 * j);
+            nm |= m << (4 * j);
+        }
+        if (cnt < 32) nm &= (1u << cnt) - 1u; // bases past the end are not N
+        reinterpret_cast<uint2 *>(b2)[w] = make_uint2(lo, hi);
         b3[w] = nm;
-        s2[2 * w] = sa;
-        s2[2 * w + 1] = sb;
     }
 }
 
-// k-mer at sampled position i (get_seed_from_enc_bits, serial_index.c:280-331)
-__device__ __forceinline__ bool sample_at(const uint32_t *__restrict__ b2, const uint32_t *__restrict__ b3,
-                                          const uint32_t *__restrict__ s2, uint64_t i, uint32_t k, uint32_t *seed,
-                                          uint32_t *lseed) {
-    const uint32_t smask = (k >= 16) ? 0xffffffffu : ((1u << (2 * k)) - 1);
-    const uint32_t nmask = (1u << k) - 1;
-    uint32_t nf = swm_fsr(b3[i / 32], b3[i / 32 + 1], (uint32_t)(i % 32)) & nmask;
-    if (nf) return false;
-    *seed = swm_fsr(s2[i / 16], s2[i / 16 + 1], (uint32_t)(i % 16) * 2) & smask;
-    const uint32_t res = SWM_SEED_STEP - 1, rmask = (1u << res) - 1;
-    uint64_t sp = (i >= res) ? i - res : 0;
-    uint32_t fl = swm_fsr(b2[(sp / 32) * 2], b2[(sp / 32 + 1) * 2], sp % 32) & rmask;
-    uint32_t fh = swm_fsr(b2[(sp / 32) * 2 + 1], b2[(sp / 32 + 1) * 2 + 1], sp % 32) & rmask;
-    sp = i + k;
-    uint32_t bl = swm_fsr(b2[(sp / 32) * 2], b2[(sp / 32 + 1) * 2], sp % 32) & rmask;
-    uint32_t bh = swm_fsr(b2[(sp / 32) * 2 + 1], b2[(sp / 32 + 1) * 2 + 1], sp % 32) & rmask;
-    fl |= bl << res;
-    fh |= bh << res;
-    *lseed = (fl | (fh << (res * 2))) & 0xffffu;
+// spread the low 16 bits of x to the even bit positions
+__device__ __forceinline__ uint32_t spread16(uint32_t x) {
+    x &= 0x0000ffffu;
+    x = (x | (x << 8)) & 0x00ff00ffu;
+    x = (x | (x << 4)) & 0x0f0f0f0fu;
+    x = (x | (x << 2)) & 0x33333333u;
+    x = (x | (x << 1)) & 0x55555555u;
+    return x;
+}
+
+// k-mer at sampled position i (get_seed_from_enc_bits, serial_index.c:280-331);
+// false when it holds an N. With FLANK also its flank code: 3 bases before
+// (bases 0 .. 2 when i is 0) and 3 after, lo bits then hi bits. One 32-base
+// window from i - 3 holds both (k <= 14).
+template <bool FLANK>
+__device__ __forceinline__ bool seed_at(const uint2 *__restrict__ b2p, const uint32_t *__restrict__ b3, uint64_t i,
+                                        uint32_t k, uint32_t *seed, uint32_t *flank) {
+    const uint32_t res = SWM_SEED_STEP - 1, rmask = (1u << res) - 1, mask = (1u << k) - 1;
+    const uint64_t w = i / 32;
+    const uint32_t sh = (uint32_t)(i % 32);
+    if (swm_fsr(b3[w], b3[w + 1], sh) & mask) return false;
+    const uint32_t f = i >= res ? res : 0u; // bases of the window before the k-mer
+    const uint64_t q = (i - f) / 32;
+    const uint32_t qs = (uint32_t)((i - f) % 32);
+    const uint2 a = b2p[q], b = b2p[q + 1];
+    const uint32_t lo = swm_fsr(a.x, b.x, qs), hi = swm_fsr(a.y, b.y, qs);
+    *seed = spread16((lo >> f) & mask) | (spread16((hi >> f) & mask) << 1);
+    if (FLANK)
+        *flank = (lo & rmask) | ((lo >> (f + k)) & rmask) << res | (hi & rmask) << (2 * res) |
+                 ((hi >> (f + k)) & rmask) << (3 * res);
     return true;
 }
 
-__global__ void kb_count(const uint32_t *__restrict__ b2, const uint32_t *__restrict__ b3,
-                         const uint32_t *__restrict__ s2, uint64_t T, uint32_t k, uint32_t *__restrict__ count) {
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < T; t += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t sd, ls;
-        if (sample_at(b2, b3, s2, t * SWM_SEED_STEP, k, &sd, &ls)) atomicAdd(&count[sd], 1u);
-    }
-}
+// ------------------------------------------------ ordering the positions
+//
+// The reference's scatter visits positions in ascending order, so a bucket's
+// entries ascend. A stable least-significant-digit radix sort of the samples
+// by k-mer gives that order with streaming passes only: 6.2 ms for 1 Gbp (250 M
+// samples, k = 12) where an atomic scatter to 8-byte slots and a sort of every
+// bucket took 35 ms (each entry's random write moved a whole DRAM burst, one
+// atomic per bucket on three counters serialised the bucket lists, and the
+// sorts read and wrote the buckets once more).
+//
+// An entry travels as one 64-bit key: flank code (12 bits), position / 4 (30)
+// and the digits of the k-mer still to be sorted by (at most 21 bits: the first
+// pass makes the key from the planes and sorts by the lowest digit right
+// away). Every pass cuts its input into one contiguous chunk per resident
+// block: the chunks' digit counts (kb_count for the first pass, kb_hist for
+// the others), scanned digit by digit, give each chunk the place of its first
+// key of every digit, and a block then moves its chunk tile by tile; no block
+// waits for another. A middle pass over 1 Gbp takes 1.33 ms and its counts 0.26;
+// one kernel whose tiles look back at the counts of the tiles before them took
+// 1.64. The ALU pipe (65% busy: ranking, 32 keys a warp) and the latency of a
+// tile's phases bound a pass, DRAM is at 3.1 TB/s; 4 blocks of 256 threads an
+// SM (64 registers) were faster than 3 (80): 1.33 against 1.37 ms.
+#define RADIX_BINS 256
+#define RADIX_THREADS 256 // one thread per digit
+#define RADIX_ITEMS 16
+#define RADIX_TILE (RADIX_THREADS * RADIX_ITEMS)
+#define RADIX_WARPS (RADIX_THREADS / 32)
+#define RADIX_BLOCKS_PER_SM 4
+#define RADIX_MAX_PASSES 4
+#define RADIX_LS_BITS 12
+#define RADIX_SEED_SHIFT 42 // flank code, then 30 bits of position / 4
 
-__global__ void kb_scatter(const uint32_t *__restrict__ b2, const uint32_t *__restrict__ b3,
-                           const uint32_t *__restrict__ s2, uint64_t T, uint32_t k, uint32_t *__restrict__ cursor,
-                           unsigned long long *__restrict__ keys) {
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < T; t += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t sd, ls;
-        const uint64_t i = t * SWM_SEED_STEP;
-        if (sample_at(b2, b3, s2, i, k, &sd, &ls)) {
-            uint32_t slot = atomicAdd(&cursor[sd], 1u);
-            keys[slot] = ((unsigned long long)i << 16) | ls;
-        }
-    }
-}
-
-#define SORT_SMALL 32
-#define SORT_MED 2048
-
-__global__ void kb_classify(const uint32_t *__restrict__ count, uint64_t nb, uint32_t *__restrict__ lists,
-                            uint32_t *__restrict__ nlist, uint64_t list_cap) {
-    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t c = count[b];
-        if (c <= 1) continue;
-        int cls = c <= SORT_SMALL ? 0 : c <= SORT_MED ? 1 : 2;
-        uint32_t at = atomicAdd(&nlist[cls], 1u);
-        if (at < list_cap) lists[(uint64_t)cls * list_cap + at] = (uint32_t)b;
-    }
-}
-
-__device__ __forceinline__ unsigned long long shfl_u64(unsigned long long v, int lane_mask) {
-    uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
-    lo = __shfl_xor_sync(0xffffffffu, lo, lane_mask);
-    hi = __shfl_xor_sync(0xffffffffu, hi, lane_mask);
-    return ((unsigned long long)hi << 32) | lo;
-}
-
-// one warp per bucket with <= 32 keys: bitonic sort across lanes
-__global__ void kb_sort_small(const uint32_t *__restrict__ list, const uint32_t *__restrict__ nlist,
-                              const uint32_t *__restrict__ off, const uint32_t *__restrict__ count,
-                              unsigned long long *__restrict__ keys) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    const uint32_t total = *nlist;
-    for (uint64_t wi = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; wi < total; wi += nwarps) {
-        const uint32_t b = list[wi];
-        const uint32_t o = off[b], c = count[b];
-        unsigned long long v = lane < c ? keys[o + lane] : ~0ull;
-#pragma unroll
-        for (int size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                unsigned long long w = shfl_u64(v, stride);
-                bool up = ((lane & size) == 0);
-                bool lower = ((lane & stride) == 0);
-                bool take_min = (lower == up);
-                v = take_min ? (w < v ? w : v) : (w > v ? w : v);
-            }
-        }
-        if (lane < c) keys[o + lane] = v;
-    }
-}
-
-// one block per bucket with <= SORT_MED keys: bitonic sort in shared memory
-__global__ void kb_sort_med(const uint32_t *__restrict__ list, const uint32_t *__restrict__ nlist,
-                            const uint32_t *__restrict__ off, const uint32_t *__restrict__ count,
-                            unsigned long long *__restrict__ keys) {
-    __shared__ unsigned long long sm[SORT_MED];
-    const uint32_t total = *nlist;
-    for (uint32_t bi = blockIdx.x; bi < total; bi += gridDim.x) {
-        const uint32_t b = list[bi];
-        const uint32_t o = off[b], c = count[b];
-        uint32_t n2 = 1;
-        while (n2 < c) n2 <<= 1;
-        for (uint32_t i = threadIdx.x; i < n2; i += blockDim.x) sm[i] = i < c ? keys[o + i] : ~0ull;
-        __syncthreads();
-        for (uint32_t size = 2; size <= n2; size <<= 1) {
-            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                for (uint32_t i = threadIdx.x; i < n2 / 2; i += blockDim.x) {
-                    uint32_t lo = 2 * i - (i & (stride - 1));
-                    uint32_t hi = lo + stride;
-                    bool up = ((lo & size) == 0);
-                    unsigned long long a = sm[lo], d = sm[hi];
-                    if ((a > d) == up) {
-                        sm[lo] = d;
-                        sm[hi] = a;
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) keys[o + i] = sm[i];
-        __syncthreads();
-    }
-}
-
-// one block per large bucket: bitonic sort in a padded global scratch region
-__global__ void kb_sort_large(const uint32_t *__restrict__ list, const uint32_t *__restrict__ off,
-                              const uint32_t *__restrict__ count, const uint64_t *__restrict__ scratch_off,
-                              unsigned long long *__restrict__ scratch, unsigned long long *__restrict__ keys) {
-    const uint32_t b = list[blockIdx.x];
-    const uint32_t o = off[b], c = count[b];
-    unsigned long long *sm = scratch + scratch_off[blockIdx.x];
-    uint32_t n2 = 1;
-    while (n2 < c) n2 <<= 1;
-    for (uint32_t i = threadIdx.x; i < n2; i += blockDim.x) sm[i] = i < c ? keys[o + i] : ~0ull;
+// Bucket counts of every sample of [0, T), and the lowest digit's count per
+// chunk of `chunk` samples (one per block) in hist[digit * gridDim.x + block].
+__global__ void __launch_bounds__(512) kb_count(const uint2 *__restrict__ b2p, const uint32_t *__restrict__ b3,
+                                                uint64_t T, uint64_t chunk, uint32_t k, uint32_t bits,
+                                                uint32_t *__restrict__ count, uint32_t *__restrict__ hist) {
+    __shared__ uint32_t h[RADIX_BINS];
+    if (threadIdx.x < RADIX_BINS) h[threadIdx.x] = 0;
     __syncthreads();
-    for (uint32_t size = 2; size <= n2; size <<= 1) {
-        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t i = threadIdx.x; i < n2 / 2; i += blockDim.x) {
-                uint32_t lo = 2 * i - (i & (stride - 1));
-                uint32_t hi = lo + stride;
-                bool up = ((lo & size) == 0);
-                unsigned long long a = sm[lo], d = sm[hi];
-                if ((a > d) == up) {
-                    sm[lo] = d;
-                    sm[hi] = a;
-                }
-            }
-            __syncthreads();
+    const uint64_t t0 = blockIdx.x * chunk, t1 = t0 + chunk < T ? t0 + chunk : T;
+    for (uint64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
+        uint32_t sd;
+        if (seed_at<false>(b2p, b3, t * SWM_SEED_STEP, k, &sd, nullptr)) {
+            atomicAdd(&count[sd], 1u);
+            atomicAdd(&h[sd & ((1u << bits) - 1)], 1u);
         }
     }
-    for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) keys[o + i] = sm[i];
+    __syncthreads();
+    if (threadIdx.x < RADIX_BINS) hist[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
 }
 
-__global__ void kb_split(const unsigned long long *__restrict__ keys, uint64_t S, uint32_t *__restrict__ pos,
-                         uint16_t *__restrict__ lseed) {
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < S; j += (uint64_t)gridDim.x * blockDim.x) {
-        unsigned long long v = keys[j];
-        if (pos) pos[j] = (uint32_t)(v >> 16);
-        if (lseed) lseed[j] = (uint16_t)(v & 0xffffu);
+// The same counts of one digit of *n keys, cut into gridDim.x chunks.
+__device__ __forceinline__ uint64_t radix_chunk(uint64_t n, uint32_t chunks) {
+    const uint64_t tiles = (n + RADIX_TILE - 1) / RADIX_TILE;
+    return (tiles + chunks - 1) / chunks * RADIX_TILE;
+}
+__global__ void __launch_bounds__(512) kb_hist(const unsigned long long *__restrict__ in,
+                                               const uint32_t *__restrict__ n, uint32_t shift, uint32_t bits,
+                                               uint32_t *__restrict__ hist) {
+    __shared__ uint32_t h[RADIX_BINS];
+    if (threadIdx.x < RADIX_BINS) h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint64_t total = *n, chunk = radix_chunk(total, gridDim.x);
+    const uint64_t t0 = blockIdx.x * chunk, t1 = t0 + chunk < total ? t0 + chunk : total;
+    const uint32_t dmask = (1u << bits) - 1;
+    // chunks start at whole tiles: two keys per load
+    for (uint64_t t = t0 + 2 * threadIdx.x; t < t1; t += 2 * blockDim.x) {
+        const ulonglong2 v = __ldcs(reinterpret_cast<const ulonglong2 *>(in + t));
+        atomicAdd(&h[(uint32_t)(v.x >> (RADIX_SEED_SHIFT + shift)) & dmask], 1u);
+        if (t + 1 < t1) atomicAdd(&h[(uint32_t)(v.y >> (RADIX_SEED_SHIFT + shift)) & dmask], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x < RADIX_BINS) hist[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
+}
+
+struct RadixSmem {
+    union {
+        unsigned long long key[RADIX_TILE];        // the tile in digit order
+        uint32_t cnt[RADIX_WARPS][RADIX_BINS];     // before that: counts per warp and digit
+    };
+    uint32_t base[RADIX_BINS]; // first output index of the digit minus its first place in the tile
+};
+
+// One pass: the block's chunk in tiles. FIRST: the keys come from the planes
+// (sample t of T at position 4 t; samples with an N are left out); otherwise
+// from in, *n of them. LAST: the entries go to pos / ls instead of out. first:
+// the scanned counts (see kb_count). A tile's keys are ranked by digit within
+// their warp (one ballot per digit bit; match instructions took 40% longer, and
+// masks made with shared-memory atomics moved the limit from the ALU to the
+// shared-memory pipe) and written through shared memory, so that each digit's
+// keys go out as one run of consecutive addresses. In shared memory a key of
+// the first pass holds its place in the tile and its digit where the position
+// goes, so that the digit can be read back.
+template <bool FIRST, bool LAST>
+__global__ void __launch_bounds__(RADIX_THREADS, RADIX_BLOCKS_PER_SM)
+    kb_radix(const uint2 *__restrict__ b2p, const uint32_t *__restrict__ b3, uint64_t T, uint64_t chunk_first, uint32_t k,
+             const unsigned long long *__restrict__ in, const uint32_t *__restrict__ n, uint32_t shift, uint32_t bits,
+             const uint32_t *__restrict__ first, unsigned long long *__restrict__ out, uint32_t *__restrict__ pos,
+             uint16_t *__restrict__ ls) {
+    __shared__ RadixSmem S;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t total = FIRST ? T : (uint64_t)*n;
+    const uint64_t chunk = FIRST ? chunk_first : radix_chunk(total, gridDim.x);
+    const uint64_t t0 = blockIdx.x * chunk, t1 = t0 + chunk < total ? t0 + chunk : total;
+    const uint32_t dmask = (1u << bits) - 1;
+    const uint32_t dsh = RADIX_SEED_SHIFT - 32 + shift; // of the digit in a key's high word
+    uint32_t lt;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    uint32_t next = first[tid * gridDim.x + blockIdx.x]; // output index of the chunk's next key of digit tid
+    uint32_t *cnt = S.cnt[warp];
+    for (uint64_t base = t0; base < t1; base += RADIX_TILE) {
+        // ---- the tile's keys: warp w holds its 512 in rows of 32
+        const uint32_t left = t1 - base < RADIX_TILE ? (uint32_t)(t1 - base) : RADIX_TILE;
+        const uint32_t w0 = warp * (32 * RADIX_ITEMS) + lane;
+        unsigned long long key[RADIX_ITEMS];
+        uint32_t at[RADIX_ITEMS]; // digit (RADIX_BINS: no key) | place << 16
+#pragma unroll
+        for (int j = 0; j < RADIX_ITEMS; j++) {
+            const uint32_t i = w0 + 32 * j;
+            at[j] = RADIX_BINS;
+            key[j] = 0;
+            if (i < left) {
+                if (FIRST) {
+                    uint32_t sd, fl;
+                    if (seed_at<true>(b2p, b3, (base + i) * SWM_SEED_STEP, k, &sd, &fl)) {
+                        at[j] = sd & dmask;
+                        key[j] = (unsigned long long)(sd >> bits) << RADIX_SEED_SHIFT | i << RADIX_LS_BITS | fl;
+                    }
+                } else {
+                    key[j] = __ldcs(in + base + i);
+                    at[j] = ((uint32_t)(key[j] >> 32) >> dsh) & dmask;
+                }
+            }
+        }
+#pragma unroll
+        for (int w = 0; w < RADIX_WARPS; w++) S.cnt[w][tid] = 0;
+        __syncthreads();
+        // ---- rank of each key among its warp's keys of the same digit
+#pragma unroll
+        for (int j = 0; j < RADIX_ITEMS; j++) {
+            const uint32_t d = at[j];
+            const bool have = d < RADIX_BINS;
+            uint32_t mm = __ballot_sync(0xffffffffu, have); // lanes with the same digit
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const bool on = (d & (1u << q)) != 0;
+                const uint32_t b = __ballot_sync(0xffffffffu, on);
+                mm &= on ? b : ~b;
+            }
+            const uint32_t below = mm & lt;
+            uint32_t c = 0;
+            if (have) c = cnt[d];
+            at[j] = d | (c + __popc(below)) << 16;
+            __syncwarp();
+            if (have && !below) cnt[d] = c + __popc(mm);
+            __syncwarp();
+        }
+        __syncthreads();
+        // ---- thread d owns digit d: the warps' counts become places in the tile
+        uint32_t mine = 0;
+#pragma unroll
+        for (int w = 0; w < RADIX_WARPS; w++) {
+            const uint32_t c = S.cnt[w][tid];
+            S.cnt[w][tid] = mine;
+            mine += c;
+        }
+        uint32_t tile_n;
+        const uint32_t loc = block_excl_scan(mine, &tile_n);
+        S.base[tid] = next - loc;
+        next += mine;
+#pragma unroll
+        for (int w = 0; w < RADIX_WARPS; w++) S.cnt[w][tid] += loc;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < RADIX_ITEMS; j++) {
+            const uint32_t d = at[j] & 0xffffu;
+            if (d < RADIX_BINS) at[j] += cnt[d] << 16;
+        }
+        __syncthreads(); // the counts are read: the keys take their place
+#pragma unroll
+        for (int j = 0; j < RADIX_ITEMS; j++) {
+            const uint32_t d = at[j] & 0xffffu;
+            if (d < RADIX_BINS) S.key[at[j] >> 16] = FIRST ? key[j] | (unsigned long long)d << 32 : key[j];
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t i = tid; i < tile_n; i += RADIX_THREADS) {
+            const unsigned long long v = S.key[i];
+            const uint32_t hi = (uint32_t)(v >> 32);
+            const uint32_t o = S.base[FIRST ? hi & (RADIX_BINS - 1) : (hi >> dsh) & dmask] + i;
+            const uint32_t t = FIRST ? (uint32_t)base + ((uint32_t)v >> RADIX_LS_BITS)
+                                     : (uint32_t)(v >> RADIX_LS_BITS) & 0x3fffffffu;
+            if (LAST) {
+                pos[o] = t * SWM_SEED_STEP;
+                ls[o] = (uint16_t)(v & ((1u << RADIX_LS_BITS) - 1));
+            } else if (FIRST) {
+                const unsigned long long ends = (1ull << RADIX_LS_BITS) - 1 | ~0ull << RADIX_SEED_SHIFT;
+                out[o] = (v & ends) | (unsigned long long)t << RADIX_LS_BITS;
+            } else {
+                out[o] = v;
+            }
+        }
+        __syncthreads(); // the next tile's counts overwrite the keys
     }
 }
 
@@ -474,7 +581,6 @@ __global__ void __launch_bounds__(CTAB_WARPS * 32) kb_ctab(const uint32_t *__res
 }
 
 // ----------------------------------------------------------- host helpers
-// ----------------------------------------------------------- host helpers
 
 static int sm_count(int device) {
     int n = 0;
@@ -494,12 +600,16 @@ static void index_release(swm_index *ix) {
     if (ix->chain_ev) cudaEventDestroy(ix->chain_ev);
     cudaFree(ix->d_ctab_off);
     cudaFree(ix->d_ctab_pos);
-    cudaFree(ix->d_count);
-    cudaFree(ix->d_off);
-    cudaFree(ix->d_pos);
-    cudaFree(ix->d_ls);
-    cudaFree(ix->d_b2);
-    cudaFree(ix->d_b3);
+    if (ix->arena) { // a built index: its arrays are parts of one allocation
+        cudaFree(ix->arena);
+    } else {
+        cudaFree(ix->d_count);
+        cudaFree(ix->d_off);
+        cudaFree(ix->d_pos);
+        cudaFree(ix->d_ls);
+        cudaFree(ix->d_b2);
+        cudaFree(ix->d_b3);
+    }
     free(ix);
 }
 
@@ -514,6 +624,16 @@ static int dalloc(T **p, uint64_t count) {
     }
     return SWM_OK;
 }
+
+// Sizes of the parts of one device allocation, each part 256-byte aligned.
+struct Parts {
+    uint64_t bytes = 0;
+    uint64_t add(uint64_t b) {
+        const uint64_t at = bytes;
+        bytes += (b + 255) / 256 * 256;
+        return at;
+    }
+};
 
 static int build_on_device(const uint8_t *d_seq, uint64_t n, uint32_t k, int device, swm_index **out) {
     if (k < 1 || k > 14 || n >= 0xffffffffull) {
@@ -532,127 +652,101 @@ static int build_on_device(const uint8_t *d_seq, uint64_t n, uint32_t k, int dev
     ix->n_words3 = W;
     ix->ref_length = ix->n_words2 * 4 * 16;
     cudaStream_t st = 0;
-    uint32_t *d_s2 = nullptr, *d_cursor = nullptr, *d_tmp = nullptr, *d_lists = nullptr, *d_nlist = nullptr;
-    unsigned long long *d_keys = nullptr; // position << 16 | lseed: sorting these sorts positions in a bucket
-    auto cleanup = [&]() {
-        cudaFree(d_keys);
-        d_keys = nullptr;
-        cudaFree(d_s2);
-        cudaFree(d_cursor);
-        cudaFree(d_tmp);
-        cudaFree(d_lists);
-        cudaFree(d_nlist);
-    };
-#define TRYC(x)                  \
-    do {                         \
-        int rc_ = (x);           \
-        if (rc_ != SWM_OK) {     \
-            cleanup();           \
-            index_release(ix);   \
-            return rc_;          \
-        }                        \
-    } while (0)
+    uint8_t *d_tmp = nullptr;
 #define CUC(x)                                                                                   \
     do {                                                                                         \
         cudaError_t e_ = (x);                                                                    \
         if (e_ != cudaSuccess) {                                                                 \
             swm_set_error("%s:%d %s: %s", __FILE__, __LINE__, #x, cudaGetErrorString(e_));       \
-            cleanup();                                                                           \
+            cudaFree(d_tmp);                                                                     \
             index_release(ix);                                                                   \
             return SWM_ERR_CUDA;                                                                 \
         }                                                                                        \
     } while (0)
-    TRYC(dalloc(&ix->d_b2, ix->n_words2 + SWM_PAD_WORDS));
-    TRYC(dalloc(&ix->d_b3, ix->n_words3 + SWM_PAD_WORDS));
-    TRYC(dalloc(&d_s2, 2 * W + SWM_PAD_WORDS));
-    TRYC(dalloc(&ix->d_count, nb));
-    TRYC(dalloc(&ix->d_off, nb + 1));
-    TRYC(dalloc(&d_cursor, nb + 1));
-    TRYC(dalloc(&d_tmp, swm_scan_tmp_words(nb)));
+    // One allocation for the index and one for the scratch: an allocation and
+    // its release cost 80 us and more (measured), which for a small genome is
+    // most of a build. There are at most T = one per four bases entries, so
+    // their arrays are sized before the count is known.
+    const uint64_t T = (n >= k) ? (n - k) / SWM_SEED_STEP + 1 : 0;
+    const uint64_t tiles = (T + RADIX_TILE - 1) / RADIX_TILE;
+    const uint64_t resident = (uint64_t)sm_count(device) * RADIX_BLOCKS_PER_SM;
+    const unsigned chunks = (unsigned)(tiles < resident ? tiles : resident);
+    const uint64_t chunk = chunks ? (tiles + chunks - 1) / chunks * RADIX_TILE : 0;
+    const uint32_t passes = (2 * k + 7) / 8;
+    uint32_t digit_at[RADIX_MAX_PASSES], digit_bits[RADIX_MAX_PASSES]; // as even as 2k bits allow
+    for (uint32_t q = 0, at = 0; q < passes; q++) {
+        digit_at[q] = at;
+        digit_bits[q] = (2 * k - at + passes - q - 1) / (passes - q);
+        at += digit_bits[q];
+    }
+    Parts ip, tp;
+    const uint64_t o_b2 = ip.add((ix->n_words2 + SWM_PAD_WORDS) * 4), o_b3 = ip.add((ix->n_words3 + SWM_PAD_WORDS) * 4);
+    const uint64_t o_count = ip.add(nb * 4), o_off = ip.add((nb + 1) * 4);
+    const uint64_t o_pos = ip.add((T + 8) * 4), o_ls = ip.add((T + 8) * 2);
+    const uint64_t nhist = (uint64_t)RADIX_BINS * chunks;
+    const uint64_t o_scan = tp.add(swm_scan_tmp_words(nb > nhist ? nb : nhist) * 4);
+    const uint64_t o_hist = tp.add(nhist * 4), o_first = tp.add((nhist + 1) * 4);
+    // keys between the passes, two buffers in turn
+    const uint64_t o_a = tp.add(passes > 1 ? T * 8 + 16 : 0), o_b = tp.add(passes > 2 ? T * 8 + 16 : 0);
+    if (cudaMalloc(&ix->arena, ip.bytes) != cudaSuccess || cudaMalloc(&d_tmp, tp.bytes) != cudaSuccess) {
+        cudaGetLastError();
+        swm_set_error("cudaMalloc(index %llu + scratch %llu bytes) failed", (unsigned long long)ip.bytes,
+                      (unsigned long long)tp.bytes);
+        index_release(ix);
+        return SWM_ERR_OOM;
+    }
+    uint8_t *base = (uint8_t *)ix->arena;
+    ix->d_b2 = (uint32_t *)(base + o_b2);
+    ix->d_b3 = (uint32_t *)(base + o_b3);
+    ix->d_count = (uint32_t *)(base + o_count);
+    ix->d_off = (uint32_t *)(base + o_off);
+    ix->d_pos = (uint32_t *)(base + o_pos);
+    ix->d_ls = (uint16_t *)(base + o_ls);
+    uint32_t *d_scan = (uint32_t *)(d_tmp + o_scan), *d_hist = (uint32_t *)(d_tmp + o_hist);
+    uint32_t *d_first = (uint32_t *)(d_tmp + o_first);
+    unsigned long long *d_key[2] = {(unsigned long long *)(d_tmp + o_a), (unsigned long long *)(d_tmp + o_b)};
+    auto scan = [&](const uint32_t *in, uint32_t *o, uint64_t count) {
+        return swm_exclusive_scan(in, o, nullptr, count, count, d_scan, nullptr, st) == SWM_OK;
+    };
+#define SCAN(in, o, count)             \
+    do {                               \
+        if (!scan(in, o, count)) {     \
+            cudaFree(d_tmp);           \
+            index_release(ix);         \
+            return SWM_ERR_CUDA;       \
+        }                              \
+    } while (0)
     CUC(cudaMemsetAsync(ix->d_b2 + ix->n_words2, 0, SWM_PAD_WORDS * 4, st));
     CUC(cudaMemsetAsync(ix->d_b3 + ix->n_words3, 0, SWM_PAD_WORDS * 4, st));
-    CUC(cudaMemsetAsync(d_s2 + 2 * W, 0, SWM_PAD_WORDS * 4, st));
     CUC(cudaMemsetAsync(ix->d_count, 0, nb * 4, st));
-    if (W) kb_encode<<<grid_for(W, 256, device, 16), 256, 0, st>>>(d_seq, n, ix->d_b2, ix->d_b3, d_s2);
-    const uint64_t T = (n >= k) ? (n - k) / SWM_SEED_STEP + 1 : 0;
-    if (T) kb_count<<<grid_for(T, 256, device, 16), 256, 0, st>>>(ix->d_b2, ix->d_b3, d_s2, T, k, ix->d_count);
+    const uint2 *b2p = (const uint2 *)ix->d_b2;
+    if (W) kb_encode<<<grid_for(W, 256, device, 16), 256, 0, st>>>(d_seq, n, ix->d_b2, ix->d_b3);
+    if (T) kb_count<<<chunks, 512, 0, st>>>(b2p, ix->d_b3, T, chunk, k, digit_bits[0], ix->d_count, d_hist);
     CUC(cudaGetLastError());
-    TRYC(swm_exclusive_scan(ix->d_count, ix->d_off, nullptr, nb, nb, d_tmp, nullptr, st));
-    uint32_t S32 = 0;
-    CUC(cudaMemcpyAsync(&S32, ix->d_off + nb, 4, cudaMemcpyDeviceToHost, st));
-    CUC(cudaStreamSynchronize(st));
-    const uint64_t S = S32;
-    ix->n_seeds = S;
-    TRYC(dalloc(&d_keys, S + 8));
-    if (S) {
-        CUC(cudaMemcpyAsync(d_cursor, ix->d_off, nb * 4, cudaMemcpyDeviceToDevice, st));
-        kb_scatter<<<grid_for(T, 256, device, 16), 256, 0, st>>>(ix->d_b2, ix->d_b3, d_s2, T, k, d_cursor, d_keys);
-        // per-bucket sort, classified by bucket size
-        const uint64_t list_cap = nb;
-        TRYC(dalloc(&d_lists, 3 * list_cap));
-        TRYC(dalloc(&d_nlist, 4));
-        CUC(cudaMemsetAsync(d_nlist, 0, 16, st));
-        kb_classify<<<grid_for(nb, 256, device, 16), 256, 0, st>>>(ix->d_count, nb, d_lists, d_nlist, list_cap);
-        kb_sort_small<<<sm_count(device) * 8, 256, 0, st>>>(d_lists, d_nlist, ix->d_off, ix->d_count, d_keys);
-        kb_sort_med<<<sm_count(device) * 4, 256, 0, st>>>(d_lists + list_cap, d_nlist + 1, ix->d_off, ix->d_count,
-                                                          d_keys);
-        CUC(cudaGetLastError());
-        uint32_t nl[3];
-        CUC(cudaMemcpyAsync(nl, d_nlist, 12, cudaMemcpyDeviceToHost, st));
-        CUC(cudaStreamSynchronize(st));
-        if (nl[2]) {
-            std::vector<uint32_t> big(nl[2]);
-            CUC(cudaMemcpy(big.data(), d_lists + 2 * list_cap, nl[2] * 4ull, cudaMemcpyDeviceToHost));
-            std::vector<uint32_t> cnt(nl[2]);
-            for (uint32_t i = 0; i < nl[2]; i++) CUC(cudaMemcpy(&cnt[i], ix->d_count + big[i], 4, cudaMemcpyDeviceToHost));
-            // process in groups whose padded scratch fits a bounded buffer
-            const uint64_t scratch_cap = 1ull << 27; // keys (1 GiB)
-            uint64_t i0 = 0;
-            while (i0 < nl[2]) {
-                std::vector<uint64_t> soff;
-                uint64_t tot = 0, i1 = i0;
-                while (i1 < nl[2]) {
-                    uint64_t n2 = 1;
-                    while (n2 < cnt[i1]) n2 <<= 1;
-                    if (tot && tot + n2 > scratch_cap) break;
-                    soff.push_back(tot);
-                    tot += n2;
-                    i1++;
-                }
-                unsigned long long *d_scr = nullptr;
-                uint64_t *d_soff = nullptr;
-                TRYC(dalloc(&d_scr, tot));
-                if (dalloc(&d_soff, soff.size()) != SWM_OK) {
-                    cudaFree(d_scr);
-                    cleanup();
-                    index_release(ix);
-                    return SWM_ERR_OOM;
-                }
-                cudaMemcpy(d_soff, soff.data(), soff.size() * 8, cudaMemcpyHostToDevice);
-                kb_sort_large<<<(unsigned)(i1 - i0), 1024, 0, st>>>(d_lists + 2 * list_cap + i0, ix->d_off,
-                                                                   ix->d_count, d_soff, d_scr, d_keys);
-                cudaError_t e = cudaStreamSynchronize(st);
-                cudaFree(d_scr);
-                cudaFree(d_soff);
-                CUC(e);
-                i0 = i1;
-            }
-        }
+    SCAN(ix->d_count, ix->d_off, nb);
+    const uint32_t *d_n = ix->d_off + nb; // entries
+    for (uint32_t q = 0; T && q < passes; q++) {
+        const bool first = q == 0, last = q + 1 == passes;
+        const uint32_t shift = first ? 0 : digit_at[q] - digit_bits[0];
+        if (!first) kb_hist<<<chunks, 512, 0, st>>>(d_key[(q + 1) & 1], d_n, shift, digit_bits[q], d_hist);
+        SCAN(d_hist, d_first, nhist);
+        auto f = first ? (last ? kb_radix<true, true> : kb_radix<true, false>)
+                       : (last ? kb_radix<false, true> : kb_radix<false, false>);
+        f<<<chunks, RADIX_THREADS, 0, st>>>(b2p, ix->d_b3, T, chunk, k, d_key[(q + 1) & 1], d_n, shift, digit_bits[q],
+                                            d_first, d_key[q & 1], ix->d_pos, ix->d_ls);
         CUC(cudaGetLastError());
     }
-    // the mapper reads the two halves separately: flank codes for every
-    // fetched entry, positions only for the entries the flank filter keeps
-    TRYC(dalloc(&ix->d_pos, S + 8));
-    TRYC(dalloc(&ix->d_ls, S + 8));
+    uint32_t S = 0;
+    CUC(cudaMemcpyAsync(&S, d_n, 4, cudaMemcpyDeviceToHost, st));
+    CUC(cudaStreamSynchronize(st));
+    ix->n_seeds = S;
     CUC(cudaMemsetAsync(ix->d_pos + S, 0, 8 * 4, st));
     CUC(cudaMemsetAsync(ix->d_ls + S, 0, 8 * 2, st));
-    if (S) kb_split<<<grid_for(S, 256, device, 16), 256, 0, st>>>(d_keys, S, ix->d_pos, ix->d_ls);
-    CUC(cudaGetLastError());
     CUC(cudaStreamSynchronize(st));
-    cleanup();
+    cudaFree(d_tmp);
     *out = ix;
     return SWM_OK;
-#undef TRYC
+#undef SCAN
 #undef CUC
 }
 

@@ -74,3 +74,33 @@ def test_gpu_index_save_open_roundtrip(cuda_lib, tmp_path):
         assert np.array_equal(a[key], b[key]), key
     assert ix2.info().n == 300001
     assert ix2.info().ref_length == ix.info().ref_length
+
+
+# the radix sort of the build: every number of passes (k), sample counts around
+# a tile (4,096) and past one tile per resident block, keys left out (N) and a
+# single digit (poly-A)
+@pytest.mark.parametrize("n,k", [(4 * 4095 + 11, 12), (4 * 4096 + 11, 12), (4 * 4096 + 12, 12), (50_021, 1),
+                                 (50_022, 4), (50_023, 5), (50_001, 9), (70_003, 11), (70_001, 14),
+                                 (11_000_017, 12)])
+def test_gpu_index_radix_tiles(cuda_lib, n, k):
+    g = genome(n, 6)
+    g[n // 3:n // 3 + 40] = ord("N")
+    g[n // 2:n // 2 + min(n // 4, 300_000)] = ord("A")
+    _same_as_oracle(cuda_lib, g, k=k)
+
+
+def test_gpu_index_unaligned_device_sequence(cuda_lib):
+    """Bases in device memory at an odd address give the same index."""
+    torch = pytest.importorskip("torch")
+    g = genome(100_003, 8)
+    g[500:600] = ord("n")
+    d = torch.empty(g.size + 16, dtype=torch.uint8, device="cuda")
+    for shift in (0, 1, 7):
+        d[shift:shift + g.size] = torch.from_numpy(g).cuda()
+        torch.cuda.synchronize()
+        got = cuda_lib.Index.build_device(d.data_ptr() + shift, g.size).download()
+        want = po.build_index(g, 12)
+        assert np.array_equal(got["positions"], want.positions)
+        assert np.array_equal(got["pos_lseeds"], want.pos_lseeds)
+        assert np.array_equal(got["base_2bits"], want.base_2bits)
+        assert np.array_equal(got["base_3bits"], want.base_3bits)
