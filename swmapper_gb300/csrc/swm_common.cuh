@@ -40,9 +40,9 @@ struct swm_index {
     uint32_t *d_b2;        // n_words2 + SWM_PAD_WORDS
     uint32_t *d_b3;        // n_words3 + SWM_PAD_WORDS
     // Candidate table (k = 12 only; device-only, derived from the arrays
-    // above): the entries of every bucket grouped, for each seed shift t, by
-    // the 6 flank bits the filter of shift t compares, so that the entries a
-    // read's seed keeps form one contiguous, position-ordered range.
+    // above): the entries grouped by 15-mer and by the shift at which their
+    // 12-mer lies in it, so that the entries a read's seed keeps form one
+    // contiguous, position-ordered range, next to those of the other shifts.
     uint32_t *d_ctab_off;  // SWM_CTAB_KEYS + 1 start offsets into d_ctab_pos
     uint32_t *d_ctab_pos;  // 4 * n_seeds (+8) positions
     uint32_t ctab_gen;     // bumped whenever the table is built or dropped
@@ -54,12 +54,23 @@ struct swm_index {
     cudaEvent_t chain_ev;
 };
 
-// Key of the candidate table: seed code << 8 | shift << 6 | flank, where
-// flank = rl | rh << 3 are the lo / hi bits of the 3 long-seed bases outside
-// the 12-mer (the bits long_seeds_filter compares, mapper_cpe.c:2107-2112).
+// spread the low 16 bits of x to the even bit positions
+__host__ __device__ __forceinline__ uint32_t swm_spread16(uint32_t x) {
+    x &= 0x0000ffffu;
+    x = (x | (x << 8)) & 0x00ff00ffu;
+    x = (x | (x << 4)) & 0x0f0f0f0fu;
+    x = (x | (x << 2)) & 0x33333333u;
+    x = (x | (x << 1)) & 0x55555555u;
+    return x;
+}
+// Keys of the candidate table: 4 key15 + shift. key15 is the 15-mer with lo / hi
+// bits lo, hi: the code of its 9 middle bases (which the 12-mers of all four
+// shifts hold), then that of its 3 first and 3 last bases.
 #define SWM_CTAB_KEYS (1ull << 32)
-__host__ __device__ __forceinline__ uint32_t swm_ctab_key(uint32_t seed, uint32_t shift, uint32_t flank) {
-    return (seed << 8) | (shift << 6) | flank;
+__host__ __device__ __forceinline__ uint32_t swm_ctab_outer(uint32_t x) { return (x & 7u) | ((x >> 12) & 7u) << 3; }
+__host__ __device__ __forceinline__ uint32_t swm_ctab_key15(uint32_t lo, uint32_t hi) {
+    return (swm_spread16((lo >> 3) & 0x1ffu) | swm_spread16((hi >> 3) & 0x1ffu) << 1) << 12 |
+           swm_spread16(swm_ctab_outer(lo)) | swm_spread16(swm_ctab_outer(hi)) << 1;
 }
 // The flank value an index entry with flank code ls offers to shift t.
 __host__ __device__ __forceinline__ uint32_t swm_ctab_flank(uint32_t ls, uint32_t t) {

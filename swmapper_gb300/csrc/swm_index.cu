@@ -252,16 +252,6 @@ __global__ void kb_encode(const uint8_t *__restrict__ seq, uint64_t n, uint32_t 
     }
 }
 
-// spread the low 16 bits of x to the even bit positions
-__device__ __forceinline__ uint32_t spread16(uint32_t x) {
-    x &= 0x0000ffffu;
-    x = (x | (x << 8)) & 0x00ff00ffu;
-    x = (x | (x << 4)) & 0x0f0f0f0fu;
-    x = (x | (x << 2)) & 0x33333333u;
-    x = (x | (x << 1)) & 0x55555555u;
-    return x;
-}
-
 // k-mer at sampled position i (get_seed_from_enc_bits, serial_index.c:280-331);
 // false when it holds an N. With FLANK also its flank code: 3 bases before
 // (bases 0 .. 2 when i is 0) and 3 after, lo bits then hi bits. One 32-base
@@ -278,7 +268,7 @@ __device__ __forceinline__ bool seed_at(const uint2 *__restrict__ b2p, const uin
     const uint32_t qs = (uint32_t)((i - f) % 32);
     const uint2 a = b2p[q], b = b2p[q + 1];
     const uint32_t lo = swm_fsr(a.x, b.x, qs), hi = swm_fsr(a.y, b.y, qs);
-    *seed = spread16((lo >> f) & mask) | (spread16((hi >> f) & mask) << 1);
+    *seed = swm_spread16((lo >> f) & mask) | (swm_spread16((hi >> f) & mask) << 1);
     if (FLANK)
         *flank = (lo & rmask) | ((lo >> (f + k)) & rmask) << res | (hi & rmask) << (2 * res) |
                  ((hi >> (f + k)) & rmask) << (3 * res);
@@ -496,87 +486,122 @@ __global__ void __launch_bounds__(RADIX_THREADS, RADIX_BLOCKS_PER_SM)
 //
 // long_seeds_filter (mapper_cpe.c:2090-2123) keeps an entry of a seed's
 // bucket when the 3 flank bits of each plane at the seed's shift equal the
-// read's, i.e. when the whole 15-base long seed matches. The table groups, for
-// every bucket and every shift t, the bucket's entries by that 6-bit flank
-// value (stable: ascending position inside a group), so that the entries one
-// (seed, shift, read flank) keeps are one contiguous range of positions, found
-// with a single offset lookup. Segment (bucket B, shift t) starts at
-// 4 * off[B] + t * count[B]; ctab_off[key(B, t, v)] is where flank value v
-// starts in it, and ctab_off[key + 1] where it ends (the next key's start,
-// also across shifts and buckets; the last entry holds 4 * n_seeds).
+// read's, i.e. when the whole 15-base long seed matches. The table groups the
+// genome's entries by 15-mer and, within one, by the shift t at which the
+// entry's 12-mer lies in it (stable: ascending position inside a group), so
+// that the entries one (seed, shift, read flank) keeps are one contiguous range
+// of positions, found with a single offset lookup, and the four shifts of a
+// long seed look up neighbouring offsets and read neighbouring ranges: a read's
+// lookups touch one sector of the 17 GiB offset array per long seed instead of
+// one per shift, and so do its positions (ordered by bucket, shift and flank,
+// the table made the candidate stage 27% and the seed stage, which stored a key
+// per seed, 32% slower: 2.18 and 0.80 against 1.72 and 0.61 ms per 524,288 reads of
+// 150 bp on 3.1 Gbp). ctab_off[4 key15 + t] is where a
+// group starts and ctab_off[4 key15 + t + 1] where it ends (the last entry
+// holds 4 * n_seeds); swm_ctab_key15 gives the key.
 
-#define CTAB_WARPS 8
+#define CTAB_THREADS 512
+#define CTAB_CORES (1u << 18)  // codes of the 9 bases every shift's 12-mer holds: one partition each
+#define CTAB_KEYS_CORE (1u << 14)
+#define CTAB_BUCKETS_CORE 256  // buckets that hold a core: 64 at each shift
 
-// One warp per bucket: for each shift a 64-bin histogram of the flank values,
-// its exclusive scan (the 64 offsets, written as one coalesced 256-byte row)
-// and a stable scatter of the positions (rank among equal values from a
-// match mask, chunk by chunk in position order).
-__global__ void __launch_bounds__(CTAB_WARPS * 32) kb_ctab(const uint32_t *__restrict__ off, uint64_t nb,
+// Bucket q of core c9: shift t = q / 64, and the 3 bases of its 12-mer outside
+// the core from q % 64 (3 - t before it, t after).
+__device__ __forceinline__ uint32_t ctab_bucket(uint32_t c9, uint32_t q) {
+    const uint32_t t = q >> 6, w = q & 63u, nl = 2 * (3 - t);
+    return (w & ((1u << nl) - 1)) | (c9 << nl) | ((w >> nl) << (24 - 2 * t));
+}
+
+// Key within the core's partition of an entry of its bucket q with flank value
+// v (swm_ctab_flank at shift t): the 15-mer's 6 outer bases, then t.
+__device__ __forceinline__ uint32_t ctab_local(uint32_t q, uint32_t v) {
+    const uint32_t t = q >> 6, w = q & 63u, nl = 2 * (3 - t);
+    const uint32_t f = (v & 1u) | (v & 8u) >> 2 | (v & 2u) << 1 | (v & 16u) >> 1 | (v & 4u) << 2 | (v & 32u); // 2 bits a base
+    const uint32_t outer = (f & ((1u << (2 * t)) - 1)) | (w & ((1u << nl) - 1)) << (2 * t) | (w >> nl) << 6 |
+                           (f >> (2 * t)) << (6 + 2 * t);
+    return outer << 2 | t;
+}
+
+// entries of every partition (a warp each)
+__global__ void __launch_bounds__(256) kb_ctab_sums(const uint32_t *__restrict__ count, uint32_t *__restrict__ sums) {
+    const uint32_t lane = threadIdx.x & 31, c9 = (blockIdx.x * 256 + threadIdx.x) >> 5;
+    if (c9 >= CTAB_CORES) return;
+    uint32_t s = 0;
+    for (uint32_t q = lane; q < CTAB_BUCKETS_CORE; q += 32) s += count[ctab_bucket(c9, q)];
+    s = __reduce_add_sync(0xffffffffu, s);
+    if (lane == 0) sums[c9] = s;
+}
+
+// One block per core at a time: a histogram of the core's 16,384 keys over the
+// entries of its 256 buckets in shared memory, its exclusive scan (written out
+// as one 64 KB row of offsets), and a stable scatter of the positions. A
+// bucket's entries have keys of their own, so one warp takes each bucket and
+// its match masks keep the order.
+__global__ void __launch_bounds__(CTAB_THREADS, 3) kb_ctab(const uint32_t *__restrict__ off,
                                                            const uint32_t *__restrict__ pos,
                                                            const uint16_t *__restrict__ ls,
+                                                           const uint32_t *__restrict__ base,
                                                            uint32_t *__restrict__ ctab_off,
                                                            uint32_t *__restrict__ ctab_pos) {
-    __shared__ uint32_t hist_all[CTAB_WARPS][64];
-    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    uint32_t *hist = hist_all[wib];
+    extern __shared__ __align__(16) uint32_t ctab_smem[];
+    uint32_t *hist = ctab_smem;                       // CTAB_KEYS_CORE
+    uint32_t *bo = ctab_smem + CTAB_KEYS_CORE;        // bucket starts
+    uint32_t *bc = bo + CTAB_BUCKETS_CORE;            // bucket counts
+    __shared__ uint32_t wtot[CTAB_THREADS / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t nwarps = CTAB_THREADS / 32;
     uint32_t lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-    const uint64_t nwarps = (uint64_t)gridDim.x * CTAB_WARPS;
-    for (uint64_t b = (uint64_t)blockIdx.x * CTAB_WARPS + wib; b < nb; b += nwarps) {
-        const uint32_t o = off[b], c = off[b + 1] - o;
-        uint32_t *row = ctab_off + (b << 8);
-        if (c == 0) { // every key of an empty bucket starts (and ends) at its segment
-            const uint32_t v = 4u * o;
-            reinterpret_cast<uint4 *>(row)[lane] = make_uint4(v, v, v, v);
-            reinterpret_cast<uint4 *>(row)[lane + 32] = make_uint4(v, v, v, v);
-            continue;
+    for (uint32_t c9 = blockIdx.x; c9 < CTAB_CORES; c9 += gridDim.x) {
+        for (uint32_t i = tid; i < CTAB_KEYS_CORE / 4; i += CTAB_THREADS)
+            reinterpret_cast<uint4 *>(hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (tid < CTAB_BUCKETS_CORE) {
+            const uint32_t b = ctab_bucket(c9, tid), o = off[b];
+            bo[tid] = o;
+            bc[tid] = off[b + 1] - o;
         }
-        // small buckets keep their entries in registers across the 4 shifts
-        const uint32_t l0 = lane < c ? ls[o + lane] : 0u;
-        const uint32_t p0 = lane < c ? pos[o + lane] : 0u;
-        for (uint32_t t = 0; t < SWM_SEED_STEP; t++) {
-            const uint32_t base = 4u * o + t * c;
-            hist[lane] = 0;
-            hist[lane + 32] = 0;
-            __syncwarp();
+        __syncthreads();
+        for (uint32_t q = warp; q < CTAB_BUCKETS_CORE; q += nwarps)
+            for (uint32_t j = lane; j < bc[q]; j += 32)
+                atomicAdd(&hist[ctab_local(q, swm_ctab_flank(ls[bo[q] + j], q >> 6))], 1u);
+        __syncthreads();
+        // exclusive scan, 1,024 keys per warp in rows of 32
+        const uint32_t per = CTAB_KEYS_CORE / nwarps, k0 = warp * per;
+        uint32_t run = 0;
+        for (uint32_t j = 0; j < per; j += 32) {
+            const uint32_t v = hist[k0 + j + lane], inc = warp_incl_scan(v);
+            hist[k0 + j + lane] = run + inc - v;
+            run += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0) wtot[warp] = run;
+        __syncthreads();
+        uint32_t at = base[c9];
+        for (uint32_t w = 0; w < warp; w++) at += wtot[w];
+        uint32_t *row = ctab_off + (uint64_t)c9 * CTAB_KEYS_CORE;
+        for (uint32_t j = lane; j < per; j += 32) {
+            const uint32_t v = hist[k0 + j] + at;
+            hist[k0 + j] = v; // now the running cursor of the key
+            __stcs(row + k0 + j, v);
+        }
+        __syncthreads();
+        for (uint32_t q = warp; q < CTAB_BUCKETS_CORE; q += nwarps) {
+            const uint32_t o = bo[q], c = bc[q];
             for (uint32_t j0 = 0; j0 < c; j0 += 32) {
                 const bool in = j0 + lane < c;
-                const uint32_t l = c <= 32 ? l0 : (in ? (uint32_t)ls[o + j0 + lane] : 0u);
-                const uint32_t v = in ? swm_ctab_flank(l, t) : 64u + lane; // out-of-range lanes match nobody
-                const uint32_t mm = __match_any_sync(0xffffffffu, v);
-                if (in && (mm & lt) == 0) hist[v] += __popc(mm); // one leader per value
-                __syncwarp();
-            }
-            // exclusive scan of the 64 bins, two per lane
-            const uint32_t a = hist[2 * lane], d = hist[2 * lane + 1];
-            uint32_t inc = a + d;
-#pragma unroll
-            for (int k = 1; k < 32; k <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, k);
-                if ((int)lane >= k) inc += y;
-            }
-            const uint32_t s0 = base + inc - (a + d);
-            reinterpret_cast<uint2 *>(row + (t << 6))[lane] = make_uint2(s0, s0 + a);
-            __syncwarp();
-            hist[2 * lane] = s0; // now the running cursor of each value
-            hist[2 * lane + 1] = s0 + a;
-            __syncwarp();
-            for (uint32_t j0 = 0; j0 < c; j0 += 32) {
-                const bool in = j0 + lane < c;
-                const uint32_t l = c <= 32 ? l0 : (in ? (uint32_t)ls[o + j0 + lane] : 0u);
-                const uint32_t p = c <= 32 ? p0 : (in ? pos[o + j0 + lane] : 0u);
-                const uint32_t v = in ? swm_ctab_flank(l, t) : 64u + lane;
-                const uint32_t mm = __match_any_sync(0xffffffffu, v);
-                uint32_t at = 0;
-                if (in) at = hist[v] + __popc(mm & lt);
+                const uint32_t p = in ? pos[o + j0 + lane] : 0u;
+                const uint32_t k = in ? ctab_local(q, swm_ctab_flank(ls[o + j0 + lane], q >> 6)) : CTAB_KEYS_CORE + lane;
+                const uint32_t mm = __match_any_sync(0xffffffffu, k); // lanes past the end match nobody
+                uint32_t w = 0;
+                if (in) w = hist[k] + __popc(mm & lt);
                 __syncwarp();
                 if (in) {
-                    ctab_pos[at] = p;
-                    if ((mm & lt) == 0) hist[v] += __popc(mm);
+                    ctab_pos[w] = p;
+                    if ((mm & lt) == 0) hist[k] += __popc(mm);
                 }
                 __syncwarp();
             }
         }
+        __syncthreads();
     }
 }
 
@@ -1079,7 +1104,7 @@ int swm_ctab_build(swm_index *ix, int forced) {
     if (ix->d_ctab_off || ix->ctab_off || ix->k != 12 || 4 * ix->n_seeds + 8 >= 0xffffffffull) return SWM_OK;
     // Built on its own only for genomes whose buckets average SWM_CTAB_MIN_MEAN
     // entries or more: its lookup is a random read of a 17 GiB array per
-    // selected seed, which costs more than filtering a bucket of a few entries
+    // selected long seed, which costs more than filtering buckets of a few entries
     // (a 100 Mbp genome averages 1.5 per bucket, a 3.1 Gbp one 44).
     if (!forced && ix->n_seeds < (uint64_t)SWM_CTAB_MIN_MEAN << (2 * ix->k)) return SWM_OK;
     SWM_CUDA(cudaSetDevice(ix->device));
@@ -1095,16 +1120,22 @@ int swm_ctab_build(swm_index *ix, int forced) {
         cudaGetLastError();
         return SWM_OK;
     }
-    const uint64_t nb = 1ull << (2 * ix->k);
     const uint32_t last = (uint32_t)(4 * ix->n_seeds);
-    cudaError_t e = cudaMemcpy(d_o + SWM_CTAB_KEYS, &last, 4, cudaMemcpyHostToDevice);
+    uint32_t *d_t = nullptr; // the partitions' sums and starts
+    cudaError_t e = cudaMalloc(&d_t, (2ull * CTAB_CORES + 64 + swm_scan_tmp_words(CTAB_CORES)) * 4);
+    if (e == cudaSuccess) e = cudaMemcpy(d_o + SWM_CTAB_KEYS, &last, 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(d_p + 4 * ix->n_seeds, 0, 32);
     if (e == cudaSuccess) {
-        kb_ctab<<<grid_for(nb * 32, CTAB_WARPS * 32, ix->device, 8), CTAB_WARPS * 32>>>(ix->d_off, nb, ix->d_pos,
-                                                                                       ix->d_ls, d_o, d_p);
+        uint32_t *d_sums = d_t, *d_base = d_t + CTAB_CORES, *d_scan = d_base + CTAB_CORES + 64;
+        const size_t smem = (CTAB_KEYS_CORE + 2 * CTAB_BUCKETS_CORE) * 4;
+        kb_ctab_sums<<<CTAB_CORES / 8, 256>>>(ix->d_count, d_sums);
+        if (swm_exclusive_scan(d_sums, d_base, nullptr, CTAB_CORES, CTAB_CORES, d_scan, nullptr, 0) == SWM_OK &&
+            cudaFuncSetAttribute(kb_ctab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
+            kb_ctab<<<sm_count(ix->device) * 3, CTAB_THREADS, smem>>>(ix->d_off, ix->d_pos, ix->d_ls, d_base, d_o, d_p);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    cudaFree(d_t);
     if (e != cudaSuccess) {
         cudaFree(d_o);
         cudaFree(d_p);

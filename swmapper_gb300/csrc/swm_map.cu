@@ -113,8 +113,9 @@ struct MapBufs {
     // per item
     uint32_t *it_w;        // items * 32: [0..15] Myers planes, [16..31] Hamming planes
     uint2 *sel;            // items * 64: (bucket start, count) of the seed of long seed l, shift t at 4 l + t
-    uint8_t *sel_fl;       // items * 64: its read flank bits rl | rh << 3 (rl, rh: 3 bits each)
-    uint32_t *sel_key;     // items * 64: its candidate-table key (k = 12)
+    uint8_t *sel_fl;       // items * 64: its read flank bits rl | rh << 3 (rl, rh: 3 bits each); with the
+                           // candidate table, bits 6-7 of long seed l's bytes hold its N mask (ctab_slot_key)
+    uint32_t *sel_key;     // items * 16: key15 of long seed l in the candidate table (k = 12)
     unsigned long long *it_perm; // items: selected slot i is record 4 * nibble(i / 4) + i % 4
     uint8_t *it_nsel, *it_e;
     uint32_t *it_nch, *it_nel, *it_nbat;
@@ -252,16 +253,6 @@ __device__ __forceinline__ uint32_t even_bits(uint32_t x) {
     return x;
 }
 
-// spread the low 16 bits of x to the even bit positions
-__device__ __forceinline__ uint32_t spread_bits(uint32_t x) {
-    x &= 0x0000ffffu;
-    x = (x | (x << 8)) & 0x00ff00ffu;
-    x = (x | (x << 4)) & 0x0f0f0f0fu;
-    x = (x | (x << 2)) & 0x33333333u;
-    x = (x | (x << 1)) & 0x55555555u;
-    return x;
-}
-
 struct ReadView { // base i of the strand being mapped (reverse_read, mapper_cpe.c:2429-2450)
     const char *src;
     uint32_t L, strand;
@@ -391,7 +382,7 @@ __global__ void __launch_bounds__(SEED_WARPS * 32) k_seed(const uint32_t *__rest
                     const uint32_t sh = (lane & 1) * 16;
                     const uint32_t lo = (SK(pl, 2 * (lane >> 1), t) >> sh) & 0xffffu;
                     const uint32_t hi = (SK(pl, 2 * (lane >> 1) + 1, t) >> sh) & 0xffffu;
-                    wv = spread_bits(lo) | (spread_bits(hi) << 1);
+                    wv = swm_spread16(lo) | (swm_spread16(hi) << 1);
                 }
                 SK(w2, lane, t) = wv;
             }
@@ -409,7 +400,7 @@ __global__ void __launch_bounds__(SEED_WARPS * 32) k_seed(const uint32_t *__rest
                         const uint32_t nhi = wj + 1 < 8 ? SK(pl, 2 * (wj + 1) + 1, t) : 0u;
                         const uint32_t lo = (swm_fsr(SK(pl, 2 * wj, t), nlo, sh) >> sft) & kmask;
                         const uint32_t hi = (swm_fsr(SK(pl, 2 * wj + 1, t), nhi, sh) >> sft) & kmask;
-                        sd = spread_bits(lo) | (spread_bits(hi) << 1);
+                        sd = swm_spread16(lo) | (swm_spread16(hi) << 1);
                     } else {
                         sd = seed_closed(rv, k, l, sft);
                     }
@@ -513,7 +504,7 @@ __global__ void __launch_bounds__(SEED_WARPS * 32) k_seed(const uint32_t *__rest
                     const uint32_t lr = swm_fsr(SK(pl, 2 * wj, t), nlo, sh) & lmask; // set_read_long_seeds, 2474-2478
                     const uint32_t hr = swm_fsr(SK(pl, 2 * wj + 1, t), nhi, sh) & lmask;
                     const uint32_t sd = has_n ? seed_closed(rv, k, l, sft)
-                                              : (spread_bits((lr >> sft) & kmask) | (spread_bits((hr >> sft) & kmask) << 1));
+                                              : (swm_spread16((lr >> sft) & kmask) | (swm_spread16((hr >> sft) & kmask) << 1));
                     const uint32_t o0 = off[sd], c = off[sd + 1] - o0;
                     const uint32_t m = (1u << sft) - 1, kk = k + sft;
                     const uint32_t rl = ((lr & m) | ((lr >> kk) << sft)) & rmask; // 2483-2495
@@ -651,7 +642,7 @@ __device__ __forceinline__ uint32_t seed12_code(uint32_t w0, uint32_t w1, uint32
     return (sh ? __funnelshift_r(w0, w1, sh) : w0) & 0xffffffu;
 }
 __device__ __forceinline__ uint32_t seed12_nfix(uint32_t sd, uint32_t nk, uint32_t sft) {
-    const uint32_t M = spread_bits(nk & 0xfffu) * 3u;
+    const uint32_t M = swm_spread16(nk & 0xfffu) * 3u;
     return (sd & ~M) | (nfill12(sft) & M);
 }
 
@@ -660,7 +651,9 @@ __device__ __forceinline__ uint32_t seed12_nfix(uint32_t sd, uint32_t nk, uint32
 // flw, where rl / rh are the lo / hi bits of the 3 long-seed bases outside
 // the 12-mer (set_read_long_seeds, 2474-2478). cnt gets the bucket counts summed per
 // long seed (choose_seed, 1372-1390), nref the refill chunks. Every lookup is
-// independent, so they all issue back to back.
+// independent, so they all issue back to back. KEYS: also the long seeds' keys
+// in the candidate table (N bases of the middle 9 with their seed codes, outer
+// ones as the planes have them and named in the flank bytes' top bits).
 template <int NL, bool HASN, bool KEYS>
 __device__ __forceinline__ void seed12_records(const uint32_t (&iw)[NL], const uint32_t (&plo)[8],
                                                const uint32_t (&phi)[8], const uint32_t (&pok)[8], uint32_t nl,
@@ -669,7 +662,7 @@ __device__ __forceinline__ void seed12_records(const uint32_t (&iw)[NL], const u
                                                uint32_t *__restrict__ keys, uint32_t (&cnt)[NL],
                                                uint32_t (&nref)[NL]) {
     static_assert(NL % 2 == 0, "flank words are stored in pairs");
-    uint32_t pf = 0;
+    uint32_t pf = 0, pk = 0;
 #pragma unroll
     for (int l = 0; l < NL; l++) {
         const bool act = (uint32_t)l < nl;
@@ -677,7 +670,21 @@ __device__ __forceinline__ void seed12_records(const uint32_t (&iw)[NL], const u
         const uint32_t nlo = wj0 + 1 < 8 ? plo[wj0 + 1] : 0u, nhi = wj0 + 1 < 8 ? phi[wj0 + 1] : 0u;
         const uint32_t lr = (sh0 ? __funnelshift_r(plo[wj0], nlo, sh0) : plo[wj0]) & 0x7fffu;
         const uint32_t hr = (sh0 ? __funnelshift_r(phi[wj0], nhi, sh0) : phi[wj0]) & 0x7fffu;
-        uint32_t csum = 0, rsum = 0, f = 0, po = 0, pc = 0, kk4[SWM_SEED_STEP];
+        uint32_t csum = 0, rsum = 0, f = 0, po = 0, pc = 0;
+        if (KEYS) {
+            uint32_t klo = lr, khi = hr;
+            if (HASN) {
+                const uint32_t nx = wj0 + 1 < 8 ? pok[wj0 + 1] : 0xffffffffu;
+                const uint32_t nk = ~(sh0 ? __funnelshift_r(pok[wj0], nx, sh0) : pok[wj0]) & 0x7fffu;
+                const uint32_t nc = nk & 0xff8u, no = swm_ctab_outer(nk);
+                klo = (klo & ~nc) | (nc & 0xaa8u); // code d % 4 of base d = 3 .. 11
+                khi = (khi & ~nc) | (nc & 0xcc8u);
+                f = (no & 3u) << 6 | (no & 12u) << 12 | (no & 48u) << 18;
+            }
+            const uint32_t key = swm_ctab_key15(klo, khi);
+            if (l & 1) __stcs(reinterpret_cast<uint2 *>(keys) + (l >> 1), make_uint2(pk, key)); // two per store
+            pk = key;
+        }
 #pragma unroll
         for (uint32_t sft = 0; sft < SWM_SEED_STEP; sft++) {
             const uint32_t o = ob + sft, w = o >> 4;
@@ -698,12 +705,10 @@ __device__ __forceinline__ void seed12_records(const uint32_t (&iw)[NL], const u
             po = o0;
             pc = c;
             f |= (rl | (rh << 3)) << (8 * sft);
-            if (KEYS) kk4[sft] = swm_ctab_key(sd, sft, rl | (rh << 3));
             csum += c;
             rsum += c > SWM_PER_FETCH ? (c - 1) / SWM_PER_FETCH : 0u;
         }
         if (l & 1) __stcs(reinterpret_cast<uint2 *>(flw) + (l >> 1), make_uint2(pf, f)); // two long seeds per store
-        if (KEYS) __stcs(reinterpret_cast<uint4 *>(keys) + l, make_uint4(kk4[0], kk4[1], kk4[2], kk4[3]));
         pf = f;
         cnt[l] = act ? csum : 0u;
         nref[l] = act ? rsum : 0u;
@@ -714,7 +719,7 @@ template <int NL, bool TABLE>
 // Items whose read length is outside [lo_len, hi_len] belong to the other
 // instantiation launched beside this one (reads of up to 164 bases take the
 // 10-long-seed kernel, longer ones the 16-long-seed kernel). TABLE: the
-// candidate table is in use, so each seed's table key is stored too.
+// candidate table is in use, so each long seed's table key is stored too.
 __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs B,
                                                            uint32_t lo_len, uint32_t hi_len) {
     const BlockParams P = *B.par;
@@ -868,7 +873,7 @@ __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs
         for (int w = 0; w < NL; w++) {
             const uint32_t l16 = (w & 1) ? (plo[w >> 1] >> 16) : plo[w >> 1];
             const uint32_t h16 = (w & 1) ? (phi[w >> 1] >> 16) : phi[w >> 1];
-            iw[w] = spread_bits(l16) | (spread_bits(h16) << 1);
+            iw[w] = swm_spread16(l16) | (swm_spread16(h16) << 1);
         }
         // ---- Myers planes: complete 2-bit words up to P are the planes, the
         // partial word is unwritten; the tail replay rewrites words P/16 and
@@ -909,7 +914,7 @@ __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs
                 else wb = v;
             };
             if (P % 16 == 15) {
-                wa = spread_bits(lwin & 0xffffu) | (spread_bits(hwin & 0xffffu) << 1);
+                wa = swm_spread16(lwin & 0xffffu) | (swm_spread16(hwin & 0xffffu) << 1);
             }
             uint32_t acc = 0;
             if (P % 16 != 15)
@@ -962,7 +967,7 @@ __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs
         const uint64_t sb = (uint64_t)item * SWM_MAX_SEL;
         uint32_t CNT[NL], IDX[NL], REF[NL];
         uint32_t *flw = reinterpret_cast<uint32_t *>(B.sel_fl + sb);
-        uint32_t *keys = B.sel_key + sb;
+        uint32_t *keys = B.sel_key + (uint64_t)item * (SWM_MAX_SEL / SWM_SEED_STEP);
         if (has_n) seed12_records<NL, true, TABLE>(iw, plo, phi, pok, nl, off, pol, sel + sb, flw, keys, CNT, REF);
         else seed12_records<NL, false, TABLE>(iw, plo, phi, pok, nl, off, pol, sel + sb, flw, keys, CNT, REF);
 #pragma unroll
@@ -1615,7 +1620,7 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS) k_cand(const
                 const uint2 sv = B.sel[sb + rs];
                 const uint32_t fb = B.sel_fl[sb + rs];
                 // base | shift << 16 | rl << 20 | rh << 24
-                S.sel[i] = (l * klong + sft) | ((SWM_SEED_STEP - 1 - sft) << 16) | ((fb & 7u) << 20) | ((fb >> 3) << 24);
+                S.sel[i] = (l * klong + sft) | ((SWM_SEED_STEP - 1 - sft) << 16) | ((fb & 7u) << 20) | ((fb >> 3 & 7u) << 24);
                 S.st[i] = sv.x;
                 S.cn[i] = sv.y;
             }
@@ -1725,7 +1730,7 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS) k_cand(const
 // ======================================================================
 //
 // With the candidate table, the entries a seed's flank filter keeps are one
-// position-ordered range of the table (key: seed code, shift, read flank), so
+// position-ordered range of the table (key: long seed, shift), so
 // a batch reads only its survivors instead of every entry of its chunks. A
 // batch's survivors of seed i are the range's entries whose bucket rank is
 // among the ranks the batch fetched for that seed: all of them when the item
@@ -1748,6 +1753,20 @@ struct CandTabSmem {
     uint32_t rb[SWM_MAX_SEL];        // its seed's base (position adjust)
     uint32_t sc[CAND_SMEM_KEEP];     // kept positions of a batch, while they fit
 };
+
+// Table key of the seed at shift sft of a long seed: 4 key15 + sft. Outer bases
+// of the 15-mer that are N (mask in bits 6-7 of the long seed's flank bytes:
+// the 3 first, then the 3 last) take their seed code where the shift's 12-mer
+// holds them (nfill12: d % 4 for base d < 12, then 3) and keep the plane's
+// elsewhere.
+__device__ __forceinline__ uint32_t ctab_slot_key(uint32_t key15, uint32_t flanks, uint32_t sft) {
+    if (flanks & 0x00c0c0c0u) {
+        const uint32_t no = (flanks >> 6 & 3u) | (flanks >> 12 & 12u) | (flanks >> 18 & 48u);
+        const uint32_t m = swm_spread16(no & (7u << sft)) * 3u;
+        key15 = (key15 & ~m) | (0xfe4u & m);
+    }
+    return key15 << 2 | sft;
+}
 
 // First index in [a, z) whose position is above p1 (positions ascending).
 __device__ __forceinline__ uint32_t upper_pos(const uint32_t *__restrict__ tp, uint32_t a, uint32_t z, uint32_t p1) {
@@ -1787,9 +1806,9 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS)
             for (uint32_t i = lane; i < ns; i += 32) {
                 const uint32_t rs = sel_slot(perm, i), l = rs / SWM_SEED_STEP, sft = rs % SWM_SEED_STEP;
                 const uint2 sv = B.sel[sb + rs];
-                const uint32_t fb = B.sel_fl[sb + rs];
-                const uint32_t key = B.sel_key[sb + rs];
-                S.sel[i] = (l * klong + sft) | ((SWM_SEED_STEP - 1 - sft) << 16) | ((fb & 7u) << 20) | ((fb >> 3) << 24);
+                const uint32_t fw = reinterpret_cast<const uint32_t *>(B.sel_fl + sb)[l], fb = fw >> (8 * sft);
+                const uint32_t key = ctab_slot_key(B.sel_key[(uint64_t)item * (SWM_MAX_SEL / SWM_SEED_STEP) + l], fw, sft);
+                S.sel[i] = (l * klong + sft) | ((SWM_SEED_STEP - 1 - sft) << 16) | ((fb & 7u) << 20) | ((fb >> 3 & 7u) << 24);
                 S.st[i] = sv.x;
                 S.cn[i] = sv.y;
                 uint32_t d0 = 0, d1 = 0;
@@ -3550,7 +3569,7 @@ static int alloc_items(swm_mapper *m) {
     rc |= dmalloc(&B.it_w, I * 32);
     rc |= dmalloc(&B.sel, I * SWM_MAX_SEL);
     rc |= dmalloc(&B.sel_fl, I * SWM_MAX_SEL);
-    rc |= dmalloc(&B.sel_key, I * SWM_MAX_SEL);
+    rc |= dmalloc(&B.sel_key, I * (SWM_MAX_SEL / SWM_SEED_STEP));
     rc |= dmalloc(&B.it_perm, I);
     rc |= dmalloc(&B.unm, I / 32 + 1);
     rc |= dmalloc(&B.it_nsel, I);

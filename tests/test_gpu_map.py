@@ -515,3 +515,22 @@ def test_gpu_records_split_past_the_record_limit(cuda_lib):
     assert max(per_item.values()) >= 2, "the workload should split some item's locations over records"
     out, _, _ = _gpu(cuda_lib, g, reads, lens, 7)
     _check(out, ref.records(), ref.unmapped)
+
+
+@pytest.mark.parametrize("table", [True, False])
+def test_gpu_n_bases_in_every_place_of_a_long_seed(cuda_lib, table):
+    """N bases take a code of their own in a seed but not in its flanks, so the
+    table key of a long seed with an outer N depends on the shift: one N at
+    every offset of a long seed, pairs of outer Ns, and runs over two seeds."""
+    g = genome(400_000, 31, "repeats100m", copies_per_family=30, rep_len_max=2000)
+    reads, lens, _, _ = synth.reads(g, 900, 100, 160, 0.01, seed=32, stride=160)
+    for i in range(900):
+        at = 15 * (i % 5)
+        for d in ((i // 5 % 15,), (i % 3, 12 + i // 3 % 3), range(i % 15, i % 15 + 3))[i // 300]:
+            reads[i, at + d] = ord("N")
+    _, mix = oracle_index(g)
+    for e in (4, 9):
+        ref = po.map_reads(mix, reads, lens, e, nthreads=8)
+        out, m, _ = _gpu(cuda_lib, g, reads, lens, e, table=table)
+        _check(out, ref.records(), ref.unmapped)
+        assert m.stats()["candidates"] == ref.stats["candidates"]
