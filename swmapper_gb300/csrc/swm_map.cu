@@ -42,7 +42,7 @@
 // item = 2 * read + strand (cur_read, mapper_cpe.c:2628)
 
 enum { VR_FAIL = 0, VR_HAM = 1, VR_TB = 2, VR_INVALID = 3, VR_NEEDTB = 4 };
-enum { OV_CHUNKS = 1, OV_ELEMS = 2, OV_CANDS = 4, OV_RECS = 8, OV_ARENA = 16, OV_BAD = 32 };
+enum { OV_CHUNKS = 1, OV_ELEMS = 2, OV_CANDS = 4, OV_RECS = 8, OV_ARENA = 16, OV_BAD = 32, OV_WAIT = 64 };
 enum {
     ST_BATCHES = 0,
     ST_CELLS,
@@ -62,6 +62,8 @@ enum {
     TOT_PLW, TOT_PLWQ, // items with refills and more selected seeds, queue head of k_plan
     TOT_CQ,            // queue head of the candidate stage (items)
     TOT_RQC, TOT_RQW,  // queue heads of the records count and write passes (groups of 32 items)
+    TOT_SC1, TOT_SC2, TOT_SC3, // tile tickets of the scans after the seed, candidate and records-count stages
+    TOT_TBDONE, TOT_RDONE,     // blocks of k_traceback and of the records write pass that are through
     TOT_N
 };
 
@@ -97,6 +99,8 @@ __device__ __forceinline__ uint32_t single_batch(uint32_t nref, uint32_t nel) {
 }
 
 #define ARENA_CAP_DEFAULT (1u << 20)
+#define SCAN_TILE_ITEMS 2048 // items per tile of k_scan_items
+#define SCAN_VALUES 6        // values scanned per block: refill chunks, positions, candidates, records, words, bytes
 
 // The inputs of one block, in device memory so that the captured launch
 // sequence of a mapper does not depend on them.
@@ -154,7 +158,8 @@ struct MapBufs {
     // bookkeeping
     uint32_t *tot;    // TOT_N
     unsigned long long *stat; // ST_N
-    uint32_t *scan_tmp;
+    unsigned long long *scan_state; // SCAN_VALUES rows of scan_tiles tile states
+    uint64_t scan_tiles;
 };
 
 // Forms of the verification stage (swm_mapper_tuning); all give the same
@@ -1030,6 +1035,139 @@ __device__ __forceinline__ uint32_t warp_scan_incl(uint32_t v) {
         if ((int)lane_id() >= d) v += t;
     }
     return v;
+}
+
+// Start of a block: its inputs from the pinned parameter block (read in place)
+// to B.par, and the totals, statistics and scan states cleared.
+__global__ void __launch_bounds__(1024) k_begin(const BlockParams *__restrict__ h, MapBufs B) {
+    __shared__ BlockParams P;
+    const uint32_t words = sizeof(BlockParams) / 4;
+    if (threadIdx.x < words) {
+        const uint32_t v = reinterpret_cast<const volatile uint32_t *>(h)[threadIdx.x];
+        reinterpret_cast<uint32_t *>(&P)[threadIdx.x] = v;
+        if (blockIdx.x == 0) reinterpret_cast<uint32_t *>(B.par)[threadIdx.x] = v;
+    }
+    if (blockIdx.x == 0) {
+        if (threadIdx.x < TOT_N) B.tot[threadIdx.x] = 0;
+        if (threadIdx.x < ST_N) B.stat[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    const uint64_t tiles = (P.nitems + SCAN_TILE_ITEMS - 1) / SCAN_TILE_ITEMS;
+    const uint64_t n = tiles * SCAN_VALUES;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        B.scan_state[i / tiles * B.scan_tiles + i % tiles] = 0;
+}
+
+// Exclusive scans of K per-item values in one launch (out gets nitems + 1
+// entries, *tot the total; one of 2^32 - 1 or more as SWM_SCAN_SATURATED, as
+// swm_exclusive_scan's). A block scans a tile of 2,048 items and adds up the
+// tiles before it by looking back at their published sums (state: sum | 1 << 62,
+// or sum of all tiles so far | 2 << 62; decoupled look-back, Merrill & Garland
+// 2016), a warp per value, 32 tiles per step. Tiles are numbered by a ticket in
+// the order their blocks start, so every predecessor is running or done and
+// the wait ends; a wait past SCAN_SPIN_LIMIT polls fails the block instead.
+// One launch replaces three per value: with those, a block was 31 launches and
+// 16 reads took 129 us on the GPU; now 15 and 108 us.
+struct ScanItems {
+    const uint32_t *in[3];
+    uint32_t *out[3];
+    uint32_t tot[3], row, ticket; // TOT_ index of each total, first row of states, TOT_ index of the ticket
+};
+#define SCAN_SPIN_LIMIT (1u << 22)
+
+template <int K>
+__global__ void __launch_bounds__(256) k_scan_items(MapBufs B, ScanItems A) {
+    constexpr int V = SCAN_TILE_ITEMS / 256;
+    static_assert(V == 8, "two 16-byte loads a thread");
+    __shared__ unsigned long long wsum[K][8], before[K], sum[K];
+    __shared__ uint32_t s_tile;
+    const uint32_t n = B.par->nitems, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tiles = n ? (n - 1) / SCAN_TILE_ITEMS + 1 : 1;
+    if (blockIdx.x >= tiles) return; // as many blocks stay as there are tiles
+    if (tid == 0) s_tile = atomicAdd(&B.tot[A.ticket], 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile, i0 = tile * SCAN_TILE_ITEMS + tid * V;
+    uint32_t v[K][V];
+    unsigned long long mine[K], incl[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (i0 + V <= n) {
+            const uint4 a = reinterpret_cast<const uint4 *>(A.in[k] + i0)[0], b = reinterpret_cast<const uint4 *>(A.in[k] + i0)[1];
+            v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
+            v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < V; j++) v[k][j] = i0 + j < n ? A.in[k][i0 + j] : 0u;
+        }
+        mine[k] = 0;
+#pragma unroll
+        for (int j = 0; j < V; j++) mine[k] += v[k][j];
+        incl[k] = mine[k];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long t = __shfl_up_sync(0xffffffffu, incl[k], d);
+            if ((int)lane >= d) incl[k] += t;
+        }
+        if (lane == 31) wsum[k][warp] = incl[k];
+    }
+    __syncthreads();
+    if (warp < K) { // warp k: the tile's sum of value k, and the sum of the tiles before
+        unsigned long long total = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) total += wsum[warp][w];
+        volatile unsigned long long *state = B.scan_state + (uint64_t)(A.row + warp) * B.scan_tiles;
+        if (lane == 0) state[tile] = total | (tile ? 1ull << 62 : 2ull << 62);
+        unsigned long long pre = 0;
+        uint32_t spins = 0;
+        for (int64_t p = (int64_t)tile - 1; p >= 0;) {
+            const unsigned long long x = p >= (int64_t)lane ? state[p - lane] : 2ull << 62;
+            const uint32_t whole = __ballot_sync(0xffffffffu, x >> 62 == 2), none = __ballot_sync(0xffffffffu, x >> 62 == 0);
+            const uint32_t use = whole ? (2u << (__ffs(whole) - 1)) - 1 : 0xffffffffu; // up to the first whole sum
+            if (none & use) { // one of them is not published yet
+                if (++spins > SCAN_SPIN_LIMIT) {
+                    if (lane == 0) atomicOr(&B.tot[TOT_FLAGS], OV_WAIT);
+                    break;
+                }
+                continue;
+            }
+            unsigned long long y = use >> lane & 1u ? x & ((1ull << 62) - 1) : 0ull;
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) y += __shfl_xor_sync(0xffffffffu, y, d);
+            pre += y;
+            if (whole) break;
+            p -= 32;
+        }
+        if (lane == 0) {
+            if (tile) state[tile] = (pre + total) | 2ull << 62;
+            before[warp] = pre;
+            sum[warp] = pre + total;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        unsigned long long ex = before[k] + incl[k] - mine[k];
+        for (uint32_t w = 0; w < warp; w++) ex += wsum[k][w];
+        uint32_t o[V];
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            o[j] = (uint32_t)ex;
+            ex += v[k][j];
+        }
+        if (i0 + V <= n) {
+            reinterpret_cast<uint4 *>(A.out[k] + i0)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            reinterpret_cast<uint4 *>(A.out[k] + i0)[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < V; j++)
+                if (i0 + j < n) A.out[k][i0 + j] = o[j];
+        }
+        if (tile == tiles - 1 && tid == 0) {
+            const uint32_t t = sum[k] < SWM_SCAN_SATURATED ? (uint32_t)sum[k] : SWM_SCAN_SATURATED;
+            A.out[k][n] = t;
+            B.tot[A.tot[k]] = t;
+        }
+    }
 }
 
 // The items whose selected buckets need refills, compacted into the planners'
@@ -2915,6 +3053,118 @@ __device__ __forceinline__ int match_run(const uint32_t *WL, const uint32_t *WH,
     return run;
 }
 
+// Traceback with the whole D0 / HP history in local memory, for the rare walks
+// whose route outgrows the shared-memory path of k_traceback (align_reads,
+// mapper_cpe.c:288-509): nslow of them, by the threads of one block.
+__device__ __noinline__ void traceback_slow(const uint32_t *__restrict__ b2, uint64_t b2_words, uint64_t ref_length,
+                                            const MapBufs &B, uint64_t cap_arena, uint32_t nslow) {
+    const uint32_t *__restrict__ lens = B.par->lens;
+    for (uint32_t q = threadIdx.x; q < nslow; q += blockDim.x) {
+        const uint64_t c = __ldcg(&B.slow_list[q]);
+        const uint32_t item = B.cc_item[c];
+        const uint32_t L = lens[item >> 1], e = B.it_e[item];
+        const uint32_t ws = B.vr_loc[c];
+        const int err = B.vr_err[c], loc = B.vr_mloc[c];
+        uint32_t rl;
+        window_start(B.cc_pos[c], L, e, ref_length, &rl);
+        uint32_t WL[SWM_WIN_WORDS], WH[SWM_WIN_WORDS];
+        load_window(b2, b2_words, ws, L, e, WL, WH);
+        const uint32_t *RW = B.it_w + (uint64_t)item * 32;
+        uint32_t rw[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) rw[i] = RW[i];
+        int start = loc - (int)L + 1;
+        uint8_t *slot = B.vr_cig + c * SWM_CIGAR_SLOT;
+        uint32_t d0h[SWM_MAX_READ_LEN], hph[SWM_MAX_READ_LEN];
+        myers_history(WL, WH, rw, L, e, d0h, hph);
+        int match_site = loc;
+        int search_site = match_site - ((int)L - 1);
+        int i = (int)L - 1, sum_err = 0, jj = 1;
+        int pre_size = 1;
+        char pre_char = 'N';
+        uint16_t rsz[3 * SWM_MAX_READ_LEN + 64];
+        char rch[3 * SWM_MAX_READ_LEN + 64];
+#define TBBIT(arr, ii_, s_) (((s_) >= 0 && (s_) < 32) ? (((arr)[ii_] >> (s_)) & 1u) : 0u)
+#define TBREF(m_) (((WL[(m_) >> 5] >> ((m_) & 31)) & 1u) | (((WH[(m_) >> 5] >> ((m_) & 31)) & 1u) << 1))
+#define TBREAD(r_) (((rw[2 * ((r_) >> 5)] >> ((r_) & 31)) & 1u) | (((rw[2 * ((r_) >> 5) + 1] >> ((r_) & 31)) & 1u) << 1))
+        if (TBBIT(d0h, i, search_site) && TBREF(match_site) == TBREAD(i)) {
+            i--; pre_size = 1; pre_char = 'M'; match_site--;
+        } else if (!TBBIT(d0h, i, search_site) && TBREF(match_site) != TBREAD(i)) {
+            i--; pre_size = 1; pre_char = 'S'; match_site--; sum_err++;
+        } else if (TBBIT(hph, i, search_site)) {
+            i--; search_site++; pre_size = 1; pre_char = 'S'; sum_err++; start++;
+        } else {
+            search_site--; pre_size = 1; pre_char = 'D'; match_site--; sum_err++; start--;
+        }
+        while (i >= 0) {
+            if (sum_err == err) break;
+            if (match_site < 0) break; // defined stop below the window start
+            if (TBBIT(d0h, i, search_site) && TBREF(match_site) == TBREAD(i)) {
+                i--; match_site--;
+                if (pre_char != 'M') { rsz[jj] = (uint16_t)pre_size; rch[jj++] = pre_char; pre_size = 1; pre_char = 'M'; }
+                else pre_size++;
+            } else if (!TBBIT(d0h, i, search_site) && TBREF(match_site) != TBREAD(i)) {
+                i--; match_site--; sum_err++;
+                if (pre_char != 'S') { rsz[jj] = (uint16_t)pre_size; rch[jj++] = pre_char; pre_size = 1; pre_char = 'S'; }
+                else pre_size++;
+            } else if (TBBIT(hph, i, search_site)) {
+                i--; search_site++; sum_err++;
+                if (pre_char != 'I') { rsz[jj] = (uint16_t)pre_size; rch[jj++] = pre_char; pre_size = 1; pre_char = 'I'; }
+                else pre_size++;
+                start++;
+            } else {
+                search_site--; match_site--; sum_err++;
+                if (pre_char != 'D') { rsz[jj] = (uint16_t)pre_size; rch[jj++] = pre_char; pre_size = 1; pre_char = 'D'; }
+                else pre_size++;
+                start--;
+            }
+        }
+#undef TBBIT
+#undef TBREF
+#undef TBREAD
+        rsz[jj] = (uint16_t)pre_size;
+        rch[jj++] = pre_char;
+        if (i >= 0) {
+            rsz[jj] = (uint16_t)(i + 1);
+            rch[jj++] = 'M';
+        }
+        uint8_t txt[TB_TEXT_MAX];
+        int n = 0;
+        for (jj = jj - 1; jj > 0; jj--) {
+            if (n > TB_TEXT_MAX - 8) break;
+            if (rch[jj] == 'M' || rch[jj] == 'S') {
+                int smv = 0;
+                while (jj > 0 && (rch[jj] == 'M' || rch[jj] == 'S')) {
+                    smv += rsz[jj];
+                    jj--;
+                }
+                jj++;
+                n += put_len(txt + n, (uint32_t)smv);
+                txt[n++] = 'M';
+            } else {
+                n += put_len(txt + n, rsz[jj]);
+                txt[n++] = (uint8_t)rch[jj];
+            }
+        }
+        slot[0] = (uint8_t)err;
+        slot[1] = (uint8_t)n;
+        if (n <= SWM_CIGAR_SLOT - 2) {
+            for (int q = 0; q < n; q++) slot[2 + q] = txt[q];
+        } else {
+            uint32_t at = atomicAdd(&B.tot[TOT_ARENA], (uint32_t)n);
+            if ((uint64_t)at + n <= cap_arena) {
+                for (int q = 0; q < n; q++) B.arena[at + q] = txt[q];
+                B.vr_aoff[c] = at;
+            } else {
+                atomicOr(&B.tot[TOT_FLAGS], OV_ARENA);
+            }
+        }
+        B.vr_tlen[c] = (uint16_t)n;
+        B.vr_loc[c] = ws + (uint32_t)start + 1;
+        B.vr_flag[c] = VR_TB;
+    }
+}
+
 __global__ void __launch_bounds__(TB_THREADS) k_traceback(const uint32_t *__restrict__ b2, uint64_t b2_words,
                                                           uint64_t ref_length, MapBufs B, uint64_t cap_chunks,
                                                           uint64_t cap_elems, uint64_t cap_cands, uint64_t cap_arena) {
@@ -3105,121 +3355,15 @@ __global__ void __launch_bounds__(TB_THREADS) k_traceback(const uint32_t *__rest
         B.vr_loc[c] = ws + (uint32_t)start + 1;
         B.vr_flag[c] = VR_TB;
     }
-}
-
-// Traceback with the whole D0 / HP history in local memory, for the rare walks
-// whose route outgrows the shared-memory path of k_traceback (align_reads,
-// mapper_cpe.c:288-509).
-__global__ void __launch_bounds__(128) k_traceback_slow(const uint32_t *__restrict__ b2, uint64_t b2_words,
-                                                        uint64_t ref_length, MapBufs B, uint64_t cap_chunks,
-                                                        uint64_t cap_elems, uint64_t cap_cands, uint64_t cap_arena) {
-    if (block_failed(B, cap_chunks, cap_elems, cap_cands)) return;
-    const uint32_t *__restrict__ lens = B.par->lens;
-    const uint64_t nslow = B.tot[TOT_SLOW];
-    for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nslow; q += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t c = B.slow_list[q];
-        const uint32_t item = B.cc_item[c];
-        const uint32_t L = lens[item >> 1], e = B.it_e[item];
-        const uint32_t ws = B.vr_loc[c];
-        const int err = B.vr_err[c], loc = B.vr_mloc[c];
-        uint32_t rl;
-        window_start(B.cc_pos[c], L, e, ref_length, &rl);
-        uint32_t WL[SWM_WIN_WORDS], WH[SWM_WIN_WORDS];
-        load_window(b2, b2_words, ws, L, e, WL, WH);
-        const uint32_t *RW = B.it_w + (uint64_t)item * 32;
-        uint32_t rw[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) rw[i] = RW[i];
-        int start = loc - (int)L + 1;
-        uint8_t *slot = B.vr_cig + c * SWM_CIGAR_SLOT;
-        uint32_t d0h[SWM_MAX_READ_LEN], hph[SWM_MAX_READ_LEN];
-        myers_history(WL, WH, rw, L, e, d0h, hph);
-        int match_site = loc;
-        int search_site = match_site - ((int)L - 1);
-        int i = (int)L - 1, sum_err = 0, jj = 1;
-        int pre_size = 1;
-        char pre_char = 'N';
-        uint16_t rsz[3 * SWM_MAX_READ_LEN + 64];
-        char rch[3 * SWM_MAX_READ_LEN + 64];
-#define TBBIT(arr, ii_, s_) (((s_) >= 0 && (s_) < 32) ? (((arr)[ii_] >> (s_)) & 1u) : 0u)
-#define TBREF(m_) (((WL[(m_) >> 5] >> ((m_) & 31)) & 1u) | (((WH[(m_) >> 5] >> ((m_) & 31)) & 1u) << 1))
-#define TBREAD(r_) (((rw[2 * ((r_) >> 5)] >> ((r_) & 31)) & 1u) | (((rw[2 * ((r_) >> 5) + 1] >> ((r_) & 31)) & 1u) << 1))
-        if (TBBIT(d0h, i, search_site) && TBREF(match_site) == TBREAD(i)) {
-            i--; pre_size = 1; pre_char = 'M'; match_site--;
-        } else if (!TBBIT(d0h, i, search_site) && TBREF(match_site) != TBREAD(i)) {
-            i--; pre_size = 1; pre_char = 'S'; match_site--; sum_err++;
-        } else if (TBBIT(hph, i, search_site)) {
-            i--; search_site++; pre_size = 1; pre_char = 'S'; sum_err++; start++;
-        } else {
-            search_site--; pre_size = 1; pre_char = 'D'; match_site--; sum_err++; start--;
-        }
-        while (i >= 0) {
-            if (sum_err == err) break;
-            if (match_site < 0) break; // defined stop below the window start
-            if (TBBIT(d0h, i, search_site) && TBREF(match_site) == TBREAD(i)) {
-                i--; match_site--;
-                if (pre_char != 'M') { rsz[jj] = (uint16_t)pre_size; rch[jj++] = pre_char; pre_size = 1; pre_char = 'M'; }
-                else pre_size++;
-            } else if (!TBBIT(d0h, i, search_site) && TBREF(match_site) != TBREAD(i)) {
-                i--; match_site--; sum_err++;
-                if (pre_char != 'S') { rsz[jj] = (uint16_t)pre_size; rch[jj++] = pre_char; pre_size = 1; pre_char = 'S'; }
-                else pre_size++;
-            } else if (TBBIT(hph, i, search_site)) {
-                i--; search_site++; sum_err++;
-                if (pre_char != 'I') { rsz[jj] = (uint16_t)pre_size; rch[jj++] = pre_char; pre_size = 1; pre_char = 'I'; }
-                else pre_size++;
-                start++;
-            } else {
-                search_site--; match_site--; sum_err++;
-                if (pre_char != 'D') { rsz[jj] = (uint16_t)pre_size; rch[jj++] = pre_char; pre_size = 1; pre_char = 'D'; }
-                else pre_size++;
-                start--;
-            }
-        }
-#undef TBBIT
-#undef TBREF
-#undef TBREAD
-        rsz[jj] = (uint16_t)pre_size;
-        rch[jj++] = pre_char;
-        if (i >= 0) {
-            rsz[jj] = (uint16_t)(i + 1);
-            rch[jj++] = 'M';
-        }
-        uint8_t txt[TB_TEXT_MAX];
-        int n = 0;
-        for (jj = jj - 1; jj > 0; jj--) {
-            if (n > TB_TEXT_MAX - 8) break;
-            if (rch[jj] == 'M' || rch[jj] == 'S') {
-                int smv = 0;
-                while (jj > 0 && (rch[jj] == 'M' || rch[jj] == 'S')) {
-                    smv += rsz[jj];
-                    jj--;
-                }
-                jj++;
-                n += put_len(txt + n, (uint32_t)smv);
-                txt[n++] = 'M';
-            } else {
-                n += put_len(txt + n, rsz[jj]);
-                txt[n++] = (uint8_t)rch[jj];
-            }
-        }
-        slot[0] = (uint8_t)err;
-        slot[1] = (uint8_t)n;
-        if (n <= SWM_CIGAR_SLOT - 2) {
-            for (int q = 0; q < n; q++) slot[2 + q] = txt[q];
-        } else {
-            uint32_t at = atomicAdd(&B.tot[TOT_ARENA], (uint32_t)n);
-            if ((uint64_t)at + n <= cap_arena) {
-                for (int q = 0; q < n; q++) B.arena[at + q] = txt[q];
-                B.vr_aoff[c] = at;
-            } else {
-                atomicOr(&B.tot[TOT_FLAGS], OV_ARENA);
-            }
-        }
-        B.vr_tlen[c] = (uint16_t)n;
-        B.vr_loc[c] = ws + (uint32_t)start + 1;
-        B.vr_flag[c] = VR_TB;
-    }
+    // the last block to get here takes the walks that did not fit
+    __shared__ uint32_t s_last;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&B.tot[TOT_TBDONE], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    const uint32_t nslow = __ldcg(&B.tot[TOT_SLOW]);
+    if (nslow) traceback_slow(b2, b2_words, ref_length, B, cap_arena, nslow);
 }
 
 // ======================================================================
@@ -3361,12 +3505,13 @@ __device__ uint32_t records_seq(const MapBufs &B, uint32_t item, uint64_t cap_re
 // the same location itself). The warp reads 32 verdict flags per load, and
 // only the passing lanes read their location and CIGAR; the rest go through
 // records_seq on lane 0. Count pass: the item's record / word / byte counts;
-// write pass: the records, and the unmapped-read bits of the group.
+// write pass: the records, and the unmapped-read bits of the group; its last
+// block copies the block's totals and statistics to the host.
 template <bool WRITE>
 __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks, uint64_t cap_elems,
                                                  uint64_t cap_cands, uint64_t cap_recs, uint64_t cap_words,
-                                                 uint64_t cap_bytes) {
-    if (block_failed(B, cap_chunks, cap_elems, cap_cands)) return;
+                                                 uint64_t cap_bytes, uint32_t *h_tot, unsigned long long *h_stat) {
+    const bool failed = block_failed(B, cap_chunks, cap_elems, cap_cands);
     const uint32_t nitems = B.par->nitems, lane = lane_id();
     const uint8_t *__restrict__ vflag = B.vr_flag;
     const uint32_t *__restrict__ vloc = B.vr_loc;
@@ -3374,8 +3519,8 @@ __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks,
     const uint8_t *__restrict__ vcig = B.vr_cig;
     uint8_t *__restrict__ out_c = B.out_c;
     uint32_t *__restrict__ out_w = B.out_w;
-    unsigned long long locs_total = 0, mapped = 0;
-    for (;;) {
+    unsigned long long locs_total = 0, mapped = 0, batches = 0;
+    for (; !failed;) {
         const uint32_t item0 = warp_take(&B.tot[WRITE ? TOT_RQW : TOT_RQC]);
         if (item0 >= nitems) break;
         // the group's scalars: lane j holds item item0 + j's
@@ -3384,7 +3529,9 @@ __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks,
         bool g_ok = true;
         if (mine < nitems) {
             g_cb = B.it_coff[mine];
-            g_nc = B.it_nbat[mine] ? B.it_ncand[mine] : 0u;
+            const uint32_t nbat = B.it_nbat[mine];
+            g_nc = nbat ? B.it_ncand[mine] : 0u;
+            batches += nbat;
             if (WRITE) {
                 g_nrec = B.it_nrec[mine];
                 g_wb = B.it_woff[mine];
@@ -3496,18 +3643,22 @@ __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks,
             }
         }
     }
-    if (WRITE) {
-        warp_add_u64(&B.stat[ST_LOCS], locs_total);
-        warp_add_u64(&B.stat[ST_MAPPED], mapped);
+    if (!WRITE) {
+        warp_add_u64(&B.stat[ST_BATCHES], batches);
+        return;
     }
-}
-
-__global__ void k_batches_stat(MapBufs B) {
-    const uint32_t nitems = B.par->nitems;
-    unsigned long long s = 0;
-    for (uint32_t item = blockIdx.x * blockDim.x + threadIdx.x; item < nitems; item += gridDim.x * blockDim.x)
-        s += B.it_nbat[item];
-    warp_add_u64(&B.stat[ST_BATCHES], s);
+    warp_add_u64(&B.stat[ST_LOCS], locs_total);
+    warp_add_u64(&B.stat[ST_MAPPED], mapped);
+    // the last block to get here hands the block's totals to the host (pinned
+    // memory), which reads them once the stream has drained
+    __shared__ uint32_t s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&B.tot[TOT_RDONE], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    if (threadIdx.x < TOT_N) h_tot[threadIdx.x] = __ldcg(&B.tot[threadIdx.x]);
+    if (threadIdx.x < ST_N) h_stat[threadIdx.x] = __ldcg(&B.stat[threadIdx.x]);
 }
 
 // ======================================================================
@@ -3553,12 +3704,10 @@ static void free_bufs(MapBufs &B) {
                   B.it_coff, B.ch_g, B.ch_meta, B.bt_c0, B.bt_c1, B.bt_e0, B.bt_cnt, B.sort_scratch, B.cand_ub, B.cc_pos,
                   B.cc_item, B.plan_keys, B.vr_flag, B.vr_loc, B.vr_err, B.vr_mloc, B.vr_tlen, B.vr_cig, B.vr_aoff, B.arena, B.tb_list,
                   B.tb_cp, B.slow_list, B.vt_x, B.vt_st, B.vt_cp,
-                  B.out_w, B.out_c, B.rec_woff, B.rec_boff, B.rec_blen, B.tot, B.stat, B.scan_tmp};
+                  B.out_w, B.out_c, B.rec_woff, B.rec_boff, B.rec_blen, B.tot, B.stat, B.scan_state};
     for (void *p : ps) cudaFree(p);
     memset(&B, 0, sizeof(B));
 }
-
-static uint64_t scan_cap(const swm_mapper *m) { return m->cap_items + 1; }
 
 static unsigned cand_grid(const swm_mapper *m) { return grid_cap(m->cap_items * 32, CAND_WARPS * 32, 8); }
 
@@ -3588,9 +3737,11 @@ static int alloc_items(swm_mapper *m) {
     rc |= dmalloc(&B.it_ncand, I);
     rc |= dmalloc(&B.plan_list, I);
     rc |= dmalloc(&B.it_coff, I + 1);
-    rc |= dmalloc(&B.tot, TOT_N);
     rc |= dmalloc(&B.stat, ST_N);
+    rc |= dmalloc(&B.tot, TOT_N);
     rc |= dmalloc(&B.par, 1);
+    B.scan_tiles = (I + SCAN_TILE_ITEMS - 1) / SCAN_TILE_ITEMS;
+    rc |= dmalloc(&B.scan_state, B.scan_tiles * SCAN_VALUES);
     m->gen++;
     return rc ? SWM_ERR_OOM : SWM_OK;
 }
@@ -3604,7 +3755,7 @@ static int alloc_work(swm_mapper *m) {
     cudaFree(B.cc_item); cudaFree(B.vr_flag); cudaFree(B.vr_loc); cudaFree(B.vr_err); cudaFree(B.vr_mloc);
     cudaFree(B.vr_tlen); cudaFree(B.vr_cig); cudaFree(B.vr_aoff); cudaFree(B.arena); cudaFree(B.out_w);
     cudaFree(B.tb_list); cudaFree(B.tb_cp); cudaFree(B.slow_list); cudaFree(B.vt_x); cudaFree(B.vt_st); cudaFree(B.vt_cp);
-    cudaFree(B.out_c); cudaFree(B.rec_woff); cudaFree(B.rec_boff); cudaFree(B.rec_blen); cudaFree(B.scan_tmp);
+    cudaFree(B.out_c); cudaFree(B.rec_woff); cudaFree(B.rec_boff); cudaFree(B.rec_blen);
     rc |= dmalloc(&B.ch_g, m->cap_chunks);
     rc |= dmalloc(&B.ch_meta, m->cap_chunks);
     rc |= dmalloc(&B.plan_keys, m->cap_chunks);
@@ -3635,7 +3786,6 @@ static int alloc_work(swm_mapper *m) {
     rc |= dmalloc(&B.rec_woff, m->cap_recs);
     rc |= dmalloc(&B.rec_boff, m->cap_recs);
     rc |= dmalloc(&B.rec_blen, m->cap_recs);
-    rc |= dmalloc(&B.scan_tmp, swm_scan_tmp_words(scan_cap(m)));
     return rc ? SWM_ERR_OOM : SWM_OK;
 }
 
@@ -3727,13 +3877,12 @@ extern "C" void swm_mapper_free(swm_mapper *m) {
 // Captured into the mapper's graph; gclass picks the seed kernel.
 static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     MapBufs &B = m->b;
-    const uint32_t *d_n = &B.par->nitems;
     const uint64_t ci = m->cap_items;
+    const unsigned scan_grid = (unsigned)B.scan_tiles;
     const swm_index *ix = m->ix;
     m->launches = 0;
-    SWM_CUDA(cudaMemcpyAsync(B.par, m->h_par, sizeof(BlockParams), cudaMemcpyHostToDevice, st));
-    SWM_CUDA(cudaMemsetAsync(B.tot, 0, TOT_N * 4, st));
-    SWM_CUDA(cudaMemsetAsync(B.stat, 0, ST_N * 8, st));
+    k_begin<<<grid_cap(B.scan_tiles * SCAN_VALUES, 1024, 1), 1024, 0, st>>>(m->h_par, B);
+    m->launches++;
     // stage events: external records become event nodes of the captured graph
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[0], st, cudaEventRecordExternal));
     const uint32_t short_max = 10 * KL12 + KL12 - 1; // 164: longest read with <= 10 long seeds
@@ -3751,11 +3900,9 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     m->launches++;
     LAUNCH_CHECK();
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[1], st, cudaEventRecordExternal));
-    int rc = swm_exclusive_scan(B.it_nch, B.it_choff, d_n, 0, ci, B.scan_tmp, B.tot + TOT_CHUNKS, st);
-    if (rc) return rc;
-    rc = swm_exclusive_scan(B.it_nel, B.it_eloff, d_n, 0, ci, B.scan_tmp, B.tot + TOT_ELEMS, st);
-    if (rc) return rc;
-    m->launches += 6;
+    k_scan_items<2><<<scan_grid, 256, 0, st>>>(
+        B, ScanItems{{B.it_nch, B.it_nel}, {B.it_choff, B.it_eloff}, {TOT_CHUNKS, TOT_ELEMS}, 0, TOT_SC1});
+    m->launches++;
     k_plan_list<<<grid_cap(ci, 256, 8), 256, 0, st>>>(B, m->cap_chunks, !table);
     k_plan_lanes<<<grid_cap(ci, PLAN_LANE_WARPS * 32, 8), PLAN_LANE_WARPS * 32, 0, st>>>(ix->d_pos, B, m->cap_chunks,
                                                                                          m->cap_elems);
@@ -3773,9 +3920,8 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     m->launches++;
     LAUNCH_CHECK();
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[3], st, cudaEventRecordExternal));
-    rc = swm_exclusive_scan(B.it_ncand, B.it_coff, d_n, 0, ci, B.scan_tmp, B.tot + TOT_CANDS, st);
-    if (rc) return rc;
-    m->launches += 3;
+    k_scan_items<1><<<scan_grid, 256, 0, st>>>(B, ScanItems{{B.it_ncand}, {B.it_coff}, {TOT_CANDS}, 2, TOT_SC2});
+    m->launches++;
     k_compact<<<grid_cap(ci, 256, 8), 256, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands);
     m->launches++;
     LAUNCH_CHECK();
@@ -3805,28 +3951,19 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     k_traceback<<<grid_cap(m->cap_cands, TB_THREADS, 16), TB_THREADS, 0, st>>>(
         ix->d_b2, ix->n_words2 + SWM_PAD_WORDS, ix->ref_length, B, m->cap_chunks, m->cap_elems, m->cap_cands,
         m->cap_arena);
-    k_traceback_slow<<<grid_cap(m->cap_cands, 128, 4), 128, 0, st>>>(
-        ix->d_b2, ix->n_words2 + SWM_PAD_WORDS, ix->ref_length, B, m->cap_chunks, m->cap_elems, m->cap_cands,
-        m->cap_arena);
-    m->launches += 2;
+    m->launches++;
     LAUNCH_CHECK();
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[6], st, cudaEventRecordExternal));
-    k_records<false><<<grid_cap(ci, 128, 32), 128, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands,
-                                                             m->cap_recs, m->cap_words, m->cap_bytes);
-    rc = swm_exclusive_scan(B.it_nrec, B.it_recoff, d_n, 0, ci, B.scan_tmp, B.tot + TOT_RECS, st);
-    if (rc) return rc;
-    rc = swm_exclusive_scan(B.it_nw, B.it_woff, d_n, 0, ci, B.scan_tmp, B.tot + TOT_WORDS, st);
-    if (rc) return rc;
-    rc = swm_exclusive_scan(B.it_nb, B.it_boff, d_n, 0, ci, B.scan_tmp, B.tot + TOT_BYTES, st);
-    if (rc) return rc;
-    k_records<true><<<grid_cap(ci, 128, 32), 128, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands,
-                                                            m->cap_recs, m->cap_words, m->cap_bytes);
-    k_batches_stat<<<grid_cap(ci, 256, 8), 256, 0, st>>>(B);
-    m->launches += 12;
+    k_records<false><<<grid_cap(ci, 128, 16), 128, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands, m->cap_recs,
+                                                             m->cap_words, m->cap_bytes, nullptr, nullptr);
+    k_scan_items<3><<<scan_grid, 256, 0, st>>>(B, ScanItems{{B.it_nrec, B.it_nw, B.it_nb},
+                                                            {B.it_recoff, B.it_woff, B.it_boff},
+                                                            {TOT_RECS, TOT_WORDS, TOT_BYTES}, 3, TOT_SC3});
+    k_records<true><<<grid_cap(ci, 128, 10), 128, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands, m->cap_recs,
+                                                            m->cap_words, m->cap_bytes, m->h_tot, m->h_stat);
+    m->launches += 3;
     LAUNCH_CHECK();
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[7], st, cudaEventRecordExternal));
-    SWM_CUDA(cudaMemcpyAsync(m->h_tot, B.tot, TOT_N * 4, cudaMemcpyDeviceToHost, st));
-    SWM_CUDA(cudaMemcpyAsync(m->h_stat, B.stat, ST_N * 8, cudaMemcpyDeviceToHost, st));
     return SWM_OK;
 }
 
@@ -3925,6 +4062,10 @@ static int finish_block(swm_mapper *m, uint32_t nreads, uint64_t retries, int *a
         swm_set_error("a read is outside the envelope (length <= %d and <= stride, threshold <= %d)",
                       SWM_MAX_READ_LEN, SWM_MAX_ERRORS);
         return SWM_ERR_ARG;
+    }
+    if (fl & OV_WAIT) {
+        swm_set_error("mapping block failed: a scan tile waited too long for the tiles before it");
+        return SWM_ERR_CUDA;
     }
     // A scan total that saturated means the block's work does not fit the
     // 32-bit offsets at all. Each total is checked once the stage that feeds

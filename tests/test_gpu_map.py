@@ -534,3 +534,24 @@ def test_gpu_n_bases_in_every_place_of_a_long_seed(cuda_lib, table):
         out, m, _ = _gpu(cuda_lib, g, reads, lens, e, table=table)
         _check(out, ref.records(), ref.unmapped)
         assert m.stats()["candidates"] == ref.stats["candidates"]
+
+
+@pytest.mark.parametrize("nreads", [0, 1, 1023, 1024, 1025, 36_000])
+def test_gpu_blocks_around_the_scan_tiles(cuda_lib, nreads):
+    """Per-item offsets come from one-launch scans over tiles of 2,048 items (two
+    a read): blocks just below, at and above a tile, of none, and of more tiles
+    than a look-back step takes (32), twice on one mapper."""
+    g = genome(300_000, 41)
+    reads, lens, _, _ = synth.reads(g, max(nreads, 1), 60, 100, 0.02, seed=42, stride=100)
+    reads, lens = reads[:nreads], lens[:nreads]
+    _, mix = oracle_index(g)
+    m = cuda_lib.Mapper(cuda_lib.Index.build(g), max_reads=40_000)
+    for e in (3, 5):
+        out = m.map(reads, lens, e)
+        if nreads == 0:
+            assert out.records() == [] and len(out.unmapped) == 0
+            continue
+        ref = po.map_reads(mix, reads, lens, e, nthreads=8)
+        _check(out, ref.records(), ref.unmapped)
+        st = m.stats()
+        assert (st["candidates"], st["batches"]) == (ref.stats["candidates"], ref.stats["batches"])
