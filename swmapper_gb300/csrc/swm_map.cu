@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(SEED_WARPS * 32) k_seed(const uint32_t *__rest
 }
 
 // ======================================================================
-// k_seed12: one thread per (read, strand), k = 12
+// k_seed12: one thread per (read, strand), k = 10 .. 14
 // ======================================================================
 //
 // The same outputs as k_seed with every register array indexed at compile
@@ -564,10 +564,15 @@ __global__ void __launch_bounds__(SEED_WARPS * 32) k_seed(const uint32_t *__rest
 // the selection is then only the rank order of the long seeds, stored as a
 // permutation (sel_slot), so no lookup is repeated and no shared memory
 // limits the occupancy. The literal tail replay touches at most two 2-bit
-// words (P >= L - 11), kept in registers.
+// words (P > L - k), kept in registers. The seed length is a template argument
+// (k = 10 .. 14, 12 the usual one): a block of 50,000 reads of 155 bp with k = 13
+// took 790 us through k_seed, which has a warp per 32 items and its state in
+// shared memory, 540 us through this kernel (its seed stage 90 us).
 
 #define K12 12u
-#define KL12 15u
+#define SEED_K_MIN 10u // seed lengths with an instantiation of k_seed12
+#define SEED_K_MAX 14u
+#define SEED_SHORT_MAX(k) (10 * ((k) + SWM_SEED_STEP - 1) + (k) + SWM_SEED_STEP - 2) // longest read with 10 long seeds
 #define SEED12_THREADS 64
 // resident blocks per SM the register budget of each k_seed12 is sized for
 // (0: the compiler's choice). The short-read kernel is latency-bound on its
@@ -600,11 +605,12 @@ __device__ __forceinline__ void decode4(uint32_t w, uint32_t &lo, uint32_t &hi, 
 // 2-bit codes an N takes at each position of the seed at shift sft: d % 4
 // for d = sft + t inside the first k bases, (k - 1) % 4 past them
 // (mapper_cpe.c:1294).
-__host__ __device__ constexpr uint32_t nfill12(uint32_t sft) {
+template <uint32_t K>
+__host__ __device__ constexpr uint32_t nfill(uint32_t sft) {
     uint32_t w = 0;
-    for (uint32_t t = 0; t < K12; t++) {
+    for (uint32_t t = 0; t < K; t++) {
         const uint32_t d = sft + t;
-        w |= (d < K12 ? d % 4u : (K12 - 1u) % 4u) << (2u * t);
+        w |= (d < K ? d % 4u : (K - 1u) % 4u) << (2u * t);
     }
     return w;
 }
@@ -638,43 +644,47 @@ __device__ __forceinline__ void bucket_range(const uint32_t *__restrict__ off, u
     c = (odd ? w : v.y) - o0;
 }
 
-// Seed code of the seed at read offset o (12 bases from o) from the
+// Seed code of the seed at read offset o (K bases from o) from the
 // interleaved words w0 = word o / 16 and w1 = the next one; with N bases
-// (nk = the "not A/C/G/T" bits of bases o .. o + 11) the N positions take
-// their code nfill12(sft).
+// (nk = the "not A/C/G/T" bits of bases o .. o + K - 1) the N positions take
+// their code nfill(sft).
+template <uint32_t K>
 __device__ __forceinline__ uint32_t seed12_code(uint32_t w0, uint32_t w1, uint32_t o) {
     const uint32_t sh = 2 * (o & 15);
-    return (sh ? __funnelshift_r(w0, w1, sh) : w0) & 0xffffffu;
+    return (sh ? __funnelshift_r(w0, w1, sh) : w0) & ((1u << (2 * K)) - 1u);
 }
+template <uint32_t K>
 __device__ __forceinline__ uint32_t seed12_nfix(uint32_t sd, uint32_t nk, uint32_t sft) {
-    const uint32_t M = swm_spread16(nk & 0xfffu) * 3u;
-    return (sd & ~M) | (nfill12(sft) & M);
+    const uint32_t M = swm_spread16(nk & ((1u << K) - 1u)) * 3u;
+    return (sd & ~M) | (nfill<K>(sft) & M);
 }
 
 // Record of every seed of long seeds 0 .. NL-1 at slot 4 l + shift: (bucket
 // start, count) in rec and the flank byte rl | rh << 3 in byte 4 l + shift of
 // flw, where rl / rh are the lo / hi bits of the 3 long-seed bases outside
-// the 12-mer (set_read_long_seeds, 2474-2478). cnt gets the bucket counts summed per
+// the k-mer (set_read_long_seeds, 2474-2478). cnt gets the bucket counts summed per
 // long seed (choose_seed, 1372-1390), nref the refill chunks. Every lookup is
 // independent, so they all issue back to back. KEYS: also the long seeds' keys
 // in the candidate table (N bases of the middle 9 with their seed codes, outer
 // ones as the planes have them and named in the flank bytes' top bits).
-template <int NL, bool HASN, bool KEYS>
-__device__ __forceinline__ void seed12_records(const uint32_t (&iw)[NL], const uint32_t (&plo)[8],
+template <uint32_t K, int NL, int NW, bool HASN, bool KEYS>
+__device__ __forceinline__ void seed12_records(const uint32_t (&iw)[NW], const uint32_t (&plo)[8],
                                                const uint32_t (&phi)[8], const uint32_t (&pok)[8], uint32_t nl,
                                                const uint32_t *__restrict__ off, uint64_t pol,
                                                uint2 *__restrict__ rec, uint32_t *__restrict__ flw,
                                                uint32_t *__restrict__ keys, uint32_t (&cnt)[NL],
                                                uint32_t (&nref)[NL]) {
     static_assert(NL % 2 == 0, "flank words are stored in pairs");
+    static_assert(!KEYS || K == K12, "the candidate table is of k = 12");
+    constexpr uint32_t KL = K + SWM_SEED_STEP - 1;
     uint32_t pf = 0, pk = 0;
 #pragma unroll
     for (int l = 0; l < NL; l++) {
         const bool act = (uint32_t)l < nl;
-        const uint32_t ob = KL12 * l, wj0 = ob >> 5, sh0 = ob & 31;
+        const uint32_t ob = KL * l, wj0 = ob >> 5, sh0 = ob & 31;
         const uint32_t nlo = wj0 + 1 < 8 ? plo[wj0 + 1] : 0u, nhi = wj0 + 1 < 8 ? phi[wj0 + 1] : 0u;
-        const uint32_t lr = (sh0 ? __funnelshift_r(plo[wj0], nlo, sh0) : plo[wj0]) & 0x7fffu;
-        const uint32_t hr = (sh0 ? __funnelshift_r(phi[wj0], nhi, sh0) : phi[wj0]) & 0x7fffu;
+        const uint32_t lr = (sh0 ? __funnelshift_r(plo[wj0], nlo, sh0) : plo[wj0]) & ((1u << KL) - 1u);
+        const uint32_t hr = (sh0 ? __funnelshift_r(phi[wj0], nhi, sh0) : phi[wj0]) & ((1u << KL) - 1u);
         uint32_t csum = 0, rsum = 0, f = 0, po = 0, pc = 0;
         if (KEYS) {
             uint32_t klo = lr, khi = hr;
@@ -693,16 +703,16 @@ __device__ __forceinline__ void seed12_records(const uint32_t (&iw)[NL], const u
 #pragma unroll
         for (uint32_t sft = 0; sft < SWM_SEED_STEP; sft++) {
             const uint32_t o = ob + sft, w = o >> 4;
-            uint32_t sd = seed12_code(iw[w], (w + 1 < (uint32_t)NL) ? iw[w + 1] : 0u, o);
+            uint32_t sd = seed12_code<K>(w < (uint32_t)NW ? iw[w] : 0u, w + 1 < (uint32_t)NW ? iw[w + 1] : 0u, o);
             if (HASN) {
                 const uint32_t wj = o >> 5, s5 = o & 31;
-                const uint32_t nx = wj + 1 < 8 ? pok[wj + 1] : 0xffffffffu;
-                sd = seed12_nfix(sd, ~(s5 ? __funnelshift_r(pok[wj], nx, s5) : pok[wj]), sft);
+                const uint32_t nt = wj < 8 ? pok[wj] : 0xffffffffu, nx = wj + 1 < 8 ? pok[wj + 1] : 0xffffffffu;
+                sd = seed12_nfix<K>(sd, ~(s5 ? __funnelshift_r(nt, nx, s5) : nt), sft);
             }
             sd = act ? sd : 0u;
             uint32_t o0, c;
             bucket_range(off, sd, pol, o0, c);
-            const uint32_t m = (1u << sft) - 1, kk = K12 + sft;
+            const uint32_t m = (1u << sft) - 1, kk = K + sft;
             const uint32_t rl = ((lr & m) | ((lr >> kk) << sft)) & 7u;
             const uint32_t rh = ((hr & m) | ((hr >> kk) << sft)) & 7u;
             if (sft & 1) // two records per 16-byte store
@@ -720,13 +730,15 @@ __device__ __forceinline__ void seed12_records(const uint32_t (&iw)[NL], const u
     }
 }
 
-template <int NL, bool TABLE>
+template <uint32_t K, int NL, bool TABLE>
 // Items whose read length is outside [lo_len, hi_len] belong to the other
-// instantiation launched beside this one (reads of up to 164 bases take the
+// instantiation launched beside this one (reads of up to SEED_SHORT_MAX bases take the
 // 10-long-seed kernel, longer ones the 16-long-seed kernel). TABLE: the
 // candidate table is in use, so each long seed's table key is stored too.
 __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs B,
                                                            uint32_t lo_len, uint32_t hi_len) {
+    constexpr uint32_t KL = K + SWM_SEED_STEP - 1;
+    constexpr int NW = (NL * KL + 15) / 16 < 16 ? (NL * KL + 15) / 16 : 16; // 2-bit words the seeds lie in
     const BlockParams P = *B.par;
     const char *__restrict__ reads = P.reads;
     const uint32_t *__restrict__ lens = P.lens;
@@ -746,7 +758,7 @@ __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs
         const uint32_t L = lens[r];
         if (L < lo_len || L > hi_len) continue; // both lanes of the read skip it
         const uint32_t e = e_arr ? e_arr[r] : e_glob;
-        if (L > SWM_MAX_READ_LEN || L > stride || e > SWM_MAX_ERRORS || L > NL * KL12 + KL12 - 1) {
+        if (L > SWM_MAX_READ_LEN || L > stride || e > SWM_MAX_ERRORS || L > NL * KL + KL - 1) {
             atomicOr(&B.tot[TOT_FLAGS], OV_BAD);
             B.it_nsel[item] = 0;
             B.it_e[item] = 0;
@@ -845,20 +857,20 @@ __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs
                 pok[b] = ok;
             }
         }
-        const uint32_t nl = L / KL12;
-        uint32_t jt = 0xffffffffu, P = nl ? nl * KL12 - 1 : 0u;
+        const uint32_t nl = L / KL;
+        uint32_t jt = 0xffffffffu, P = nl ? nl * KL - 1 : 0u;
         if (nl) {
 #pragma unroll
             for (uint32_t sft = 0; sft < SWM_SEED_STEP; sft++) {
-                const uint32_t rp = (nl - 1) * KL12 + sft + K12 - 1;
-                if (jt == 0xffffffffu && L - rp < K12) {
+                const uint32_t rp = (nl - 1) * KL + sft + K - 1;
+                if (jt == 0xffffffffu && L - rp < K) {
                     jt = (nl - 1) * SWM_SEED_STEP + sft;
                     P = rp;
                 }
             }
         }
-        const uint32_t vis = nl ? (jt != 0xffffffffu ? L : nl * KL12) : 0u;
-        const uint32_t span = nl * KL12;
+        const uint32_t vis = nl ? (jt != 0xffffffffu ? L : nl * KL) : 0u;
+        const uint32_t span = nl * KL;
         bool has_n = false;
 #pragma unroll
         for (int b = 0; b < 8; b++) { // planes hold the visited bases only; N flag over seed windows
@@ -873,9 +885,9 @@ __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs
         }
         // ---- interleaved 2-bit words of the strand (base 16 w + i at bits
         // 2i, 2i + 1)
-        uint32_t iw[NL];
+        uint32_t iw[NW];
 #pragma unroll
-        for (int w = 0; w < NL; w++) {
+        for (int w = 0; w < NW; w++) {
             const uint32_t l16 = (w & 1) ? (plo[w >> 1] >> 16) : plo[w >> 1];
             const uint32_t h16 = (w & 1) ? (phi[w >> 1] >> 16) : phi[w >> 1];
             iw[w] = swm_spread16(l16) | (swm_spread16(h16) << 1);
@@ -925,7 +937,7 @@ __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs
             if (P % 16 != 15)
                 for (uint32_t q = base0; q <= P; q++) acc |= code_at(q) << ((q % 16) * 2);
             for (uint32_t j = jt; j < nl * SWM_SEED_STEP; j++) {
-                const uint32_t rp = (j / SWM_SEED_STEP) * KL12 + j % SWM_SEED_STEP + K12 - 1;
+                const uint32_t rp = (j / SWM_SEED_STEP) * KL + j % SWM_SEED_STEP + K - 1;
                 if (j > jt) { // the one base this call's main loop adds
                     acc |= code_at(rp) << ((rp % 16) * 2);
                     if (rp % 16 == 15) {
@@ -973,8 +985,8 @@ __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs
         uint32_t CNT[NL], IDX[NL], REF[NL];
         uint32_t *flw = reinterpret_cast<uint32_t *>(B.sel_fl + sb);
         uint32_t *keys = B.sel_key + (uint64_t)item * (SWM_MAX_SEL / SWM_SEED_STEP);
-        if (has_n) seed12_records<NL, true, TABLE>(iw, plo, phi, pok, nl, off, pol, sel + sb, flw, keys, CNT, REF);
-        else seed12_records<NL, false, TABLE>(iw, plo, phi, pok, nl, off, pol, sel + sb, flw, keys, CNT, REF);
+        if (has_n) seed12_records<K, NL, NW, true, TABLE>(iw, plo, phi, pok, nl, off, pol, sel + sb, flw, keys, CNT, REF);
+        else seed12_records<K, NL, NW, false, TABLE>(iw, plo, phi, pok, nl, off, pol, sel + sb, flw, keys, CNT, REF);
 #pragma unroll
         for (int l = 0; l < NL; l++) IDX[l] = l;
         // exchange sort (1391-1399), unrolled
@@ -1895,7 +1907,7 @@ struct CandTabSmem {
 // Table key of the seed at shift sft of a long seed: 4 key15 + sft. Outer bases
 // of the 15-mer that are N (mask in bits 6-7 of the long seed's flank bytes:
 // the 3 first, then the 3 last) take their seed code where the shift's 12-mer
-// holds them (nfill12: d % 4 for base d < 12, then 3) and keep the plane's
+// holds them (nfill: d % 4 for base d < 12, then 3) and keep the plane's
 // elsewhere.
 __device__ __forceinline__ uint32_t ctab_slot_key(uint32_t key15, uint32_t flanks, uint32_t sft) {
     if (flanks & 0x00c0c0c0u) {
@@ -3885,10 +3897,12 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     m->launches++;
     // stage events: external records become event nodes of the captured graph
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[0], st, cudaEventRecordExternal));
-    const uint32_t short_max = 10 * KL12 + KL12 - 1; // 164: longest read with <= 10 long seeds
+    const uint32_t short_max = SEED_SHORT_MAX(ix->k);
     const bool table = ix->d_ctab_off && ix->k == K12;
-    auto seed10 = table ? k_seed12<10, true> : k_seed12<10, false>;
-    auto seed16 = table ? k_seed12<16, true> : k_seed12<16, false>;
+    auto seed10 = table ? k_seed12<12, 10, true> : ix->k == 10 ? k_seed12<10, 10, false> : ix->k == 11 ? k_seed12<11, 10, false>
+                : ix->k == 13 ? k_seed12<13, 10, false> : ix->k == 14 ? k_seed12<14, 10, false> : k_seed12<12, 10, false>;
+    auto seed16 = table ? k_seed12<12, 16, true> : ix->k == 10 ? k_seed12<10, 16, false> : ix->k == 11 ? k_seed12<11, 16, false>
+                : ix->k == 13 ? k_seed12<13, 16, false> : ix->k == 14 ? k_seed12<14, 16, false> : k_seed12<12, 16, false>;
     if (gclass == 1) {
         seed10<<<grid_cap(ci, SEED12_THREADS, 16), SEED12_THREADS, 0, st>>>(ix->d_off, B, 0u, 0xffffffffu);
     } else if (gclass == 2) { // each read to the instantiation of its length
@@ -3977,7 +3991,7 @@ static void drop_graph(swm_mapper *m, int gclass, int h) {
 // synchronisation.
 static int enqueue(swm_mapper *m, const char *d_reads, const uint32_t *d_lens, uint64_t stride, uint32_t nreads,
                    uint32_t errors, const uint8_t *d_e) {
-    const int gclass = m->ix->k != K12 ? 0 : (stride <= 10 * KL12 + KL12 - 1 ? 1 : 2);
+    const int gclass = m->ix->k < SEED_K_MIN || m->ix->k > SEED_K_MAX ? 0 : (stride <= SEED_SHORT_MAX(m->ix->k) ? 1 : 2);
     BlockParams *P = m->h_par;
     P->reads = d_reads;
     P->lens = d_lens;

@@ -555,3 +555,32 @@ def test_gpu_blocks_around_the_scan_tiles(cuda_lib, nreads):
         _check(out, ref.records(), ref.unmapped)
         st = m.stats()
         assert (st["candidates"], st["batches"]) == (ref.stats["candidates"], ref.stats["batches"])
+
+
+@pytest.mark.parametrize("k", [9, 10, 11, 13, 14])
+def test_gpu_seed_kernels_of_other_lengths(cuda_lib, k):
+    """k = 10 .. 14 share the register seed kernel, other k the general one: read
+    lengths at the edges of both of its instantiations (10 long seeds, 16) and of
+    long seeds, N and lowercase bases, and the recorded encodings."""
+    kl = k + 3
+    top = min(254, 17 * kl - 1)
+    short = 10 * kl + kl - 1
+    g = genome(300_000, 51, "repeats100m", copies_per_family=30, rep_len_max=2000)
+    edges = [x for b in (kl, 2 * kl, 5 * kl, 10 * kl, short, short + 1, 13 * kl, top) for x in (b - 1, b, b + 1, b + k - 2)
+             if 15 <= x <= top]
+    for stride in (min(short, top), top):
+        reads, lens, _, _ = synth.reads(g, 800, 30, stride, 0.02, seed=52, stride=stride)
+        for i, L in enumerate(edges):
+            if L <= stride:
+                lens[i::len(edges)] = np.minimum(lens[i::len(edges)], L)
+        reads[::4, 3] = ord("N")
+        reads[1::4, 11] = ord("n")
+        reads[2::4, 17] = ord("N")
+        ix = cuda_lib.Index.build(g, k=k)
+        mix = po.MapIndex(po.build_index(g, k))
+        m = cuda_lib.Mapper(ix, max_reads=800)
+        for e in (2, 9):
+            out = m.map(reads, lens, e)
+            ref = po.map_reads(mix, reads, lens, e, nthreads=8)
+            _check(out, ref.records(), ref.unmapped)
+            assert m.stats()["candidates"] == ref.stats["candidates"]
