@@ -45,6 +45,11 @@ struct swm_index {
     // contiguous, position-ordered range, next to those of the other shifts.
     uint32_t *d_ctab_off;  // SWM_CTAB_KEYS + 1 start offsets into d_ctab_pos
     uint32_t *d_ctab_pos;  // 4 * n_seeds (+8) positions
+    // Heap keys of the refill schedule (indexes of large buckets; device-only):
+    // word g / 32 holds pos[g] for every entry g that ends a fetch of 32 of a
+    // bucket with entries left after it (g = start + 32 j + 31, so a bucket's keys
+    // are consecutive words and no two buckets share one)
+    uint32_t *d_keys32;    // n_seeds / 32 + 1
     uint32_t ctab_gen;     // bumped whenever the table is built or dropped
     int ctab_off;          // the caller dropped the table: no automatic build
     // swm_index_serialize_mappers: when chain is set, every mapper of this
@@ -82,6 +87,10 @@ __host__ __device__ __forceinline__ uint32_t swm_ctab_flank(uint32_t ls, uint32_
 // indexes averaging SWM_CTAB_MIN_MEAN or more entries per bucket).
 #define SWM_CTAB_MIN_MEAN 8
 int swm_ctab_build(swm_index *ix, int forced);
+// Build the refill keys when they are missing and the buckets average
+// SWM_CTAB_MIN_MEAN entries (swm_index.cu); without room for them the planners
+// read the position array.
+int swm_keys32_build(swm_index *ix);
 
 // Exclusive scan of n u32 values (n read from *d_n when d_n is not NULL,
 // else n_host; clamped to n_cap); out gets n + 1 entries, out[n] = total,

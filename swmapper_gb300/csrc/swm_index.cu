@@ -605,6 +605,19 @@ __global__ void __launch_bounds__(CTAB_THREADS, 3) kb_ctab(const uint32_t *__res
     }
 }
 
+// ------------------------------------------------------ refill schedule keys
+
+// one thread per bucket (most have a few keys; a large one's are 128 bytes
+// apart, so its thread's reads are no worse than others')
+__global__ void __launch_bounds__(256) kb_keys32(const uint32_t *__restrict__ off, uint64_t nb,
+                                                 const uint32_t *__restrict__ pos, uint32_t *__restrict__ keys) {
+    for (uint64_t b = (uint64_t)blockIdx.x * 256 + threadIdx.x; b < nb; b += (uint64_t)gridDim.x * 256) {
+        const uint32_t end = off[b + 1];
+        for (uint64_t g = (uint64_t)off[b] + SWM_PER_FETCH - 1; g + 1 < end; g += SWM_PER_FETCH)
+            keys[g / SWM_PER_FETCH] = pos[g];
+    }
+}
+
 // ----------------------------------------------------------- host helpers
 
 static int sm_count(int device) {
@@ -625,6 +638,7 @@ static void index_release(swm_index *ix) {
     if (ix->chain_ev) cudaEventDestroy(ix->chain_ev);
     cudaFree(ix->d_ctab_off);
     cudaFree(ix->d_ctab_pos);
+    cudaFree(ix->d_keys32);
     if (ix->arena) { // a built index: its arrays are parts of one allocation
         cudaFree(ix->arena);
     } else {
@@ -1145,6 +1159,28 @@ int swm_ctab_build(swm_index *ix, int forced) {
     ix->d_ctab_off = d_o;
     ix->d_ctab_pos = d_p;
     ix->ctab_gen++;
+    return SWM_OK;
+}
+
+int swm_keys32_build(swm_index *ix) {
+    std::lock_guard<std::mutex> lk(g_ctab_mu);
+    if (ix->d_keys32 || ix->n_seeds < (uint64_t)SWM_CTAB_MIN_MEAN << (2 * ix->k)) return SWM_OK;
+    SWM_CUDA(cudaSetDevice(ix->device));
+    uint32_t *d = nullptr;
+    if (cudaMalloc(&d, (ix->n_seeds / SWM_PER_FETCH + 1) * 4) != cudaSuccess) {
+        cudaGetLastError();
+        return SWM_OK;
+    }
+    const uint64_t nb = 1ull << (2 * ix->k);
+    kb_keys32<<<grid_for(nb, 256, ix->device, 8), 256>>>(ix->d_off, nb, ix->d_pos, d);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) {
+        cudaFree(d);
+        swm_set_error("building the refill keys: %s", cudaGetErrorString(e));
+        return SWM_ERR_CUDA;
+    }
+    ix->d_keys32 = d;
     return SWM_OK;
 }
 

@@ -58,8 +58,9 @@ enum {
     TOT_CHUNKS = 0, TOT_ELEMS, TOT_CANDS, TOT_RECS, TOT_WORDS, TOT_BYTES, TOT_ARENA, TOT_FLAGS, TOT_TB, TOT_SLOW,
     TOT_VQ, TOT_TBQ, // work-queue heads of k_verify and k_traceback
     TOT_VT, TOT_VTQ, // candidates alive after the head of verification, and their queue head
-    TOT_PLN, TOT_PLQ,  // items with refills and at most 32 selected seeds, queue head of k_plan_lanes
-    TOT_PLW, TOT_PLWQ, // items with refills and more selected seeds, queue head of k_plan
+    TOT_PLN, TOT_PLQ,  // items with several batches, short schedules of at most 32 seeds; queue head of k_plan_lanes
+    TOT_PLM, TOT_PLMQ, // the same with more selected seeds
+    TOT_PLW, TOT_PLWQ, // and those with long schedules; queue head of k_plan
     TOT_CQ,            // queue head of the candidate stage (items)
     TOT_RQC, TOT_RQW,  // queue heads of the records count and write passes (groups of 32 items)
     TOT_SC1, TOT_SC2, TOT_SC3, // tile tickets of the scans after the seed, candidate and records-count stages
@@ -127,7 +128,8 @@ struct MapBufs {
     uint32_t *it_nrec, *it_nw, *it_nb;
     uint32_t *it_recoff, *it_woff, *it_boff; // items + 1
     uint32_t *it_ncand, *it_coff;            // candidates per item, dense offsets (items + 1)
-    uint32_t *plan_list; // items with refills: k_plan_lanes' from the front, k_plan's from the back (items)
+    uint32_t *plan_list; // items with several batches: of few seeds from the front, long schedules from the back
+    uint32_t *plan_more; // (items each) and of more seeds
     // per chunk / batch slot (cap_chunks; batch b of an item sits at slot it_choff + b)
     uint32_t *ch_g, *ch_meta;
     uint32_t *bt_c0, *bt_c1, *bt_e0, *bt_cnt; // cap_chunks + cap_items slots
@@ -208,6 +210,8 @@ struct swm_mapper {
     uint32_t tot[TOT_N];
     swm_map_stats stats;
     cudaEvent_t ev[9];
+    cudaStream_t side[2];      // branches of the captured pipeline (the planners)
+    cudaEvent_t fork, join[2];
     float stage_ms[8];
     uint64_t launches;
     // the block's launch sequence, captured once per buffer set and read
@@ -1049,6 +1053,16 @@ __device__ __forceinline__ uint32_t warp_scan_incl(uint32_t v) {
     return v;
 }
 
+// Heap key of a seed whose next entry to fetch is cu (it has some left): the
+// position of the entry before it. From the key array a bucket's keys are
+// neighbours (eight a sector) and all of them 3% of the position array, where
+// each is a DRAM burst of its own (k_plan_lanes ran at the device's rate for
+// random reads: 490 us, against 380, for 524,288 reads on 3.1 Gbp).
+__device__ __forceinline__ uint32_t refill_key(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ keys32,
+                                               uint32_t cu) {
+    return keys32 ? keys32[(cu - 1) / SWM_PER_FETCH] : pos[cu - 1];
+}
+
 // Start of a block: its inputs from the pinned parameter block (read in place)
 // to B.par, and the totals, statistics and scan states cleared.
 __global__ void __launch_bounds__(1024) k_begin(const BlockParams *__restrict__ h, MapBufs B) {
@@ -1182,11 +1196,18 @@ __global__ void __launch_bounds__(256) k_scan_items(MapBufs B, ScanItems A) {
     }
 }
 
-// The items whose selected buckets need refills, compacted into the planners'
+// The items whose refills span several batches, compacted into the planners'
 // work lists (warp-aggregated appends; order does not matter, items are
-// independent): items with at most PLAN_LANE_SEEDS selected seeds from the
-// front for k_plan_lanes, the others from the back for k_plan.
+// independent): those of at most PLAN_LANE_REFILLS refills for k_plan_lanes, by
+// their number of seeds (its shared memory is sized by it), the others for
+// k_plan. A refill takes a lane some 1,000 cycles, and a warp of k_plan 200 but
+// ten times the issue slots: the many short schedules go to lanes, and the
+// few long ones, which would be the tail of the stage, to warps.
 #define PLAN_LANE_SEEDS 32
+#ifndef PLAN_LANE_REFILLS
+#define PLAN_LANE_REFILLS 512
+#endif
+__device__ __forceinline__ bool several_batches(uint32_t nref, uint32_t nel) { return nref && !single_batch(nref, nel); }
 // chunks: write the refill chunks of the single-batch items (the candidate
 // kernel without the candidate table gathers from them; k_cand_table reads
 // chunks only of items with several batches).
@@ -1195,18 +1216,25 @@ __global__ void __launch_bounds__(256) k_plan_list(MapBufs B, uint64_t cap_chunk
     const uint32_t lane = lane_id();
     for (uint32_t base = blockIdx.x * 256 + (threadIdx.x & ~31u); base < nitems; base += gridDim.x * 256) {
         const uint32_t item = base + lane;
-        const bool has = item < nitems && B.it_nch[item] != 0 && B.it_nbat[item] == 0;
-        const bool few = has && B.it_nsel[item] <= PLAN_LANE_SEEDS;
-        const uint32_t mf = __ballot_sync(0xffffffffu, few), mm = __ballot_sync(0xffffffffu, has && !few);
-        uint32_t af = 0, am = 0;
-        if (lane == 0 && mf) af = atomicAdd(&B.tot[TOT_PLN], (uint32_t)__popc(mf));
-        if (lane == 0 && mm) am = atomicAdd(&B.tot[TOT_PLW], (uint32_t)__popc(mm));
-        af = __shfl_sync(0xffffffffu, af, 0);
-        am = __shfl_sync(0xffffffffu, am, 0);
-        if (few) B.plan_list[af + __popc(mf & lanemask_lt())] = item;
-        if (has && !few) B.plan_list[nitems - 1 - (am + __popc(mm & lanemask_lt()))] = item;
+        const bool has = item < nitems && several_batches(B.it_nch[item], B.it_nel[item]);
+        const bool lng = has && B.it_nch[item] > PLAN_LANE_REFILLS;
+        const bool few = has && !lng && B.it_nsel[item] <= PLAN_LANE_SEEDS, more = has && !lng && !few;
+        if (__any_sync(0xffffffffu, has)) {
+            const uint32_t mf = __ballot_sync(0xffffffffu, few), mm = __ballot_sync(0xffffffffu, more),
+                           ml = __ballot_sync(0xffffffffu, lng);
+            uint32_t at = 0;
+            if (lane == 0 && mf) at = atomicAdd(&B.tot[TOT_PLN], (uint32_t)__popc(mf));
+            if (lane == 1 && mm) at = atomicAdd(&B.tot[TOT_PLM], (uint32_t)__popc(mm));
+            if (lane == 2 && ml) at = atomicAdd(&B.tot[TOT_PLW], (uint32_t)__popc(ml));
+            const uint32_t af = __shfl_sync(0xffffffffu, at, 0), am = __shfl_sync(0xffffffffu, at, 1),
+                           al = __shfl_sync(0xffffffffu, at, 2);
+            if (few) B.plan_list[af + __popc(mf & lanemask_lt())] = item;
+            if (more) B.plan_more[am + __popc(mm & lanemask_lt())] = item;
+            if (lng) B.plan_list[nitems - 1 - (al + __popc(ml & lanemask_lt()))] = item;
+        }
         // items whose refills all fit in one batch (single_batch) need no heap:
-        // the warp writes their refill chunks seed by seed and the batch record
+        // the warp writes their refill chunks seed by seed
+        if (!chunks) continue;
         uint32_t one = __ballot_sync(0xffffffffu, item < nitems && B.it_nch[item] != 0 && B.it_nbat[item] == 1);
         while (one) {
             const uint32_t it = base + __ffs(one) - 1;
@@ -1222,7 +1250,7 @@ __global__ void __launch_bounds__(256) k_plan_list(MapBufs B, uint64_t cap_chunk
             const unsigned long long perm = B.it_perm[it];
             const uint64_t sb = (uint64_t)it * SWM_MAX_SEL;
             uint32_t q = 0;
-            for (uint32_t i0 = 0; chunks && i0 < ns; i0 += 32) {
+            for (uint32_t i0 = 0; i0 < ns; i0 += 32) {
                 const uint32_t i = i0 + lane;
                 const uint2 sv = i < ns ? B.sel[sb + sel_slot(perm, i)] : make_uint2(0u, 0u);
                 const uint32_t r = sv.y > SWM_PER_FETCH ? (sv.y - 1) / SWM_PER_FETCH : 0u;
@@ -1235,36 +1263,50 @@ __global__ void __launch_bounds__(256) k_plan_list(MapBufs B, uint64_t cap_chunk
                 }
                 q += __shfl_sync(0xffffffffu, rinc, 31);
             }
-            if (lane == 0) {
-                const uint32_t sbase = rb + it;
-                B.bt_c0[sbase] = rb; // batch 0 also holds every initial chunk
-                B.bt_c1[sbase] = rb + nref;
-                B.bt_e0[sbase] = B.it_eloff[it];
-            }
         }
     }
 }
 
 #define PLAN_WARPS 4
-#define PLAN_KEYS 512 // heap keys of an item held in shared memory; more go to global scratch
+#define PLAN_KEYS 2048 // heap keys of an item held in shared memory; more go to global scratch
 
 struct PlanSmem {
-    uint32_t sst[SWM_MAX_SEL], scn[SWM_MAX_SEL], pc[SWM_MAX_SEL], koff[SWM_MAX_SEL + 1];
-    uint32_t hloc[SWM_MAX_SEL + 8], hidx[SWM_MAX_SEL + 8];
+    uint4 seed[SWM_MAX_SEL];        // next position to fetch, end of the bucket, index of the next key, next key
+    uint32_t koff[SWM_MAX_SEL + 1]; // index of each seed's first key
     uint32_t key[PLAN_KEYS];
 };
 
-// One warp per item whose buckets need refills (a warp looks at 32 items at
-// a time and takes those with refills one by one). The heap keys (the raw
-// position of the last element of every chunk that leaves a seed with
-// positions to fetch: pos[start + 32 (j + 1) - 1] for refill j) are all
-// known up front, so the lanes load them in parallel; lane 0 then runs the
-// seed heap of alignment_rmdup (2194-2419) on shared memory only.
-__global__ void __launch_bounds__(PLAN_WARPS * 32) k_plan(const uint32_t *__restrict__ pos, MapBufs B,
+// One warp per item. The heap keys (the raw position of the last element of
+// every chunk that leaves a seed with positions to fetch: pos[start + 32 (j + 1)
+// - 1] for refill j) are all known up front, so the lanes load them in parallel.
+// The seed heap of alignment_rmdup (2194-2419) then lives in registers, node
+// p + 1 of the reference in lane p % 32 (k0, k1: keys of places p and p + 32; i0,
+// i1: their seeds), and a pop is a handful of votes and shuffles instead of a
+// walk: which child of every node is the smaller is one comparison per lane
+// (kept as a mask); a place is on the path from the root along smaller children
+// when the mask holds all its ancestors; the new root key sinks along the path
+// to the first place whose key is not below it, and the places passed move up
+// by one shuffle. (One lane walking a heap in shared memory, for every item of
+// more than 32 seeds, took 0.83 ms of the 1.08 ms stage for 65,536 uneven reads on
+// 3.1 Gbp; with this kernel for the long items and lanes for the others the
+// stage takes 0.36.) The sift's loop bound is the reference's (q * 2 < size,
+// 1946).
+__global__ void __launch_bounds__(PLAN_WARPS * 32) k_plan(const uint32_t *__restrict__ pos,
+                                                          const uint32_t *__restrict__ keys32, MapBufs B,
                                                           uint64_t cap_chunks, uint64_t cap_elems) {
     __shared__ PlanSmem sm_all[PLAN_WARPS];
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
     PlanSmem &S = sm_all[wib];
+    typedef unsigned long long u64;
+    // place p and its ancestors without the root, as a mask, for p = lane and lane + 32
+    u64 anc0 = 0, anc1 = 0;
+    for (uint32_t p = lane; p; p = (p - 1) >> 1) anc0 |= 1ull << p;
+    for (uint32_t p = lane + 32; p; p = (p - 1) >> 1) anc1 |= 1ull << p;
+    const bool left = lane & 1; // odd places are left children (in both halves)
+    const uint32_t sib = (left ? lane + 1 : lane - 1) & 31, up0 = (lane - 1) >> 1, up1 = (lane + 31) >> 1; // sibling, parents
+    auto both = [](bool a, bool b) { // a mask over the 64 places
+        return (u64)__ballot_sync(0xffffffffu, a) | (u64)__ballot_sync(0xffffffffu, b) << 32;
+    };
     // warps take the items with refills one at a time from the list k_plan_list
     // built: a heavy item (a read in a large repeat family has thousands of
     // refills) keeps one warp, and the others move on
@@ -1288,21 +1330,23 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32) k_plan(const uint32_t *__rest
         const uint32_t ns = B.it_nsel[item];
         const uint64_t sb = (uint64_t)item * SWM_MAX_SEL;
         const unsigned long long perm = B.it_perm[item];
-        // seed records in rank order and the offsets of their keys
-        uint32_t carry = 0;
+        // seed records in rank order, the initial fetch (2194-2236) and the
+        // offsets of their keys
+        uint32_t carry = 0, e = 0, runs = 0;
         for (uint32_t i0 = 0; i0 < ns; i0 += 32) {
             const uint32_t i = i0 + lane;
-            uint32_t r = 0;
+            uint32_t r = 0, pc = 0;
             if (i < ns) {
                 const uint2 sv = B.sel[sb + sel_slot(perm, i)];
-                S.sst[i] = sv.x;
-                S.scn[i] = sv.y;
-                S.pc[i] = sv.y > SWM_PER_FETCH ? SWM_PER_FETCH : sv.y; // initial fetch, 2194-2236
+                pc = sv.y > SWM_PER_FETCH ? SWM_PER_FETCH : sv.y;
                 r = sv.y > SWM_PER_FETCH ? (sv.y - 1) / SWM_PER_FETCH : 0u;
+                S.seed[i] = make_uint4(sv.x + pc, sv.x + sv.y, 0u, 0u);
             }
             const uint32_t inc = warp_scan_incl(r);
             if (i < ns) S.koff[i] = carry + inc - r;
             carry += __shfl_sync(0xffffffffu, inc, 31);
+            e += __reduce_add_sync(0xffffffffu, pc);
+            runs += __popc(__ballot_sync(0xffffffffu, pc != 0));
         }
         if (lane == 0) S.koff[ns] = carry; // == nref
         __syncwarp();
@@ -1314,95 +1358,125 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32) k_plan(const uint32_t *__rest
                 if (S.koff[mid] <= c) lo = mid;
                 else hi = mid;
             }
-            const uint32_t j = c - S.koff[lo];
-            keys[c] = pos[S.sst[lo] + SWM_PER_FETCH * (j + 1) - 1];
+            keys[c] = refill_key(pos, keys32, S.seed[lo].x + SWM_PER_FETCH * (c - S.koff[lo]));
         }
         __syncwarp();
-        if (lane == 0) {
-            uint32_t hs = 0, rc = 0, e = 0, b = 0, br0 = 0, be0 = 0, npos = 0, runs = 0;
-            for (uint32_t i = 0; i < ns; i++) {
-                e += S.pc[i];
-                npos += S.pc[i];
-                runs += S.pc[i] ? 1u : 0u;
+        for (uint32_t i = lane; i < ns; i += 32) // the key a seed goes back into the heap with after its first pop
+            S.seed[i].z = S.koff[i] + 1;
+        __syncwarp();
+        for (uint32_t i = lane; i < ns; i += 32) S.seed[i].w = S.koff[i + 1] > S.koff[i] + 1 ? keys[S.koff[i] + 1] : 0u;
+        __syncwarp();
+        // ---- seeds_heap_insert (1919-1935) of the seeds with positions left, in
+        // seed order: the ancestors of the new place above the key move down
+        uint32_t k0 = 0, k1 = 0, i0 = 0, i1 = 0, hs = 0;
+        for (uint32_t i = 0; i < ns; i++) {
+            if (S.koff[i + 1] == S.koff[i]) continue;
+            const uint32_t x = keys[S.koff[i]], q = hs++;
+            u64 anc = 0; // ancestors of place q
+            for (uint32_t p = q; p;) {
+                p = (p - 1) >> 1;
+                anc |= 1ull << p;
             }
-            auto key_of = [&](uint32_t i) { return keys[S.koff[i] + S.pc[i] / SWM_PER_FETCH - 1]; };
-            for (uint32_t i = 0; i < ns; i++) { // seeds_heap_insert, 1919-1935 (keys: raw positions)
-                if (S.pc[i] != S.scn[i]) {
-                    hs++;
-                    S.hloc[hs] = key_of(i);
-                    S.hidx[hs] = i;
-                    uint32_t q = hs;
-                    while (q > 1) {
-                        const uint32_t t = q / 2;
-                        if (S.hloc[t] > S.hloc[q]) {
-                            uint32_t a = S.hloc[t];
-                            S.hloc[t] = S.hloc[q];
-                            S.hloc[q] = a;
-                            a = S.hidx[t];
-                            S.hidx[t] = S.hidx[q];
-                            S.hidx[q] = a;
-                        } else break;
-                        q = t;
-                    }
-                }
+            const u64 stay = anc & ~both(k0 > x, k1 > x);
+            const u64 move = stay ? anc & ~((2ull << (63 - __clzll(stay))) - 1) : anc; // below the deepest that stays
+            const u64 path = anc | 1ull << q;
+            const uint32_t pk0 = __shfl_sync(0xffffffffu, k0, up0), pi0 = __shfl_sync(0xffffffffu, i0, up0);
+            const uint32_t pk1 = __shfl_sync(0xffffffffu, k0, up1), pi1 = __shfl_sync(0xffffffffu, i0, up1);
+            const uint32_t dest = move ? __ffsll(move) - 1 : q; // the highest place that moved, or the new one
+            if (lane && (path >> lane & 1) && (move >> up0 & 1)) {
+                k0 = pk0;
+                i0 = pi0;
             }
-            for (;;) { // 2261-2419
-                if (hs > 0 && npos + SWM_PER_FETCH <= SWM_BATCH_POSITIONS && 1 + 2 * runs < SWM_MAX_RUNS_BLOCK) {
-                    const uint32_t i = S.hidx[1];
-                    const uint32_t left = S.scn[i] - S.pc[i];
-                    const uint32_t get = left > SWM_PER_FETCH ? SWM_PER_FETCH : left;
-                    B.ch_g[rb + rc] = S.sst[i] + S.pc[i];
+            if ((path >> (lane + 32) & 1) && (move >> up1 & 1)) {
+                k1 = pk1;
+                i1 = pi1;
+            }
+            if (dest == lane) {
+                k0 = x;
+                i0 = i;
+            }
+            if (dest == lane + 32) {
+                k1 = x;
+                i1 = i;
+            }
+        }
+        // ---- refills and batches (2261-2419)
+        uint32_t rc = 0, b = 0, br0 = 0, be0 = 0, npos = e;
+        for (;;) {
+            if (hs > 0 && npos + SWM_PER_FETCH <= SWM_BATCH_POSITIONS && 1 + 2 * runs < SWM_MAX_RUNS_BLOCK) {
+                // the smaller child of every node the sift may look at (from the keys alone)
+                const uint32_t a0 = __shfl_sync(0xffffffffu, lane == 0 ? k1 : k0, sib);
+                const uint32_t a1 = __shfl_sync(0xffffffffu, lane == 31 ? k0 : k1, sib);
+                const uint32_t i = __shfl_sync(0xffffffffu, i0, 0);
+                const uint4 sd = S.seed[i];
+                const uint32_t have = sd.y - sd.x, get = have > SWM_PER_FETCH ? SWM_PER_FETCH : have;
+                if (lane == 0) {
+                    B.ch_g[rb + rc] = sd.x;
                     B.ch_meta[rb + rc] = get | (i << 8);
-                    rc++;
-                    S.pc[i] += get;
-                    e += get;
-                    npos += get;
-                    runs++;
-                    // seeds_heap_pop_and_insert, 1936-1962 (loop bound i * 2 < size)
-                    if (S.pc[i] == S.scn[i]) {
-                        S.hloc[1] = S.hloc[hs];
-                        S.hidx[1] = S.hidx[hs];
-                        hs--;
-                    } else {
-                        S.hloc[1] = key_of(i);
-                    }
-                    uint32_t q = 1;
-                    while (q * 2 < hs) {
-                        uint32_t t = q * 2;
-                        if (q * 2 + 1 <= hs && S.hloc[q * 2] > S.hloc[q * 2 + 1]) t = q * 2 + 1;
-                        if (S.hloc[t] < S.hloc[q]) {
-                            uint32_t a = S.hloc[t];
-                            S.hloc[t] = S.hloc[q];
-                            S.hloc[q] = a;
-                            a = S.hidx[t];
-                            S.hidx[t] = S.hidx[q];
-                            S.hidx[q] = a;
-                        } else break;
-                        q = t;
-                    }
                 }
-                if (npos + SWM_PER_FETCH > SWM_BATCH_POSITIONS || hs == 0 || 1 + 2 * runs >= SWM_MAX_RUNS_BLOCK) {
-                    if (npos > 0) {
+                rc++;
+                e += get;
+                npos += get;
+                runs++;
+                // seeds_heap_pop_and_insert (1936-1962)
+                uint32_t x, xi;
+                if (get == have) {
+                    hs--;
+                    x = __shfl_sync(0xffffffffu, hs < 32 ? k0 : k1, hs & 31);
+                    xi = __shfl_sync(0xffffffffu, hs < 32 ? i0 : i1, hs & 31);
+                } else {
+                    x = sd.w;
+                    xi = i;
+                }
+                const u64 smaller = both(lane && 2 * (up0 + 1) < hs && (left ? !(k0 > a0) : a0 > k0),
+                                         2 * (up1 + 1) < hs && (left ? !(k1 > a1) : a1 > k1));
+                const bool on0 = lane && (smaller & anc0) == anc0, on1 = (smaller & anc1) == anc1;
+                const u64 path = both(on0, on1), stop = path & ~both(k0 < x, k1 < x);
+                const u64 move = stop ? path & ((stop & (0 - stop)) - 1) : path; // above the first that is not below x
+                const uint32_t dest = move ? 63 - __clzll(move) : 0;
+                const uint32_t c1 = 2 * lane + 1, c = move >> c1 & 1 ? c1 : c1 + 1; // child of place `lane` that moves up
+                const bool take = lane < 31 ? move >> c & 1 : move >> 63 & 1;
+                const uint32_t s = (lane < 31 ? c : 63u) & 31;
+                const uint32_t ka = __shfl_sync(0xffffffffu, k0, s), kb = __shfl_sync(0xffffffffu, k1, s);
+                const uint32_t ia = __shfl_sync(0xffffffffu, i0, s), ib = __shfl_sync(0xffffffffu, i1, s);
+                if (take) {
+                    k0 = c < 32 ? ka : kb;
+                    i0 = c < 32 ? ia : ib;
+                }
+                if (dest == lane) {
+                    k0 = x;
+                    i0 = xi;
+                }
+                if (dest == lane + 32) {
+                    k1 = x;
+                    i1 = xi;
+                }
+                if (lane == 0 && get != have) // (a seed's last key index + 1 may lie one past its keys: never used)
+                    S.seed[i] = make_uint4(sd.x + get, sd.y, sd.z + 1, sd.z + 1 < S.koff[i + 1] ? keys[sd.z + 1] : 0u);
+                __syncwarp();
+            }
+            if (npos + SWM_PER_FETCH > SWM_BATCH_POSITIONS || hs == 0 || 1 + 2 * runs >= SWM_MAX_RUNS_BLOCK) {
+                if (npos > 0) {
+                    if (lane == 0) {
                         B.bt_c0[sbase + b] = rb + br0; // refill chunks of the batch; batch 0 also
                         B.bt_c1[sbase + b] = rb + rc;  // holds every initial chunk
                         B.bt_e0[sbase + b] = eb + be0;
-                        b++;
                     }
-                    br0 = rc;
-                    be0 = e;
-                    npos = 0;
-                    runs = 0;
-                    if (hs == 0) break;
+                    b++;
                 }
+                br0 = rc;
+                be0 = e;
+                npos = 0;
+                runs = 0;
+                if (hs == 0) break;
             }
-            B.it_nbat[item] = b;
         }
+        if (lane == 0) B.it_nbat[item] = b;
         __syncwarp();
     }
 }
 
-// Lane-per-item refill planning for the items with at most PLAN_LANE_SEEDS
-// selected seeds: each lane runs one item's seed heap, the same schedule as
+// Lane-per-item refill planning for the items of short schedules: each lane runs one item's seed heap, the same schedule as
 // k_plan (alignment_rmdup 2194-2419 with the heap of 1919-1962 and its sift
 // bound), and a lane whose item is planned takes the next item from the list.
 // The heap key of seed i is the raw position of the last entry fetched from
@@ -1417,20 +1491,27 @@ __global__ void __launch_bounds__(PLAN_WARPS * 32) k_plan(const uint32_t *__rest
 // Per lane (one item each): every selected seed's next position index and
 // the end of its bucket (global indices into the position array), and the
 // seed heap (keys and seed indices). Two words per seed, not three, keep the
-// block at 26.5 KB: 8 resident blocks per SM instead of 6 -- the kernel waits
-// on one position-array key per refill, so resident lanes are what it runs on.
+// block at 26.5 KB for 32 seeds (8 resident blocks per SM instead of 6) and 53 KB
+// for 64 -- the kernel waits on one position-array key per refill, so resident
+// lanes are what it runs on.
+template <uint32_t SEEDS>
 struct PlanLaneSmem {
-    uint32_t cur[PLAN_LANE_SEEDS][32], end[PLAN_LANE_SEEDS][32];
-    uint32_t hloc[PLAN_LANE_SEEDS + 1][32];
-    uint8_t hidx[PLAN_LANE_SEEDS + 1][32];
+    uint32_t cur[SEEDS][32], end[SEEDS][32];
+    uint32_t hloc[SEEDS + 1][32];
+    uint8_t hidx[SEEDS + 1][32];
 };
 
-__global__ void __launch_bounds__(PLAN_LANE_WARPS * 32) k_plan_lanes(const uint32_t *__restrict__ pos, MapBufs B,
+template <uint32_t SEEDS>
+__global__ void __launch_bounds__(PLAN_LANE_WARPS * 32) k_plan_lanes(const uint32_t *__restrict__ pos,
+                                                                     const uint32_t *__restrict__ keys32, MapBufs B,
                                                                      uint64_t cap_chunks, uint64_t cap_elems) {
-    __shared__ PlanLaneSmem sm_all[PLAN_LANE_WARPS];
+    extern __shared__ __align__(16) unsigned char plan_smem[];
     const uint32_t lane = lane_id();
-    PlanLaneSmem &S = sm_all[threadIdx.x >> 5];
-    const uint32_t nlist = B.tot[TOT_PLN];
+    PlanLaneSmem<SEEDS> &S = reinterpret_cast<PlanLaneSmem<SEEDS> *>(plan_smem)[threadIdx.x >> 5];
+    const uint32_t nlist = B.tot[SEEDS == PLAN_LANE_SEEDS ? TOT_PLN : TOT_PLM];
+    const uint32_t *__restrict__ list = SEEDS == PLAN_LANE_SEEDS ? B.plan_list : B.plan_more;
+    uint32_t *queue = &B.tot[SEEDS == PLAN_LANE_SEEDS ? TOT_PLQ : TOT_PLMQ];
+    if (!nlist) return;
     bool active = false, drained = false;
     uint32_t item = 0, hs = 0, rc = 0, rb = 0, eb = 0, sbase = 0, e = 0, b = 0, br0 = 0, be0 = 0, npos = 0, runs = 0;
     for (;;) {
@@ -1442,14 +1523,14 @@ __global__ void __launch_bounds__(PLAN_LANE_WARPS * 32) k_plan_lanes(const uint3
         if (m && (__popc(m) >= PLAN_LANE_REFILL || !__any_sync(0xffffffffu, active))) {
             const uint32_t leader = __ffs(m) - 1;
             uint32_t first = 0;
-            if (lane == leader) first = atomicAdd(&B.tot[TOT_PLQ], (uint32_t)__popc(m));
+            if (lane == leader) first = atomicAdd(queue, (uint32_t)__popc(m));
             first = __shfl_sync(0xffffffffu, first, leader);
             if (need) {
                 const uint32_t idx = first + __popc(m & lanemask_lt());
                 if (idx >= nlist) {
                     drained = true;
                 } else {
-                    item = B.plan_list[idx];
+                    item = list[idx];
                     const uint32_t nref = B.it_nch[item];
                     rb = B.it_choff[item];
                     eb = B.it_eloff[item];
@@ -1488,7 +1569,7 @@ __global__ void __launch_bounds__(PLAN_LANE_WARPS * 32) k_plan_lanes(const uint3
                             for (uint32_t j = 0; j < 8; j++) {
                                 const uint32_t i = i0 + j;
                                 ins[j] = i < ns && S.cur[i][lane] != S.end[i][lane];
-                                key[j] = pos[ins[j] ? S.cur[i][lane] - 1 : 0u];
+                                key[j] = ins[j] ? refill_key(pos, keys32, S.cur[i][lane]) : 0u;
                             }
 #pragma unroll
                             for (uint32_t j = 0; j < 8; j++) {
@@ -1541,7 +1622,7 @@ __global__ void __launch_bounds__(PLAN_LANE_WARPS * 32) k_plan_lanes(const uint3
                 xi = S.hidx[hs][lane];
                 hs--;
             } else {
-                xk = pos[cu - 1];
+                xk = refill_key(pos, keys32, cu);
                 xi = i;
             }
             uint32_t q = 1;
@@ -1776,8 +1857,10 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS) k_cand(const
             }
             __syncwarp();
             for (uint32_t b = 0; b < nb; b++) {
-                uint32_t c0 = 0, c1 = 0, e0;
-                if (nref == 0) {
+                uint32_t c0, c1, e0;
+                if (nb == 1) { // every refill chunk; batch 0 also holds every initial chunk
+                    c0 = sbase - item;
+                    c1 = c0 + nref;
                     e0 = B.it_eloff[item];
                 } else {
                     c0 = B.bt_c0[sbase + b];
@@ -1979,8 +2062,10 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS)
             }
             uint32_t g0 = s0 != 0xffffffffu ? S.st[s0] : 0u;
             for (uint32_t b = 0; b < nb; b++) {
-                uint32_t c0 = 0, c1 = 0, e0;
-                if (nref == 0) {
+                uint32_t c0, c1, e0;
+                if (nb == 1) { // every refill chunk; batch 0 also holds every initial chunk
+                    c0 = sbase - item;
+                    c1 = c0 + nref;
                     e0 = B.it_eloff[item];
                 } else {
                     c0 = B.bt_c0[sbase + b];
@@ -2099,11 +2184,10 @@ __global__ void __launch_bounds__(256) k_compact(MapBufs B, uint64_t cap_chunks,
         // one thread per item: its scalars in one round trip, then its few
         // candidates batch by batch; items with many candidates are left to
         // the whole warp below
-        uint32_t nb = 0, nref = 0, o0 = 0, nc = 0, sbase = 0, eloff = 0;
+        uint32_t nb = 0, o0 = 0, nc = 0, sbase = 0, eloff = 0;
         bool heavy = false;
         if (item < nitems) {
             nb = B.it_nbat[item];
-            nref = B.it_nch[item];
             o0 = B.it_coff[item];
             nc = B.it_ncand[item];
             sbase = B.it_choff[item] + item;
@@ -2116,8 +2200,8 @@ __global__ void __launch_bounds__(256) k_compact(MapBufs B, uint64_t cap_chunks,
             if (nb && !heavy) {
                 uint32_t o = o0;
                 for (uint32_t b = 0; b < nb; b++) {
-                    const uint32_t n = nref ? B.bt_cnt[sbase + b] : nc; // one batch when there are no refills
-                    const uint32_t e0 = nref ? B.bt_e0[sbase + b] : eloff;
+                    const uint32_t n = nb > 1 ? B.bt_cnt[sbase + b] : nc;
+                    const uint32_t e0 = nb > 1 ? B.bt_e0[sbase + b] : eloff;
                     for (uint32_t j = 0; j < n; j++) {
                         B.cc_pos[o + j] = B.cand_ub[e0 + j];
                         B.cc_item[o + j] = item;
@@ -2130,13 +2214,13 @@ __global__ void __launch_bounds__(256) k_compact(MapBufs B, uint64_t cap_chunks,
         while (hm) { // the warp copies each heavy item of the group, lanes over its candidates
             const uint32_t src = __ffs(hm) - 1;
             hm &= hm - 1;
-            const uint32_t hnb = __shfl_sync(0xffffffffu, nb, src), hnref = __shfl_sync(0xffffffffu, nref, src);
+            const uint32_t hnb = __shfl_sync(0xffffffffu, nb, src);
             const uint32_t hnc = __shfl_sync(0xffffffffu, nc, src), hsb = __shfl_sync(0xffffffffu, sbase, src);
             const uint32_t hel = __shfl_sync(0xffffffffu, eloff, src);
             uint32_t o = __shfl_sync(0xffffffffu, o0, src);
             for (uint32_t b = 0; b < hnb; b++) {
-                const uint32_t n = hnref ? B.bt_cnt[hsb + b] : hnc;
-                const uint32_t e0 = hnref ? B.bt_e0[hsb + b] : hel;
+                const uint32_t n = hnb > 1 ? B.bt_cnt[hsb + b] : hnc;
+                const uint32_t e0 = hnb > 1 ? B.bt_e0[hsb + b] : hel;
                 for (uint32_t j = lane; j < n; j += 32) {
                     B.cc_pos[o + j] = B.cand_ub[e0 + j];
                     B.cc_item[o + j] = item0 + src;
@@ -3712,7 +3796,7 @@ static int dmalloc(T **p, uint64_t count) {
 
 static void free_bufs(MapBufs &B) {
     void *ps[] = {B.par, B.it_w, B.sel, B.sel_fl, B.sel_key, B.it_perm, B.unm, B.it_nsel, B.it_e, B.it_nch, B.it_nel, B.it_nbat,
-                  B.it_choff, B.it_eloff, B.it_nrec, B.it_nw, B.it_nb, B.it_recoff, B.it_woff, B.it_boff, B.it_ncand, B.plan_list,
+                  B.it_choff, B.it_eloff, B.it_nrec, B.it_nw, B.it_nb, B.it_recoff, B.it_woff, B.it_boff, B.it_ncand, B.plan_list, B.plan_more,
                   B.it_coff, B.ch_g, B.ch_meta, B.bt_c0, B.bt_c1, B.bt_e0, B.bt_cnt, B.sort_scratch, B.cand_ub, B.cc_pos,
                   B.cc_item, B.plan_keys, B.vr_flag, B.vr_loc, B.vr_err, B.vr_mloc, B.vr_tlen, B.vr_cig, B.vr_aoff, B.arena, B.tb_list,
                   B.tb_cp, B.slow_list, B.vt_x, B.vt_st, B.vt_cp,
@@ -3748,6 +3832,7 @@ static int alloc_items(swm_mapper *m) {
     rc |= dmalloc(&B.it_boff, I + 1);
     rc |= dmalloc(&B.it_ncand, I);
     rc |= dmalloc(&B.plan_list, I);
+    rc |= dmalloc(&B.plan_more, I);
     rc |= dmalloc(&B.it_coff, I + 1);
     rc |= dmalloc(&B.stat, ST_N);
     rc |= dmalloc(&B.tot, TOT_N);
@@ -3806,7 +3891,8 @@ extern "C" int swm_mapper_create(swm_index *ix, uint64_t max_reads, swm_mapper *
     SWM_CUDA(cudaSetDevice(ix->device));
     // the index's candidate table (k = 12), built once when the device has room
     // and the buckets are large enough for it to pay
-    const int trc = swm_ctab_build(ix, 0);
+    int trc = swm_ctab_build(ix, 0);
+    if (!trc) trc = swm_keys32_build(ix);
     if (trc) return trc;
     swm_mapper *m = (swm_mapper *)calloc(1, sizeof(swm_mapper));
     if (!m) return SWM_ERR_OOM;
@@ -3827,6 +3913,11 @@ extern "C" int swm_mapper_create(swm_index *ix, uint64_t max_reads, swm_mapper *
     if (cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking) != cudaSuccess) rc = SWM_ERR_CUDA;
     for (int i = 0; i < 9 && rc == SWM_OK; i++)
         if (cudaEventCreate(&m->ev[i]) != cudaSuccess) rc = SWM_ERR_CUDA;
+    if (rc == SWM_OK && cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming) != cudaSuccess) rc = SWM_ERR_CUDA;
+    for (int i = 0; i < 2 && rc == SWM_OK; i++)
+        if (cudaStreamCreateWithFlags(&m->side[i], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&m->join[i], cudaEventDisableTiming) != cudaSuccess)
+            rc = SWM_ERR_CUDA;
     if (rc == SWM_OK) rc = alloc_items(m);
     if (rc == SWM_OK) rc = alloc_work(m);
     if (rc == SWM_OK && (dmalloc(&m->d_lens, max_reads) || dmalloc(&m->d_e, max_reads))) rc = SWM_ERR_OOM;
@@ -3871,6 +3962,11 @@ extern "C" void swm_mapper_free(swm_mapper *m) {
     cudaFreeHost(m->h_par);
     for (int i = 0; i < 9; i++)
         if (m->ev[i]) cudaEventDestroy(m->ev[i]);
+    if (m->fork) cudaEventDestroy(m->fork);
+    for (int i = 0; i < 2; i++) {
+        if (m->join[i]) cudaEventDestroy(m->join[i]);
+        if (m->side[i]) cudaStreamDestroy(m->side[i]);
+    }
     if (m->st) cudaStreamDestroy(m->st);
     free(m);
 }
@@ -3918,10 +4014,25 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
         B, ScanItems{{B.it_nch, B.it_nel}, {B.it_choff, B.it_eloff}, {TOT_CHUNKS, TOT_ELEMS}, 0, TOT_SC1});
     m->launches++;
     k_plan_list<<<grid_cap(ci, 256, 8), 256, 0, st>>>(B, m->cap_chunks, !table);
-    k_plan_lanes<<<grid_cap(ci, PLAN_LANE_WARPS * 32, 8), PLAN_LANE_WARPS * 32, 0, st>>>(ix->d_pos, B, m->cap_chunks,
-                                                                                         m->cap_elems);
-    k_plan<<<grid_cap(ci, PLAN_WARPS * 32, 16), PLAN_WARPS * 32, 0, st>>>(ix->d_pos, B, m->cap_chunks,
-                                                                          m->cap_elems);
+    m->launches++;
+    LAUNCH_CHECK();
+    // the three planners beside each other: each waits on the serial schedules of
+    // its longest items
+    SWM_CUDA(cudaEventRecord(m->fork, st));
+    for (int i = 0; i < 2; i++) SWM_CUDA(cudaStreamWaitEvent(m->side[i], m->fork, 0));
+    k_plan<<<grid_cap(ci, PLAN_WARPS * 32, 6), PLAN_WARPS * 32, 0, m->side[0]>>>(ix->d_pos, ix->d_keys32, B, m->cap_chunks,
+                                                                                m->cap_elems);
+    const size_t smem_few = sizeof(PlanLaneSmem<PLAN_LANE_SEEDS>) * PLAN_LANE_WARPS,
+                 smem_more = sizeof(PlanLaneSmem<SWM_MAX_SEL>) * PLAN_LANE_WARPS;
+    SWM_CUDA(cudaFuncSetAttribute(k_plan_lanes<SWM_MAX_SEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_more));
+    k_plan_lanes<SWM_MAX_SEL><<<grid_cap(ci, PLAN_LANE_WARPS * 32, 4), PLAN_LANE_WARPS * 32, smem_more, m->side[1]>>>(
+        ix->d_pos, ix->d_keys32, B, m->cap_chunks, m->cap_elems);
+    k_plan_lanes<PLAN_LANE_SEEDS><<<grid_cap(ci, PLAN_LANE_WARPS * 32, 8), PLAN_LANE_WARPS * 32, smem_few, st>>>(
+        ix->d_pos, ix->d_keys32, B, m->cap_chunks, m->cap_elems);
+    for (int i = 0; i < 2; i++) {
+        SWM_CUDA(cudaEventRecord(m->join[i], m->side[i]));
+        SWM_CUDA(cudaStreamWaitEvent(st, m->join[i], 0));
+    }
     m->launches += 3;
     LAUNCH_CHECK();
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[2], st, cudaEventRecordExternal));

@@ -584,3 +584,31 @@ def test_gpu_seed_kernels_of_other_lengths(cuda_lib, k):
             ref = po.map_reads(mix, reads, lens, e, nthreads=8)
             _check(out, ref.records(), ref.unmapped)
             assert m.stats()["candidates"] == ref.stats["candidates"]
+
+
+@pytest.mark.parametrize("n,k,copies,e", [(1_000_000, 6, 0, 7), (1_000_000, 6, 0, 15), (6_000_000, 6, 0, 15),
+                                          (1_200_000, 12, 6000, 7), (1_200_000, 12, 6000, 12), (2_300_000, 12, 12000, 7)])
+def test_gpu_refill_schedules_of_every_planner(cuda_lib, n, k, copies, e):
+    """Schedules of a few dozen to a few thousand refills over up to 64 seeds:
+    short ones of at most 32 seeds, of more, and long ones, whose keys outgrow
+    shared memory at 12,000 copies; k = 6 has large buckets, so the planners read
+    their keys from the key array (the others from the positions)."""
+    rng = np.random.default_rng(61)
+    g = genome(n, 62)
+    if copies:
+        unit, step = rng.choice(np.frombuffer(b"ACGT", np.uint8), 160), n // copies
+        assert step > 170
+        at = np.arange(copies)[:, None] * step + rng.integers(0, 8, copies)[:, None] + np.arange(160)[None, :]
+        mut = rng.random((copies, 160)) < 0.02
+        g[at] = np.where(mut, rng.choice(np.frombuffer(b"ACGT", np.uint8), (copies, 160)), unit)
+    reads, lens, _, _ = synth.reads(g, 120, 120, 150, 0.02, seed=63, stride=150)
+    mix = po.MapIndex(po.build_index(g, k))
+    ref = po.map_reads(mix, reads, lens, e, nthreads=8, cap_records=40_000)
+    for table in (False, True) if k == 12 else (False,):
+        ix = cuda_lib.Index.build(g, k=k)
+        assert (ix.candidate_table(table) > 0) == table
+        m = cuda_lib.Mapper(ix, max_reads=120)
+        out = m.map(reads, lens, e, records_cap=40_000)
+        _check(out, ref.records(), ref.unmapped)
+        st = m.stats()
+        assert (st["batches"], st["candidates"]) == (ref.stats["batches"], ref.stats["candidates"])
