@@ -48,7 +48,6 @@ enum {
     ST_CELLS,
     ST_PASSED,
     ST_LOCS,
-    ST_MAPPED,
     ST_STEPS, // Myers steps (read bases) run by k_verify
     ST_KEPT,  // positions the flank filter kept, before each batch's merge
     ST_N
@@ -63,6 +62,7 @@ enum {
     TOT_PLW, TOT_PLWQ, // and those with long schedules; queue head of k_plan
     TOT_CQ,            // queue head of the candidate stage (items)
     TOT_RQC, TOT_RQW,  // queue heads of the records count and write passes (groups of 32 items)
+    TOT_UNM,                   // reads without a location
     TOT_SC1, TOT_SC2, TOT_SC3, // tile tickets of the scans after the seed, candidate and records-count stages
     TOT_TBDONE, TOT_RDONE,     // blocks of k_traceback and of the records write pass that are through
     TOT_N
@@ -101,7 +101,8 @@ __device__ __forceinline__ uint32_t single_batch(uint32_t nref, uint32_t nel) {
 
 #define ARENA_CAP_DEFAULT (1u << 20)
 #define SCAN_TILE_ITEMS 2048 // items per tile of k_scan_items
-#define SCAN_VALUES 6        // values scanned per block: refill chunks, positions, candidates, records, words, bytes
+#define SCAN_VALUES 7        // values scanned per block: refill chunks, positions, candidates, records, words, bytes,
+                             // and reads without a record
 
 // The inputs of one block, in device memory so that the captured launch
 // sequence of a mapper does not depend on them.
@@ -145,7 +146,7 @@ struct MapBufs {
     uint8_t *vr_cig;  // cap_cands * SWM_CIGAR_SLOT
     uint32_t *vr_aoff;
     uint8_t *arena;   // long CIGAR texts
-    uint16_t *unm;       // bit j of halfword w: read 16 w + j has no location (cap_items / 32 + 1)
+    uint32_t *unm;       // cur_read ids (2 * read + 1) of the reads without a location, in read order (items / 2)
     uint2 *vt_x;         // candidates alive after the head of verification: (candidate, ones) (cap_cands)
     uint4 *vt_st;        // and their Myers state (VP, VN, checkpoint before base 16) (cap_cands)
     uint4 *vt_cp;        // and the checkpoints before bases 32 and 48 (cap_cands)
@@ -190,9 +191,9 @@ struct swm_mapper {
     uint8_t *h_e;
     // pinned result staging
     uint32_t *h_w, *h_rw, *h_rb, *h_rl;
-    uint16_t *h_unm;
+    uint32_t *h_unm;
     uint8_t *h_c;
-    uint64_t h_cap_w, h_cap_c, h_cap_rw, h_cap_rb, h_cap_rl, h_cap_items;
+    uint64_t h_cap_w, h_cap_c, h_cap_rw, h_cap_rb, h_cap_rl, h_cap_unm;
     uint32_t *h_tot;           // pinned copy of B.tot
     unsigned long long *h_stat; // pinned copy of B.stat
     // state of the block in flight / last block
@@ -1094,6 +1095,11 @@ __global__ void __launch_bounds__(1024) k_begin(const BlockParams *__restrict__ 
 // the wait ends; a wait past SCAN_SPIN_LIMIT polls fails the block instead.
 // One launch replaces three per value: with those, a block was 31 launches and
 // 16 reads took 129 us on the GPU; now 15 and 108 us.
+//
+// UNM: in[0] holds the items' record counts, and one more value is scanned, 1
+// for the second item of a read neither of whose items has a record: its
+// prefix is the place of the read in the list of unmapped reads, which is
+// written here (mapper_cpe.c:1455-1458).
 struct ScanItems {
     const uint32_t *in[3];
     uint32_t *out[3];
@@ -1101,9 +1107,9 @@ struct ScanItems {
 };
 #define SCAN_SPIN_LIMIT (1u << 22)
 
-template <int K>
+template <int KIN, bool UNM>
 __global__ void __launch_bounds__(256) k_scan_items(MapBufs B, ScanItems A) {
-    constexpr int V = SCAN_TILE_ITEMS / 256;
+    constexpr int V = SCAN_TILE_ITEMS / 256, K = KIN + (UNM ? 1 : 0);
     static_assert(V == 8, "two 16-byte loads a thread");
     __shared__ unsigned long long wsum[K][8], before[K], sum[K];
     __shared__ uint32_t s_tile;
@@ -1117,7 +1123,10 @@ __global__ void __launch_bounds__(256) k_scan_items(MapBufs B, ScanItems A) {
     unsigned long long mine[K], incl[K];
 #pragma unroll
     for (int k = 0; k < K; k++) {
-        if (i0 + V <= n) {
+        if (k == KIN) { // a read's two items are neighbours in one thread
+#pragma unroll
+            for (int j = 0; j < V; j++) v[k][j] = (j & 1) && i0 + j < n && (v[0][j - (j & 1)] | v[0][j]) == 0 ? 1u : 0u;
+        } else if (i0 + V <= n) {
             const uint4 a = reinterpret_cast<const uint4 *>(A.in[k] + i0)[0], b = reinterpret_cast<const uint4 *>(A.in[k] + i0)[1];
             v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
             v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
@@ -1179,6 +1188,13 @@ __global__ void __launch_bounds__(256) k_scan_items(MapBufs B, ScanItems A) {
         for (int j = 0; j < V; j++) {
             o[j] = (uint32_t)ex;
             ex += v[k][j];
+        }
+        if (k == KIN) {
+#pragma unroll
+            for (int j = 1; j < V; j += 2)
+                if (v[k][j]) B.unm[o[j]] = i0 + j;
+            if (tile == tiles - 1 && tid == 0) B.tot[TOT_UNM] = (uint32_t)sum[k];
+            continue;
         }
         if (i0 + V <= n) {
             reinterpret_cast<uint4 *>(A.out[k] + i0)[0] = make_uint4(o[0], o[1], o[2], o[3]);
@@ -3601,7 +3617,7 @@ __device__ uint32_t records_seq(const MapBufs &B, uint32_t item, uint64_t cap_re
 // the same location itself). The warp reads 32 verdict flags per load, and
 // only the passing lanes read their location and CIGAR; the rest go through
 // records_seq on lane 0. Count pass: the item's record / word / byte counts;
-// write pass: the records, and the unmapped-read bits of the group; its last
+// write pass: the records; its last
 // block copies the block's totals and statistics to the host.
 template <bool WRITE>
 __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks, uint64_t cap_elems,
@@ -3615,7 +3631,7 @@ __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks,
     const uint8_t *__restrict__ vcig = B.vr_cig;
     uint8_t *__restrict__ out_c = B.out_c;
     uint32_t *__restrict__ out_w = B.out_w;
-    unsigned long long locs_total = 0, mapped = 0, batches = 0;
+    unsigned long long locs_total = 0, batches = 0;
     for (; !failed;) {
         const uint32_t item0 = warp_take(&B.tot[WRITE ? TOT_RQW : TOT_RQC]);
         if (item0 >= nitems) break;
@@ -3726,25 +3742,12 @@ __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks,
                 }
             }
         }
-        if (WRITE) {
-            // unmapped reads as bits, 16 reads (the group's 32 items) per halfword
-            const uint32_t prev = __shfl_up_sync(0xffffffffu, g_nrec, 1);
-            const bool valid = mine < nitems;
-            const bool mp = (lane & 1) && (g_nrec + prev) > 0;
-            const unsigned bal = __ballot_sync(0xffffffffu, valid && (lane & 1) && !mp);
-            const unsigned mb = __ballot_sync(0xffffffffu, valid && mp);
-            if (lane == 0) {
-                B.unm[item0 >> 5] = (uint16_t)even_bits(bal >> 1);
-                mapped += __popc(mb);
-            }
-        }
     }
     if (!WRITE) {
         warp_add_u64(&B.stat[ST_BATCHES], batches);
         return;
     }
     warp_add_u64(&B.stat[ST_LOCS], locs_total);
-    warp_add_u64(&B.stat[ST_MAPPED], mapped);
     // the last block to get here hands the block's totals to the host (pinned
     // memory), which reads them once the stream has drained
     __shared__ uint32_t s_last;
@@ -3816,7 +3819,7 @@ static int alloc_items(swm_mapper *m) {
     rc |= dmalloc(&B.sel_fl, I * SWM_MAX_SEL);
     rc |= dmalloc(&B.sel_key, I * (SWM_MAX_SEL / SWM_SEED_STEP));
     rc |= dmalloc(&B.it_perm, I);
-    rc |= dmalloc(&B.unm, I / 32 + 1);
+    rc |= dmalloc(&B.unm, I / 2);
     rc |= dmalloc(&B.it_nsel, I);
     rc |= dmalloc(&B.it_e, I);
     rc |= dmalloc(&B.it_nch, I);
@@ -3923,7 +3926,6 @@ extern "C" int swm_mapper_create(swm_index *ix, uint64_t max_reads, swm_mapper *
     if (rc == SWM_OK && (dmalloc(&m->d_lens, max_reads) || dmalloc(&m->d_e, max_reads))) rc = SWM_ERR_OOM;
     if (rc == SWM_OK && (cudaHostAlloc((void **)&m->h_lens, max_reads * 4, 0) != cudaSuccess ||
                          cudaHostAlloc((void **)&m->h_e, max_reads, 0) != cudaSuccess ||
-                         cudaHostAlloc((void **)&m->h_unm, (m->cap_items / 32 + 1) * 2, 0) != cudaSuccess ||
                          cudaHostAlloc((void **)&m->h_tot, TOT_N * 4, 0) != cudaSuccess ||
                          cudaHostAlloc((void **)&m->h_stat, ST_N * 8, 0) != cudaSuccess ||
                          cudaHostAlloc((void **)&m->h_par, sizeof(BlockParams), 0) != cudaSuccess))
@@ -3932,7 +3934,6 @@ extern "C" int swm_mapper_create(swm_index *ix, uint64_t max_reads, swm_mapper *
         swm_mapper_free(m);
         return rc;
     }
-    m->h_cap_items = m->cap_items / 32 + 1;
     *out = m;
     return SWM_OK;
 }
@@ -4010,7 +4011,7 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     m->launches++;
     LAUNCH_CHECK();
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[1], st, cudaEventRecordExternal));
-    k_scan_items<2><<<scan_grid, 256, 0, st>>>(
+    k_scan_items<2, false><<<scan_grid, 256, 0, st>>>(
         B, ScanItems{{B.it_nch, B.it_nel}, {B.it_choff, B.it_eloff}, {TOT_CHUNKS, TOT_ELEMS}, 0, TOT_SC1});
     m->launches++;
     k_plan_list<<<grid_cap(ci, 256, 8), 256, 0, st>>>(B, m->cap_chunks, !table);
@@ -4045,7 +4046,7 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     m->launches++;
     LAUNCH_CHECK();
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[3], st, cudaEventRecordExternal));
-    k_scan_items<1><<<scan_grid, 256, 0, st>>>(B, ScanItems{{B.it_ncand}, {B.it_coff}, {TOT_CANDS}, 2, TOT_SC2});
+    k_scan_items<1, false><<<scan_grid, 256, 0, st>>>(B, ScanItems{{B.it_ncand}, {B.it_coff}, {TOT_CANDS}, 2, TOT_SC2});
     m->launches++;
     k_compact<<<grid_cap(ci, 256, 8), 256, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands);
     m->launches++;
@@ -4081,7 +4082,7 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     SWM_CUDA(cudaEventRecordWithFlags(m->ev[6], st, cudaEventRecordExternal));
     k_records<false><<<grid_cap(ci, 128, 16), 128, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands, m->cap_recs,
                                                              m->cap_words, m->cap_bytes, nullptr, nullptr);
-    k_scan_items<3><<<scan_grid, 256, 0, st>>>(B, ScanItems{{B.it_nrec, B.it_nw, B.it_nb},
+    k_scan_items<3, true><<<scan_grid, 256, 0, st>>>(B, ScanItems{{B.it_nrec, B.it_nw, B.it_nb},
                                                             {B.it_recoff, B.it_woff, B.it_boff},
                                                             {TOT_RECS, TOT_WORDS, TOT_BYTES}, 3, TOT_SC3});
     k_records<true><<<grid_cap(ci, 128, 10), 128, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands, m->cap_recs,
@@ -4259,7 +4260,7 @@ static int finish_block(swm_mapper *m, uint32_t nreads, uint64_t retries, int *a
     S.passed = stat[ST_PASSED];
     S.records = m->tot[TOT_RECS];
     S.locations = stat[ST_LOCS];
-    S.mapped_reads = stat[ST_MAPPED];
+    S.mapped_reads = nreads - m->tot[TOT_UNM];
     S.myers_steps = stat[ST_STEPS];
     S.kept = stat[ST_KEPT];
     S.retries = retries;
@@ -4382,38 +4383,42 @@ static bool is_pinned(const void *p) {
     return a.type == cudaMemoryTypeHost;
 }
 
-// Copy the packed records of the last block to pinned staging.
-// cur_read ids (2 * read + 1) of the reads without a location, in read
-// order, from the device's bit list (mapper_cpe.c:1455-1458).
-static uint64_t unmapped_list(const swm_mapper *m, uint32_t *out, uint64_t cap, int *status) {
-    uint64_t nu = 0;
-    const uint64_t nh = (m->cur_n + 15) / 16;
-    for (uint64_t w = 0; w < nh; w++) {
-        uint32_t bits = m->h_unm[w];
-        while (bits) {
-            const uint32_t j = (uint32_t)__builtin_ctz(bits);
-            bits &= bits - 1;
-            const uint64_t rd = 16 * w + j;
-            if (rd >= m->cur_n) break;
-            if (nu < cap && out) out[nu] = (uint32_t)(2 * rd + 1);
-            else *status = SWM_ERR_OVERFLOW;
-            nu++;
-        }
+// Queue the copy of the unmapped read ids into the caller's buffer when it is
+// page-locked and holds them, else into pinned staging (*staged).
+static int queue_unmapped(swm_mapper *m, const uint32_t *out, uint64_t cap, bool *staged) {
+    const uint64_t n = m->tot[TOT_UNM];
+    *staged = false;
+    if (!n) return SWM_OK;
+    uint32_t *to = const_cast<uint32_t *>(out);
+    if (!out || n > cap || !is_pinned(out)) {
+        const int rc = ensure_host((void **)&m->h_unm, &m->h_cap_unm, n, 4);
+        if (rc) return rc;
+        to = m->h_unm;
+        *staged = true;
     }
-    return nu;
+    SWM_CUDA(cudaMemcpyAsync(to, m->b.unm, n * 4, cudaMemcpyDeviceToHost, m->st));
+    return SWM_OK;
 }
 
-static int download_results(swm_mapper *m) {
+// The ids are in pinned memory: hand over the staged ones.
+static uint64_t unmapped_list(const swm_mapper *m, uint32_t *out, uint64_t cap, bool staged, int *status) {
+    const uint64_t n = m->tot[TOT_UNM];
+    if (staged && out) memcpy(out, m->h_unm, (n < cap ? n : cap) * 4);
+    if (n && (!out || n > cap)) *status = SWM_ERR_OVERFLOW;
+    return n;
+}
+
+// Copy the packed records of the last block to pinned staging.
+static int download_results(swm_mapper *m, const uint32_t *unmapped, uint64_t unmapped_cap, bool *staged) {
     if (!m->have_result) return SWM_ERR_STATE;
     SWM_CUDA(cudaSetDevice(m->device));
-    const uint64_t nitems = 2 * m->cur_n;
     const uint64_t nrec = m->tot[TOT_RECS], nw = m->tot[TOT_WORDS], nby = m->tot[TOT_BYTES];
     int rc = ensure_host((void **)&m->h_w, &m->h_cap_w, nw, 4);
     if (!rc) rc = ensure_host((void **)&m->h_c, &m->h_cap_c, nby, 1);
     if (!rc) rc = ensure_host((void **)&m->h_rw, &m->h_cap_rw, nrec, 4);
     if (!rc) rc = ensure_host((void **)&m->h_rb, &m->h_cap_rb, nrec, 4);
     if (!rc) rc = ensure_host((void **)&m->h_rl, &m->h_cap_rl, nrec, 4);
-    if (!rc) rc = ensure_host((void **)&m->h_unm, &m->h_cap_items, nitems / 32 + 1, 2);
+    if (!rc) rc = queue_unmapped(m, unmapped, unmapped_cap, staged);
     if (rc) return rc;
     cudaStream_t st = m->st;
     if (nw) SWM_CUDA(cudaMemcpyAsync(m->h_w, m->b.out_w, nw * 4, cudaMemcpyDeviceToHost, st));
@@ -4423,10 +4428,8 @@ static int download_results(swm_mapper *m) {
         SWM_CUDA(cudaMemcpyAsync(m->h_rb, m->b.rec_boff, nrec * 4, cudaMemcpyDeviceToHost, st));
         SWM_CUDA(cudaMemcpyAsync(m->h_rl, m->b.rec_blen, nrec * 4, cudaMemcpyDeviceToHost, st));
     }
-    const uint64_t nunm = (m->cur_n + 15) / 16;
-    if (nunm) SWM_CUDA(cudaMemcpyAsync(m->h_unm, m->b.unm, nunm * 2, cudaMemcpyDeviceToHost, st));
     SWM_CUDA(cudaStreamSynchronize(st));
-    m->stats.d2h_bytes = nw * 4 + nby + nrec * 12 + nunm * 2 + TOT_N * 4 + ST_N * 8;
+    m->stats.d2h_bytes = nw * 4 + nby + nrec * 12 + m->tot[TOT_UNM] * 4ull + TOT_N * 4 + ST_N * 8;
     return SWM_OK;
 }
 
@@ -4434,7 +4437,8 @@ static int download_results(swm_mapper *m) {
 // (records at SWM_RECORD_WORDS, CIGARs at SWM_CIGAR_STRIDE, unmapped ids).
 extern "C" int swm_map_fetch(swm_mapper *m, swm_result *r) {
     if (!m || !r) return SWM_ERR_ARG;
-    int rc = download_results(m);
+    bool staged = false;
+    int rc = download_results(m, r->unmapped, r->unmapped_cap, &staged);
     if (rc) return rc;
     const uint64_t nrec = m->tot[TOT_RECS];
     int status = SWM_OK;
@@ -4454,7 +4458,7 @@ extern "C" int swm_map_fetch(swm_mapper *m, swm_result *r) {
             status = SWM_ERR_OVERFLOW;
         }
     }
-    r->n_unmapped = unmapped_list(m, r->unmapped, r->unmapped_cap, &status);
+    r->n_unmapped = unmapped_list(m, r->unmapped, r->unmapped_cap, staged, &status);
     if (status) swm_set_error("result buffers too small (records %llu, unmapped %llu)", (unsigned long long)nrec,
                               (unsigned long long)r->n_unmapped);
     return status;
@@ -4468,26 +4472,25 @@ extern "C" int swm_map_fetch_packed(swm_mapper *m, swm_packed_result *r) {
         is_pinned(r->cigar) && (!r->record_cigar_len || is_pinned(r->record_cigar_len))) {
         // page-locked caller buffers: copy the packed results straight into them
         SWM_CUDA(cudaSetDevice(m->device));
-        const uint64_t nitems = 2 * m->cur_n;
-        int rc0 = ensure_host((void **)&m->h_unm, &m->h_cap_items, nitems / 32 + 1, 2);
+        bool staged;
+        const int rc0 = queue_unmapped(m, r->unmapped, r->unmapped_cap, &staged);
         if (rc0) return rc0;
         cudaStream_t st = m->st;
         if (nw) SWM_CUDA(cudaMemcpyAsync(r->words, m->b.out_w, nw * 4, cudaMemcpyDeviceToHost, st));
         if (nby) SWM_CUDA(cudaMemcpyAsync(r->cigar, m->b.out_c, nby, cudaMemcpyDeviceToHost, st));
         if (nrec && r->record_cigar_len)
             SWM_CUDA(cudaMemcpyAsync(r->record_cigar_len, m->b.rec_blen, nrec * 4, cudaMemcpyDeviceToHost, st));
-        const uint64_t nunm = (m->cur_n + 15) / 16;
-        if (nunm) SWM_CUDA(cudaMemcpyAsync(m->h_unm, m->b.unm, nunm * 2, cudaMemcpyDeviceToHost, st));
         SWM_CUDA(cudaStreamSynchronize(st));
-        m->stats.d2h_bytes = nw * 4 + nby + (r->record_cigar_len ? nrec * 4 : 0) + nunm * 2 + TOT_N * 4 + ST_N * 8;
+        m->stats.d2h_bytes = nw * 4 + nby + (r->record_cigar_len ? nrec * 4 : 0) + m->tot[TOT_UNM] * 4ull + TOT_N * 4 + ST_N * 8;
         r->n_records = nrec;
         r->n_words = nw;
         r->n_cigar = nby;
         int status = SWM_OK;
-        r->n_unmapped = unmapped_list(m, r->unmapped, r->unmapped_cap, &status);
+        r->n_unmapped = unmapped_list(m, r->unmapped, r->unmapped_cap, staged, &status);
         return status;
     }
-    int rc = download_results(m);
+    bool staged = false;
+    int rc = download_results(m, r->unmapped, r->unmapped_cap, &staged);
     if (rc) return rc;
     r->n_records = nrec;
     r->n_words = nw;
@@ -4502,7 +4505,7 @@ extern "C" int swm_map_fetch_packed(swm_mapper *m, swm_packed_result *r) {
         if (nby) memcpy(r->cigar, m->h_c, nby);
         if (r->record_cigar_len && nrec) memcpy(r->record_cigar_len, m->h_rl, nrec * 4);
     }
-    r->n_unmapped = unmapped_list(m, r->unmapped, r->unmapped_cap, &status);
+    r->n_unmapped = unmapped_list(m, r->unmapped, r->unmapped_cap, staged, &status);
     if (status) swm_set_error("packed result buffers too small (words %llu, bytes %llu, records %llu)",
                               (unsigned long long)nw, (unsigned long long)nby, (unsigned long long)nrec);
     return status;
