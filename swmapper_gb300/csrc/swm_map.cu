@@ -4301,18 +4301,28 @@ static int check_batch(const swm_mapper *m, uint64_t nreads, uint64_t stride, ui
     return SWM_OK;
 }
 
+// Longest read a block may hold: the envelope, the stride, and 16 long seeds.
+static uint32_t longest_read(const swm_mapper *m, uint64_t stride) {
+    const uint32_t klong = m->ix->k + SWM_SEED_STEP - 1, seeds = 17 * klong - 1;
+    const uint32_t top = seeds < SWM_MAX_READ_LEN ? seeds : SWM_MAX_READ_LEN;
+    return stride < top ? (uint32_t)stride : top;
+}
+
+// Two maxima over the block (which the compiler vectorises; one test per read,
+// with a division, took 2 ns a read), and only for a bad one the read.
 static int check_host_reads(const swm_mapper *m, const uint32_t *lens, const uint8_t *e_arr, uint64_t nreads,
                             uint64_t stride) {
-    const uint32_t klong = m->ix->k + SWM_SEED_STEP - 1;
-    for (uint64_t r = 0; r < nreads; r++) {
-        if (lens[r] > SWM_MAX_READ_LEN || lens[r] > stride || lens[r] / klong > 16 ||
-            (e_arr && e_arr[r] > SWM_MAX_ERRORS)) {
-            swm_set_error("read %llu: length %u or threshold outside the envelope (L <= %d, L <= stride, e <= %d)",
-                          (unsigned long long)r, lens[r], SWM_MAX_READ_LEN, SWM_MAX_ERRORS);
-            return SWM_ERR_ARG;
-        }
-    }
-    return SWM_OK;
+    const uint32_t top = longest_read(m, stride);
+    uint32_t longest = 0;
+    uint8_t most = 0;
+    for (uint64_t r = 0; r < nreads; r++) longest = lens[r] > longest ? lens[r] : longest;
+    for (uint64_t r = 0; e_arr && r < nreads; r++) most = e_arr[r] > most ? e_arr[r] : most;
+    if (longest <= top && most <= SWM_MAX_ERRORS) return SWM_OK;
+    uint64_t r = 0;
+    while (lens[r] <= top && !(e_arr && e_arr[r] > SWM_MAX_ERRORS)) r++;
+    swm_set_error("read %llu: length %u or threshold outside the envelope (L <= %d, L <= stride, e <= %d)",
+                  (unsigned long long)r, lens[r], SWM_MAX_READ_LEN, SWM_MAX_ERRORS);
+    return SWM_ERR_ARG;
 }
 
 extern "C" int swm_map_device(swm_mapper *m, const char *d_reads, const uint32_t *d_lens, uint64_t stride,
@@ -4515,8 +4525,6 @@ static int stage_inputs(swm_mapper *m, const swm_batch *b) {
     const uint64_t n = b->reads_num;
     int rc = check_batch(m, n, b->stride, b->errors);
     if (rc) return rc;
-    rc = check_host_reads(m, b->reads_len, b->errors_per_read, n, b->stride);
-    if (rc) return rc;
     const uint64_t bytes = n * b->stride;
     if (bytes > m->stride_cap) {
         cudaFree(m->d_reads);
@@ -4549,6 +4557,12 @@ static int stage_inputs(swm_mapper *m, const swm_batch *b) {
     SWM_CUDA(cudaMemcpyAsync(m->d_reads, src_reads, bytes, cudaMemcpyHostToDevice, m->st));
     SWM_CUDA(cudaMemcpyAsync(m->d_lens, src_lens, n * 4, cudaMemcpyHostToDevice, m->st));
     if (b->errors_per_read) SWM_CUDA(cudaMemcpyAsync(m->d_e, src_e, n, cudaMemcpyHostToDevice, m->st));
+    // the lengths and thresholds are looked over while the reads are copied
+    rc = check_host_reads(m, b->reads_len, b->errors_per_read, n, b->stride);
+    if (rc) {
+        cudaStreamSynchronize(m->st); // the caller's buffers are its own again
+        return rc;
+    }
     m->h2d_pending = bytes + n * 4 + (b->errors_per_read ? n : 0);
     return SWM_OK;
 }

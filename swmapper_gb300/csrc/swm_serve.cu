@@ -385,10 +385,10 @@ extern "C" int swm_serve_submit(swm_server *s, const swm_batch *b, uint64_t *id)
         return SWM_ERR_ARG;
     }
     const uint64_t n = b->reads_num, sstride = s->cfg.stride;
-    const uint32_t klong = s->ix->k + SWM_SEED_STEP - 1;
+    const uint32_t seeds = 17 * (s->ix->k + SWM_SEED_STEP - 1) - 1; // longest read of 16 long seeds
     for (uint64_t r = 0; r < n; r++) {
         const uint32_t L = b->reads_len[r];
-        if (L > SWM_MAX_READ_LEN || L > b->stride || L > sstride || L / klong > 16 ||
+        if (L > SWM_MAX_READ_LEN || L > b->stride || L > sstride || L > seeds ||
             (b->errors_per_read && b->errors_per_read[r] > SWM_MAX_ERRORS)) {
             swm_set_error("swm_serve_submit: read %llu: length %u or threshold outside the envelope "
                           "(L <= %d, L <= the request and server strides, e <= %d)",
