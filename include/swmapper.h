@@ -231,8 +231,8 @@ int swm_map_wait_packed(swm_mapper *m, swm_packed_result *r);
 
 int swm_mapper_stats(const swm_mapper *m, swm_map_stats *s);
 
-/* Per-stage device time of the last block in milliseconds (CUDA events on the
- * mapper's stream); names are "seed", "plan", "candidates", "compact",
+/* Per-stage device time of the last block in milliseconds (the device's clock
+ * where each stage's first kernel starts); names are "seed", "plan", "candidates", "compact",
  * "verify", "traceback", "records", "total". Returns SWM_ERR_ARG for an
  * unknown name. */
 int swm_mapper_stage_ms(const swm_mapper *m, const char *stage, float *ms);

@@ -50,7 +50,8 @@ enum {
     ST_LOCS,
     ST_STEPS, // Myers steps (read bases) run by k_verify
     ST_KEPT,  // positions the flank filter kept, before each batch's merge
-    ST_N
+    ST_T0,    // start of each stage and the block's end (global timer, ns)
+    ST_N = ST_T0 + 8
 };
 // device totals (u32), written by the scans
 enum {
@@ -165,6 +166,25 @@ struct MapBufs {
     uint64_t scan_tiles;
 };
 
+// Stage i of the block starts here (its first kernel, after in_order).
+__device__ __forceinline__ void stamp(const MapBufs &B, int i) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        B.stat[ST_T0 + i] = t;
+    }
+}
+
+// in_order for a kernel whose successor is a persistent one of a full SM's
+// blocks: launched while this one runs, those go where there is room and stay
+// unevenly spread (524,288 reads: tracebacks 8% slower), so only a small block's,
+// which leave the chip half empty anyway, are launched early.
+#define EARLY_ITEMS 32768
+__device__ __forceinline__ void in_order(const MapBufs &B) {
+    cudaGridDependencySynchronize();
+    if (B.par->nitems <= EARLY_ITEMS) cudaTriggerProgrammaticLaunchCompletion();
+}
+
 // Forms of the verification stage (swm_mapper_tuning); all give the same
 // results. HEAD32 / HEAD64: a head pass over the first 32 / 64 bases of every
 // candidate, then a tail pass over the ones still alive. STREAM8 / STREAM16:
@@ -210,7 +230,6 @@ struct swm_mapper {
     int have_result;
     uint32_t tot[TOT_N];
     swm_map_stats stats;
-    cudaEvent_t ev[9];
     cudaStream_t side[2];      // branches of the captured pipeline (the planners)
     cudaEvent_t fork, join[2];
     float stage_ms[8];
@@ -263,6 +282,15 @@ __device__ __forceinline__ uint32_t even_bits(uint32_t x) {
     return x;
 }
 
+// Every kernel of a block starts with this: nothing is read or written before
+// the kernel before it is complete, and the next one may be launched once all
+// its blocks are running (programmatic dependent launch: a launch and the event
+// node between two stages cost 2-3 us of a small block's 16; 16 reads took 167 us
+// with them and 125 without, 4,096 reads on 1 Gbp 455 and 421).
+__device__ __forceinline__ void in_order() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
 struct ReadView { // base i of the strand being mapped (reverse_read, mapper_cpe.c:2429-2450)
     const char *src;
     uint32_t L, strand;
@@ -325,6 +353,7 @@ struct SeedSmem {
 #define SK(arr, w, t) S.arr[(w)][((t) + (w)) & 31]
 
 __global__ void __launch_bounds__(SEED_WARPS * 32) k_seed(const uint32_t *__restrict__ off, uint32_t k, MapBufs B) {
+    in_order();
     __shared__ SeedSmem sm_all[SEED_WARPS];
     const BlockParams P = *B.par;
     const char *__restrict__ reads = P.reads;
@@ -742,6 +771,7 @@ template <uint32_t K, int NL, bool TABLE>
 // candidate table is in use, so each long seed's table key is stored too.
 __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs B,
                                                            uint32_t lo_len, uint32_t hi_len) {
+    in_order();
     constexpr uint32_t KL = K + SWM_SEED_STEP - 1;
     constexpr int NW = (NL * KL + 15) / 16 < 16 ? (NL * KL + 15) / 16 : 16; // 2-bit words the seeds lie in
     const BlockParams P = *B.par;
@@ -1068,6 +1098,7 @@ __device__ __forceinline__ uint32_t refill_key(const uint32_t *__restrict__ pos,
 // to B.par, and the totals, statistics and scan states cleared.
 __global__ void __launch_bounds__(1024) k_begin(const BlockParams *__restrict__ h, MapBufs B) {
     __shared__ BlockParams P;
+    in_order();
     const uint32_t words = sizeof(BlockParams) / 4;
     if (threadIdx.x < words) {
         const uint32_t v = reinterpret_cast<const volatile uint32_t *>(h)[threadIdx.x];
@@ -1079,6 +1110,7 @@ __global__ void __launch_bounds__(1024) k_begin(const BlockParams *__restrict__ 
         if (threadIdx.x < ST_N) B.stat[threadIdx.x] = 0;
     }
     __syncthreads();
+    stamp(B, 0);
     const uint64_t tiles = (P.nitems + SCAN_TILE_ITEMS - 1) / SCAN_TILE_ITEMS;
     const uint64_t n = tiles * SCAN_VALUES;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
@@ -1104,11 +1136,14 @@ struct ScanItems {
     const uint32_t *in[3];
     uint32_t *out[3];
     uint32_t tot[3], row, ticket; // TOT_ index of each total, first row of states, TOT_ index of the ticket
+    int stage;                    // the stage that starts here, or -1
 };
 #define SCAN_SPIN_LIMIT (1u << 22)
 
 template <int KIN, bool UNM>
 __global__ void __launch_bounds__(256) k_scan_items(MapBufs B, ScanItems A) {
+    in_order();
+    if (A.stage >= 0) stamp(B, A.stage);
     constexpr int V = SCAN_TILE_ITEMS / 256, K = KIN + (UNM ? 1 : 0);
     static_assert(V == 8, "two 16-byte loads a thread");
     __shared__ unsigned long long wsum[K][8], before[K], sum[K];
@@ -1228,6 +1263,7 @@ __device__ __forceinline__ bool several_batches(uint32_t nref, uint32_t nel) { r
 // kernel without the candidate table gathers from them; k_cand_table reads
 // chunks only of items with several batches).
 __global__ void __launch_bounds__(256) k_plan_list(MapBufs B, uint64_t cap_chunks, bool chunks) {
+    in_order();
     const uint32_t nitems = B.par->nitems;
     const uint32_t lane = lane_id();
     for (uint32_t base = blockIdx.x * 256 + (threadIdx.x & ~31u); base < nitems; base += gridDim.x * 256) {
@@ -1310,6 +1346,7 @@ struct PlanSmem {
 __global__ void __launch_bounds__(PLAN_WARPS * 32) k_plan(const uint32_t *__restrict__ pos,
                                                           const uint32_t *__restrict__ keys32, MapBufs B,
                                                           uint64_t cap_chunks, uint64_t cap_elems) {
+    in_order();
     __shared__ PlanSmem sm_all[PLAN_WARPS];
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
     PlanSmem &S = sm_all[wib];
@@ -1521,6 +1558,7 @@ template <uint32_t SEEDS>
 __global__ void __launch_bounds__(PLAN_LANE_WARPS * 32) k_plan_lanes(const uint32_t *__restrict__ pos,
                                                                      const uint32_t *__restrict__ keys32, MapBufs B,
                                                                      uint64_t cap_chunks, uint64_t cap_elems) {
+    in_order();
     extern __shared__ __align__(16) unsigned char plan_smem[];
     const uint32_t lane = lane_id();
     PlanLaneSmem<SEEDS> &S = reinterpret_cast<PlanLaneSmem<SEEDS> *>(plan_smem)[threadIdx.x >> 5];
@@ -1840,6 +1878,8 @@ struct CandSmem {
 __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS) k_cand(const uint32_t *__restrict__ pos,
                                                              const uint16_t *__restrict__ lsd, MapBufs B,
                                                              uint64_t cap_chunks, uint64_t cap_elems, uint32_t klong) {
+    in_order();
+    stamp(B, 2);
     const uint32_t nitems = B.par->nitems;
     __shared__ CandSmem sm_all[CAND_WARPS];
     if (B.tot[TOT_FLAGS] != 0 || B.tot[TOT_CHUNKS] > cap_chunks || B.tot[TOT_ELEMS] > cap_elems) return;
@@ -2031,6 +2071,8 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS)
     k_cand_table(const uint32_t *__restrict__ pos, const uint16_t *__restrict__ lsd,
                  const uint32_t *__restrict__ ctab_off, const uint32_t *__restrict__ ctab_pos, MapBufs B,
                  uint64_t cap_chunks, uint64_t cap_elems, uint32_t klong) {
+    in_order();
+    stamp(B, 2);
     const uint32_t nitems = B.par->nitems;
     __shared__ CandTabSmem sm_all[CAND_WARPS];
     if (B.tot[TOT_FLAGS] != 0 || B.tot[TOT_CHUNKS] > cap_chunks || B.tot[TOT_ELEMS] > cap_elems) return;
@@ -2190,6 +2232,7 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS)
 
 __global__ void __launch_bounds__(256) k_compact(MapBufs B, uint64_t cap_chunks, uint64_t cap_elems,
                                                  uint64_t cap_cands) {
+    in_order(B);
     const uint32_t nitems = B.par->nitems;
     if (B.tot[TOT_FLAGS] != 0 || B.tot[TOT_CHUNKS] > cap_chunks || B.tot[TOT_ELEMS] > cap_elems) return;
     const uint32_t lane = lane_id();
@@ -2464,6 +2507,8 @@ __global__ void __launch_bounds__(128, HEAD ? 10 : 0) k_verify(const uint32_t *_
                                                 uint64_t b2_words, uint64_t ref_length, MapBufs B,
                                                 uint64_t cap_chunks, uint64_t cap_elems, uint64_t cap_cands,
                                                 uint64_t cap_arena) {
+    in_order(B);
+    if (HEAD) stamp(B, 4);
     if (block_failed(B, cap_chunks, cap_elems, cap_cands)) return;
     const uint32_t *__restrict__ lens = B.par->lens;
     uint64_t n;
@@ -2620,6 +2665,8 @@ template <int CH>
 __global__ void __launch_bounds__(128, VERIFY_BLOCKS_PER_SM)
     k_verify_stream(const uint32_t *__restrict__ b2, uint64_t b2_words, uint64_t ref_length, MapBufs B,
                     uint64_t cap_chunks, uint64_t cap_elems, uint64_t cap_cands) {
+    in_order(B);
+    stamp(B, 4);
     static_assert(CH == 8 || CH == 16, "a chunk moves the window by at most one word pair");
     if (block_failed(B, cap_chunks, cap_elems, cap_cands)) return;
     const uint2 *__restrict__ b2p = reinterpret_cast<const uint2 *>(b2); // (lo, hi) word pairs
@@ -2812,6 +2859,8 @@ template <int CH>
 __global__ void __launch_bounds__(128, VERIFY_BLOCKS_PER_SM)
     k_verify_pair(const uint32_t *__restrict__ b2, uint64_t b2_words, uint64_t ref_length, MapBufs B,
                   uint64_t cap_chunks, uint64_t cap_elems, uint64_t cap_cands) {
+    in_order(B);
+    stamp(B, 4);
     static_assert(CH == 16, "a chunk is 16 read bases: one halfword of read bits per half");
     if (block_failed(B, cap_chunks, cap_elems, cap_cands)) return;
     const uint2 *__restrict__ b2p = reinterpret_cast<const uint2 *>(b2);
@@ -2991,6 +3040,7 @@ __global__ void __launch_bounds__(128, VERIFY_BLOCKS_PER_SM)
 __global__ void __launch_bounds__(128, 8) k_verify_finish(const uint32_t *__restrict__ b2, uint64_t b2_words,
                                                        uint64_t ref_length, MapBufs B, uint64_t cap_chunks,
                                                        uint64_t cap_elems, uint64_t cap_cands, uint64_t cap_arena) {
+    in_order(B);
     if (block_failed(B, cap_chunks, cap_elems, cap_cands)) return;
     const uint2 *__restrict__ b2p = reinterpret_cast<const uint2 *>(b2);
     const uint64_t npairs = b2_words / 2;
@@ -3280,6 +3330,8 @@ __device__ __noinline__ void traceback_slow(const uint32_t *__restrict__ b2, uin
 __global__ void __launch_bounds__(TB_THREADS) k_traceback(const uint32_t *__restrict__ b2, uint64_t b2_words,
                                                           uint64_t ref_length, MapBufs B, uint64_t cap_chunks,
                                                           uint64_t cap_elems, uint64_t cap_cands, uint64_t cap_arena) {
+    in_order(B);
+    stamp(B, 5);
     __shared__ TbSmem T;
     if (block_failed(B, cap_chunks, cap_elems, cap_cands)) return;
     const uint32_t *__restrict__ lens = B.par->lens;
@@ -3623,6 +3675,8 @@ template <bool WRITE>
 __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks, uint64_t cap_elems,
                                                  uint64_t cap_cands, uint64_t cap_recs, uint64_t cap_words,
                                                  uint64_t cap_bytes, uint32_t *h_tot, unsigned long long *h_stat) {
+    in_order();
+    if (!WRITE) stamp(B, 6);
     const bool failed = block_failed(B, cap_chunks, cap_elems, cap_cands);
     const uint32_t nitems = B.par->nitems, lane = lane_id();
     const uint8_t *__restrict__ vflag = B.vr_flag;
@@ -3757,7 +3811,8 @@ __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks,
     __syncthreads();
     if (!s_last) return;
     if (threadIdx.x < TOT_N) h_tot[threadIdx.x] = __ldcg(&B.tot[threadIdx.x]);
-    if (threadIdx.x < ST_N) h_stat[threadIdx.x] = __ldcg(&B.stat[threadIdx.x]);
+    if (threadIdx.x < ST_N - 1) h_stat[threadIdx.x] = __ldcg(&B.stat[threadIdx.x]);
+    if (threadIdx.x == ST_N - 1) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(h_stat[ST_N - 1]));
 }
 
 // ======================================================================
@@ -3914,8 +3969,6 @@ extern "C" int swm_mapper_create(swm_index *ix, uint64_t max_reads, swm_mapper *
     m->vmode = VMODE_STREAM16;
     int rc = SWM_OK;
     if (cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking) != cudaSuccess) rc = SWM_ERR_CUDA;
-    for (int i = 0; i < 9 && rc == SWM_OK; i++)
-        if (cudaEventCreate(&m->ev[i]) != cudaSuccess) rc = SWM_ERR_CUDA;
     if (rc == SWM_OK && cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming) != cudaSuccess) rc = SWM_ERR_CUDA;
     for (int i = 0; i < 2 && rc == SWM_OK; i++)
         if (cudaStreamCreateWithFlags(&m->side[i], cudaStreamNonBlocking) != cudaSuccess ||
@@ -3961,8 +4014,6 @@ extern "C" void swm_mapper_free(swm_mapper *m) {
     cudaFreeHost(m->h_tot);
     cudaFreeHost(m->h_stat);
     cudaFreeHost(m->h_par);
-    for (int i = 0; i < 9; i++)
-        if (m->ev[i]) cudaEventDestroy(m->ev[i]);
     if (m->fork) cudaEventDestroy(m->fork);
     for (int i = 0; i < 2; i++) {
         if (m->join[i]) cudaEventDestroy(m->join[i]);
@@ -3972,124 +4023,108 @@ extern "C" void swm_mapper_free(swm_mapper *m) {
     free(m);
 }
 
-#define LAUNCH_CHECK()                                                                              \
-    do {                                                                                            \
-        cudaError_t e_ = cudaGetLastError();                                                        \
-        if (e_ != cudaSuccess) {                                                                    \
-            swm_set_error("kernel launch: %s", cudaGetErrorString(e_));                             \
-            return SWM_ERR_CUDA;                                                                    \
-        }                                                                                           \
-    } while (0)
+// Launch f; overlap: while the kernel before it on the stream runs (both start
+// with in_order).
+template <typename... P, typename... A>
+static cudaError_t launch(void (*f)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, bool overlap,
+                          A... args) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&c, f, static_cast<P>(args)...);
+}
 
 // The whole pipeline of one block on st, every size read on the device (the
 // grids cover the buffers' capacity; kernels loop over what the block has).
 // Captured into the mapper's graph; gclass picks the seed kernel.
 static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     MapBufs &B = m->b;
-    const uint64_t ci = m->cap_items;
+    const uint64_t ci = m->cap_items, cch = m->cap_chunks, cel = m->cap_elems, cca = m->cap_cands;
     const unsigned scan_grid = (unsigned)B.scan_tiles;
     const swm_index *ix = m->ix;
+    const BlockParams *h_par = m->h_par;
     m->launches = 0;
-    k_begin<<<grid_cap(B.scan_tiles * SCAN_VALUES, 1024, 1), 1024, 0, st>>>(m->h_par, B);
-    m->launches++;
-    // stage events: external records become event nodes of the captured graph
-    SWM_CUDA(cudaEventRecordWithFlags(m->ev[0], st, cudaEventRecordExternal));
+#define LAUNCH(...)                   \
+    do {                              \
+        SWM_CUDA(launch(__VA_ARGS__)); \
+        m->launches++;                \
+    } while (0)
+    LAUNCH(k_begin, grid_cap(B.scan_tiles * SCAN_VALUES, 1024, 1), 1024, 0, st, false, h_par, B);
     const uint32_t short_max = SEED_SHORT_MAX(ix->k);
     const bool table = ix->d_ctab_off && ix->k == K12;
     auto seed10 = table ? k_seed12<12, 10, true> : ix->k == 10 ? k_seed12<10, 10, false> : ix->k == 11 ? k_seed12<11, 10, false>
                 : ix->k == 13 ? k_seed12<13, 10, false> : ix->k == 14 ? k_seed12<14, 10, false> : k_seed12<12, 10, false>;
     auto seed16 = table ? k_seed12<12, 16, true> : ix->k == 10 ? k_seed12<10, 16, false> : ix->k == 11 ? k_seed12<11, 16, false>
                 : ix->k == 13 ? k_seed12<13, 16, false> : ix->k == 14 ? k_seed12<14, 16, false> : k_seed12<12, 16, false>;
+    const unsigned g10 = grid_cap(ci, SEED12_THREADS, 16), g16 = grid_cap(ci, SEED12_THREADS, 8);
     if (gclass == 1) {
-        seed10<<<grid_cap(ci, SEED12_THREADS, 16), SEED12_THREADS, 0, st>>>(ix->d_off, B, 0u, 0xffffffffu);
+        LAUNCH(seed10, g10, SEED12_THREADS, 0, st, true, ix->d_off, B, 0u, 0xffffffffu);
     } else if (gclass == 2) { // each read to the instantiation of its length
-        seed10<<<grid_cap(ci, SEED12_THREADS, 16), SEED12_THREADS, 0, st>>>(ix->d_off, B, 0u, short_max);
-        seed16<<<grid_cap(ci, SEED12_THREADS, 8), SEED12_THREADS, 0, st>>>(ix->d_off, B, short_max + 1, 0xffffffffu);
-        m->launches++;
-    } else
-        k_seed<<<grid_cap(ci, SEED_WARPS * 32, 8), SEED_WARPS * 32, 0, st>>>(ix->d_off, ix->k, B);
-    m->launches++;
-    LAUNCH_CHECK();
-    SWM_CUDA(cudaEventRecordWithFlags(m->ev[1], st, cudaEventRecordExternal));
-    k_scan_items<2, false><<<scan_grid, 256, 0, st>>>(
-        B, ScanItems{{B.it_nch, B.it_nel}, {B.it_choff, B.it_eloff}, {TOT_CHUNKS, TOT_ELEMS}, 0, TOT_SC1});
-    m->launches++;
-    k_plan_list<<<grid_cap(ci, 256, 8), 256, 0, st>>>(B, m->cap_chunks, !table);
-    m->launches++;
-    LAUNCH_CHECK();
+        LAUNCH(seed10, g10, SEED12_THREADS, 0, st, true, ix->d_off, B, 0u, short_max);
+        LAUNCH(seed16, g16, SEED12_THREADS, 0, st, true, ix->d_off, B, short_max + 1, 0xffffffffu);
+    } else {
+        LAUNCH(k_seed, grid_cap(ci, SEED_WARPS * 32, 8), SEED_WARPS * 32, 0, st, true, ix->d_off, ix->k, B);
+    }
+    LAUNCH(k_scan_items<2, false>, scan_grid, 256, 0, st, true, B,
+           ScanItems{{B.it_nch, B.it_nel}, {B.it_choff, B.it_eloff}, {TOT_CHUNKS, TOT_ELEMS}, 0, TOT_SC1, 1});
+    LAUNCH(k_plan_list, grid_cap(ci, 256, 8), 256, 0, st, true, B, cch, !table);
     // the three planners beside each other: each waits on the serial schedules of
     // its longest items
     SWM_CUDA(cudaEventRecord(m->fork, st));
     for (int i = 0; i < 2; i++) SWM_CUDA(cudaStreamWaitEvent(m->side[i], m->fork, 0));
-    k_plan<<<grid_cap(ci, PLAN_WARPS * 32, 6), PLAN_WARPS * 32, 0, m->side[0]>>>(ix->d_pos, ix->d_keys32, B, m->cap_chunks,
-                                                                                m->cap_elems);
+    LAUNCH(k_plan, grid_cap(ci, PLAN_WARPS * 32, 6), PLAN_WARPS * 32, 0, m->side[0], false, ix->d_pos, ix->d_keys32, B, cch,
+           cel);
     const size_t smem_few = sizeof(PlanLaneSmem<PLAN_LANE_SEEDS>) * PLAN_LANE_WARPS,
                  smem_more = sizeof(PlanLaneSmem<SWM_MAX_SEL>) * PLAN_LANE_WARPS;
     SWM_CUDA(cudaFuncSetAttribute(k_plan_lanes<SWM_MAX_SEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_more));
-    k_plan_lanes<SWM_MAX_SEL><<<grid_cap(ci, PLAN_LANE_WARPS * 32, 4), PLAN_LANE_WARPS * 32, smem_more, m->side[1]>>>(
-        ix->d_pos, ix->d_keys32, B, m->cap_chunks, m->cap_elems);
-    k_plan_lanes<PLAN_LANE_SEEDS><<<grid_cap(ci, PLAN_LANE_WARPS * 32, 8), PLAN_LANE_WARPS * 32, smem_few, st>>>(
-        ix->d_pos, ix->d_keys32, B, m->cap_chunks, m->cap_elems);
+    LAUNCH(k_plan_lanes<SWM_MAX_SEL>, grid_cap(ci, PLAN_LANE_WARPS * 32, 4), PLAN_LANE_WARPS * 32, smem_more, m->side[1],
+           false, ix->d_pos, ix->d_keys32, B, cch, cel);
+    LAUNCH(k_plan_lanes<PLAN_LANE_SEEDS>, grid_cap(ci, PLAN_LANE_WARPS * 32, 8), PLAN_LANE_WARPS * 32, smem_few, st, false,
+           ix->d_pos, ix->d_keys32, B, cch, cel);
     for (int i = 0; i < 2; i++) {
         SWM_CUDA(cudaEventRecord(m->join[i], m->side[i]));
         SWM_CUDA(cudaStreamWaitEvent(st, m->join[i], 0));
     }
-    m->launches += 3;
-    LAUNCH_CHECK();
-    SWM_CUDA(cudaEventRecordWithFlags(m->ev[2], st, cudaEventRecordExternal));
     if (table)
-        k_cand_table<<<cand_grid(m), CAND_WARPS * 32, 0, st>>>(ix->d_pos, ix->d_ls, ix->d_ctab_off, ix->d_ctab_pos, B,
-                                                               m->cap_chunks, m->cap_elems, ix->k + SWM_SEED_STEP - 1);
+        LAUNCH(k_cand_table, cand_grid(m), CAND_WARPS * 32, 0, st, false, ix->d_pos, ix->d_ls, ix->d_ctab_off, ix->d_ctab_pos,
+               B, cch, cel, ix->k + SWM_SEED_STEP - 1);
     else
-        k_cand<<<cand_grid(m), CAND_WARPS * 32, 0, st>>>(ix->d_pos, ix->d_ls, B, m->cap_chunks, m->cap_elems,
-                                                         ix->k + SWM_SEED_STEP - 1);
-    m->launches++;
-    LAUNCH_CHECK();
-    SWM_CUDA(cudaEventRecordWithFlags(m->ev[3], st, cudaEventRecordExternal));
-    k_scan_items<1, false><<<scan_grid, 256, 0, st>>>(B, ScanItems{{B.it_ncand}, {B.it_coff}, {TOT_CANDS}, 2, TOT_SC2});
-    m->launches++;
-    k_compact<<<grid_cap(ci, 256, 8), 256, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands);
-    m->launches++;
-    LAUNCH_CHECK();
-    SWM_CUDA(cudaEventRecordWithFlags(m->ev[4], st, cudaEventRecordExternal));
-    {
-        const unsigned vg = grid_cap(m->cap_cands, 128, 16);
-        const uint64_t nw = ix->n_words2 + SWM_PAD_WORDS;
-        if (vmode == VMODE_STREAM8 || vmode == VMODE_STREAM16 || vmode == VMODE_PAIR16) {
-            auto stream = vmode == VMODE_STREAM8 ? k_verify_stream<8>
-                          : vmode == VMODE_STREAM16 ? k_verify_stream<16> : k_verify_pair<16>;
-            stream<<<grid_cap(m->cap_cands, 128, VERIFY_BLOCKS_PER_SM), 128, 0, st>>>(ix->d_b2, nw, ix->ref_length, B, m->cap_chunks,
-                                                                     m->cap_elems, m->cap_cands);
-            k_verify_finish<<<vg, 128, 0, st>>>(ix->d_b2, nw, ix->ref_length, B, m->cap_chunks, m->cap_elems,
-                                                m->cap_cands, m->cap_arena);
-        } else {
-            auto head = vmode == VMODE_HEAD32 ? k_verify<true, 1> : k_verify<true, 2>;
-            auto tail = vmode == VMODE_HEAD32 ? k_verify<false, 1> : k_verify<false, 2>;
-            head<<<vg, 128, 0, st>>>(ix->d_b2, nw, ix->ref_length, B, m->cap_chunks, m->cap_elems, m->cap_cands,
-                                     m->cap_arena);
-            tail<<<vg, 128, 0, st>>>(ix->d_b2, nw, ix->ref_length, B, m->cap_chunks, m->cap_elems, m->cap_cands,
-                                     m->cap_arena);
-        }
+        LAUNCH(k_cand, cand_grid(m), CAND_WARPS * 32, 0, st, false, ix->d_pos, ix->d_ls, B, cch, cel,
+               ix->k + SWM_SEED_STEP - 1);
+    LAUNCH(k_scan_items<1, false>, scan_grid, 256, 0, st, true, B,
+           ScanItems{{B.it_ncand}, {B.it_coff}, {TOT_CANDS}, 2, TOT_SC2, 3});
+    LAUNCH(k_compact, grid_cap(ci, 256, 8), 256, 0, st, true, B, cch, cel, cca);
+    const unsigned vg = grid_cap(cca, 128, 16);
+    const uint64_t nw = ix->n_words2 + SWM_PAD_WORDS;
+    if (vmode == VMODE_STREAM8 || vmode == VMODE_STREAM16 || vmode == VMODE_PAIR16) {
+        auto stream = vmode == VMODE_STREAM8 ? k_verify_stream<8>
+                      : vmode == VMODE_STREAM16 ? k_verify_stream<16> : k_verify_pair<16>;
+        LAUNCH(stream, grid_cap(cca, 128, VERIFY_BLOCKS_PER_SM), 128, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel,
+               cca);
+        LAUNCH(k_verify_finish, vg, 128, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca, m->cap_arena);
+    } else {
+        auto head = vmode == VMODE_HEAD32 ? k_verify<true, 1> : k_verify<true, 2>;
+        auto tail = vmode == VMODE_HEAD32 ? k_verify<false, 1> : k_verify<false, 2>;
+        LAUNCH(head, vg, 128, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca, m->cap_arena);
+        LAUNCH(tail, vg, 128, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca, m->cap_arena);
     }
-    m->launches += 2;
-    LAUNCH_CHECK();
-    SWM_CUDA(cudaEventRecordWithFlags(m->ev[5], st, cudaEventRecordExternal));
-    k_traceback<<<grid_cap(m->cap_cands, TB_THREADS, 16), TB_THREADS, 0, st>>>(
-        ix->d_b2, ix->n_words2 + SWM_PAD_WORDS, ix->ref_length, B, m->cap_chunks, m->cap_elems, m->cap_cands,
-        m->cap_arena);
-    m->launches++;
-    LAUNCH_CHECK();
-    SWM_CUDA(cudaEventRecordWithFlags(m->ev[6], st, cudaEventRecordExternal));
-    k_records<false><<<grid_cap(ci, 128, 16), 128, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands, m->cap_recs,
-                                                             m->cap_words, m->cap_bytes, nullptr, nullptr);
-    k_scan_items<3, true><<<scan_grid, 256, 0, st>>>(B, ScanItems{{B.it_nrec, B.it_nw, B.it_nb},
-                                                            {B.it_recoff, B.it_woff, B.it_boff},
-                                                            {TOT_RECS, TOT_WORDS, TOT_BYTES}, 3, TOT_SC3});
-    k_records<true><<<grid_cap(ci, 128, 10), 128, 0, st>>>(B, m->cap_chunks, m->cap_elems, m->cap_cands, m->cap_recs,
-                                                            m->cap_words, m->cap_bytes, m->h_tot, m->h_stat);
-    m->launches += 3;
-    LAUNCH_CHECK();
-    SWM_CUDA(cudaEventRecordWithFlags(m->ev[7], st, cudaEventRecordExternal));
+    LAUNCH(k_traceback, grid_cap(cca, TB_THREADS, 16), TB_THREADS, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca,
+           m->cap_arena);
+    LAUNCH(k_records<false>, grid_cap(ci, 128, 16), 128, 0, st, true, B, cch, cel, cca, m->cap_recs, m->cap_words,
+           m->cap_bytes, m->h_tot, m->h_stat);
+    LAUNCH(k_scan_items<3, true>, scan_grid, 256, 0, st, true, B,
+           ScanItems{{B.it_nrec, B.it_nw, B.it_nb}, {B.it_recoff, B.it_woff, B.it_boff}, {TOT_RECS, TOT_WORDS, TOT_BYTES}, 3,
+                     TOT_SC3, -1});
+    LAUNCH(k_records<true>, grid_cap(ci, 128, 10), 128, 0, st, true, B, cch, cel, cca, m->cap_recs, m->cap_words,
+           m->cap_bytes, m->h_tot, m->h_stat);
+#undef LAUNCH
     return SWM_OK;
 }
 
@@ -4241,11 +4276,9 @@ static int finish_block(swm_mapper *m, uint32_t nreads, uint64_t retries, int *a
         *again = 1;
         return alloc_work(m);
     }
-    float t;
     for (int i = 0; i < 8; i++) {
-        const cudaError_t te = cudaEventElapsedTime(&t, m->ev[i < 7 ? i : 0], m->ev[i < 7 ? i + 1 : 7]);
-        m->stage_ms[i] = te == cudaSuccess ? t : 0.0f;
-        if (te != cudaSuccess) cudaGetLastError(); // timing only: no stale error for later calls
+        const unsigned long long *t = m->h_stat + ST_T0;
+        m->stage_ms[i] = (i < 7 ? t[i + 1] - t[i] : t[7] - t[0]) * 1e-6f;
     }
     const unsigned long long *stat = m->h_stat;
     swm_map_stats &S = m->stats;
