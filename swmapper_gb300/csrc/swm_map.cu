@@ -64,6 +64,7 @@ enum {
     TOT_CQ,            // queue head of the candidate stage (items)
     TOT_RQC, TOT_RQW,  // queue heads of the records count and write passes (groups of 32 items)
     TOT_UNM,                   // reads without a location
+    TOT_SS, TOT_SL,            // short and long reads of a block of both (k_seed_split)
     TOT_SC1, TOT_SC2, TOT_SC3, // tile tickets of the scans after the seed, candidate and records-count stages
     TOT_TBDONE, TOT_RDONE,     // blocks of k_traceback and of the records write pass that are through
     TOT_N
@@ -117,6 +118,7 @@ struct BlockParams {
 
 struct MapBufs {
     BlockParams *par;      // the block's inputs (device copy)
+    uint32_t *seed_list;   // reads of a block of several lengths: short ones from the front, long ones from the back
     // per item
     uint32_t *it_w;        // items * 32: [0..15] Myers planes, [16..31] Hamming planes
     uint2 *sel;            // items * 64: (bucket start, count) of the seed of long seed l, shift t at 4 l + t
@@ -239,8 +241,8 @@ struct swm_mapper {
     BlockParams *h_par;        // pinned
     // one captured graph per (seed-kernel class, verification head length),
     // with the buffer and candidate-table generations it was captured with
-    cudaGraphExec_t gx[3][VMODE_N];
-    uint32_t gx_gen[3][VMODE_N], gx_tab[3][VMODE_N];
+    cudaGraphExec_t gx[4][VMODE_N];
+    uint32_t gx_gen[4][VMODE_N], gx_tab[4][VMODE_N];
     uint32_t gen;              // buffer generation now
     int vmode;                 // verification form (VMODE_*)
 };
@@ -606,6 +608,7 @@ __global__ void __launch_bounds__(SEED_WARPS * 32) k_seed(const uint32_t *__rest
 #define K12 12u
 #define SEED_K_MIN 10u // seed lengths with an instantiation of k_seed12
 #define SEED_K_MAX 14u
+#define SEED_SPLIT_READS 8192 // reads of a block of several lengths from which listing them first pays
 #define SEED_SHORT_MAX(k) (10 * ((k) + SWM_SEED_STEP - 1) + (k) + SWM_SEED_STEP - 2) // longest read with 10 long seeds
 #define SEED12_THREADS 64
 // resident blocks per SM the register budget of each k_seed12 is sized for
@@ -764,13 +767,37 @@ __device__ __forceinline__ void seed12_records(const uint32_t (&iw)[NW], const u
     }
 }
 
+// The reads of a block that may hold both kinds, listed by the instantiation
+// that takes them: up to short_max bases the one of 10 long seeds, longer ones
+// the one of 16. (Both instantiations going over every read and leaving out the
+// other's ran each with half its lanes idle, one after the other: 375 us for
+// 200,003 reads of 50-250 bp on 100 Mbp, 262 listed and side by side. Small
+// blocks (below SEED_SPLIT_READS) are left unlisted: the launch and the detour
+// through the list cost a request of 483 reads more than the idle lanes.)
+__global__ void __launch_bounds__(256) k_seed_split(MapBufs B, uint32_t short_max) {
+    in_order();
+    const uint32_t nreads = B.par->nreads, lane = lane_id();
+    const uint32_t *__restrict__ lens = B.par->lens;
+    for (uint32_t r0 = blockIdx.x * 256 + (threadIdx.x & ~31u); r0 < nreads; r0 += gridDim.x * 256) {
+        const uint32_t r = r0 + lane;
+        const bool in = r < nreads, brief = in && lens[r] <= short_max;
+        const uint32_t ms = __ballot_sync(0xffffffffu, brief), ml = __ballot_sync(0xffffffffu, in && !brief);
+        uint32_t at = 0;
+        if (lane == 0 && ms) at = atomicAdd(&B.tot[TOT_SS], (uint32_t)__popc(ms));
+        if (lane == 1 && ml) at = atomicAdd(&B.tot[TOT_SL], (uint32_t)__popc(ml));
+        const uint32_t as = __shfl_sync(0xffffffffu, at, 0), al = __shfl_sync(0xffffffffu, at, 1);
+        if (brief) B.seed_list[as + __popc(ms & lanemask_lt())] = r;
+        else if (in) B.seed_list[nreads - 1 - (al + __popc(ml & lanemask_lt()))] = r;
+    }
+}
+
+// list: the block's reads were listed by length and this kernel takes those of
+// its own (10 long seeds: the short ones); otherwise the reads of lo .. hi bases
+// of all of them (the other instantiation beside it takes the others). TABLE: the candidate table is in use,
+// so each long seed's table key is stored too.
 template <uint32_t K, int NL, bool TABLE>
-// Items whose read length is outside [lo_len, hi_len] belong to the other
-// instantiation launched beside this one (reads of up to SEED_SHORT_MAX bases take the
-// 10-long-seed kernel, longer ones the 16-long-seed kernel). TABLE: the
-// candidate table is in use, so each long seed's table key is stored too.
-__global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs B,
-                                                           uint32_t lo_len, uint32_t hi_len) {
+__global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs B, bool list,
+                                       uint32_t lo_len, uint32_t hi_len) {
     in_order();
     constexpr uint32_t KL = K + SWM_SEED_STEP - 1;
     constexpr int NW = (NL * KL + 15) / 16 < 16 ? (NL * KL + 15) / 16 : 16; // 2-bit words the seeds lie in
@@ -783,13 +810,14 @@ __global__ void SEED12_BOUNDS k_seed12(const uint32_t *__restrict__ off, MapBufs
     uint2 *__restrict__ sel = B.sel;
     uint32_t *__restrict__ it_w = B.it_w;
     const uint32_t tid = threadIdx.x;
-    const uint32_t nitems = 2 * nreads;
     const char *const limit = reads + (uint64_t)nreads * stride;
     const uint64_t pol = l2_keep_policy();
-    for (uint32_t item = blockIdx.x * blockDim.x + tid; item < nitems; item += gridDim.x * blockDim.x) {
+    const uint32_t n = list ? 2 * B.tot[NL == 10 ? TOT_SS : TOT_SL] : 2 * nreads;
+    for (uint32_t i = blockIdx.x * blockDim.x + tid; i < n; i += gridDim.x * blockDim.x) {
         // items 2r and 2r + 1 sit in adjacent lanes (even block size and stride)
         const uint32_t pair = 3u << (lane_id() & ~1u);
-        const uint32_t r = item >> 1, strand = item & 1;
+        const uint32_t r = list ? B.seed_list[NL == 10 ? i >> 1 : nreads - 1 - (i >> 1)] : i >> 1;
+        const uint32_t strand = i & 1, item = 2 * r + strand;
         const uint32_t L = lens[r];
         if (L < lo_len || L > hi_len) continue; // both lanes of the read skip it
         const uint32_t e = e_arr ? e_arr[r] : e_glob;
@@ -3853,7 +3881,7 @@ static int dmalloc(T **p, uint64_t count) {
 }
 
 static void free_bufs(MapBufs &B) {
-    void *ps[] = {B.par, B.it_w, B.sel, B.sel_fl, B.sel_key, B.it_perm, B.unm, B.it_nsel, B.it_e, B.it_nch, B.it_nel, B.it_nbat,
+    void *ps[] = {B.par, B.seed_list, B.it_w, B.sel, B.sel_fl, B.sel_key, B.it_perm, B.unm, B.it_nsel, B.it_e, B.it_nch, B.it_nel, B.it_nbat,
                   B.it_choff, B.it_eloff, B.it_nrec, B.it_nw, B.it_nb, B.it_recoff, B.it_woff, B.it_boff, B.it_ncand, B.plan_list, B.plan_more,
                   B.it_coff, B.ch_g, B.ch_meta, B.bt_c0, B.bt_c1, B.bt_e0, B.bt_cnt, B.sort_scratch, B.cand_ub, B.cc_pos,
                   B.cc_item, B.plan_keys, B.vr_flag, B.vr_loc, B.vr_err, B.vr_mloc, B.vr_tlen, B.vr_cig, B.vr_aoff, B.arena, B.tb_list,
@@ -3869,6 +3897,7 @@ static int alloc_items(swm_mapper *m) {
     MapBufs &B = m->b;
     const uint64_t I = m->cap_items;
     int rc = SWM_OK;
+    rc |= dmalloc(&B.seed_list, I / 2);
     rc |= dmalloc(&B.it_w, I * 32);
     rc |= dmalloc(&B.sel, I * SWM_MAX_SEL);
     rc |= dmalloc(&B.sel_fl, I * SWM_MAX_SEL);
@@ -3995,7 +4024,7 @@ extern "C" void swm_mapper_free(swm_mapper *m) {
     if (!m) return;
     cudaSetDevice(m->device);
     if (m->st) cudaStreamSynchronize(m->st);
-    for (int a = 0; a < 3; a++)
+    for (int a = 0; a < 4; a++)
         for (int h = 0; h < VMODE_N; h++)
             if (m->gx[a][h]) cudaGraphExecDestroy(m->gx[a][h]);
     free_bufs(m->b);
@@ -4057,22 +4086,28 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
         m->launches++;                \
     } while (0)
     LAUNCH(k_begin, grid_cap(B.scan_tiles * SCAN_VALUES, 1024, 1), 1024, 0, st, false, h_par, B);
-    const uint32_t short_max = SEED_SHORT_MAX(ix->k);
     const bool table = ix->d_ctab_off && ix->k == K12;
     auto seed10 = table ? k_seed12<12, 10, true> : ix->k == 10 ? k_seed12<10, 10, false> : ix->k == 11 ? k_seed12<11, 10, false>
                 : ix->k == 13 ? k_seed12<13, 10, false> : ix->k == 14 ? k_seed12<14, 10, false> : k_seed12<12, 10, false>;
     auto seed16 = table ? k_seed12<12, 16, true> : ix->k == 10 ? k_seed12<10, 16, false> : ix->k == 11 ? k_seed12<11, 16, false>
                 : ix->k == 13 ? k_seed12<13, 16, false> : ix->k == 14 ? k_seed12<14, 16, false> : k_seed12<12, 16, false>;
     const unsigned g10 = grid_cap(ci, SEED12_THREADS, 16), g16 = grid_cap(ci, SEED12_THREADS, 8);
-    if (gclass == 1) {
-        LAUNCH(seed10, g10, SEED12_THREADS, 0, st, true, ix->d_off, B, 0u, 0xffffffffu);
-    } else if (gclass == 2) { // each read to the instantiation of its length
-        LAUNCH(seed10, g10, SEED12_THREADS, 0, st, true, ix->d_off, B, 0u, short_max);
-        LAUNCH(seed16, g16, SEED12_THREADS, 0, st, true, ix->d_off, B, short_max + 1, 0xffffffffu);
-    } else {
+    const uint32_t short_max = SEED_SHORT_MAX(ix->k);
+    if (gclass == 0) {
         LAUNCH(k_seed, grid_cap(ci, SEED_WARPS * 32, 8), SEED_WARPS * 32, 0, st, true, ix->d_off, ix->k, B);
+    } else if (gclass == 1) {
+        LAUNCH(seed10, g10, SEED12_THREADS, 0, st, true, ix->d_off, B, false, 0u, 0xffffffffu);
+    } else { // each read to the instantiation of its length, both at once
+        const bool list = gclass == 3;
+        if (list) LAUNCH(k_seed_split, grid_cap(m->max_reads, 256, 8), 256, 0, st, true, B, short_max);
+        SWM_CUDA(cudaEventRecord(m->fork, st));
+        SWM_CUDA(cudaStreamWaitEvent(m->side[0], m->fork, 0));
+        LAUNCH(seed16, g16, SEED12_THREADS, 0, m->side[0], false, ix->d_off, B, list, short_max + 1, 0xffffffffu);
+        LAUNCH(seed10, g10, SEED12_THREADS, 0, st, false, ix->d_off, B, list, 0u, short_max);
+        SWM_CUDA(cudaEventRecord(m->join[0], m->side[0]));
+        SWM_CUDA(cudaStreamWaitEvent(st, m->join[0], 0));
     }
-    LAUNCH(k_scan_items<2, false>, scan_grid, 256, 0, st, true, B,
+    LAUNCH(k_scan_items<2, false>, scan_grid, 256, 0, st, gclass <= 1, B,
            ScanItems{{B.it_nch, B.it_nel}, {B.it_choff, B.it_eloff}, {TOT_CHUNKS, TOT_ELEMS}, 0, TOT_SC1, 1});
     LAUNCH(k_plan_list, grid_cap(ci, 256, 8), 256, 0, st, true, B, cch, !table);
     // the three planners beside each other: each waits on the serial schedules of
@@ -4138,7 +4173,7 @@ static void drop_graph(swm_mapper *m, int gclass, int h) {
 // synchronisation.
 static int enqueue(swm_mapper *m, const char *d_reads, const uint32_t *d_lens, uint64_t stride, uint32_t nreads,
                    uint32_t errors, const uint8_t *d_e) {
-    const int gclass = m->ix->k < SEED_K_MIN || m->ix->k > SEED_K_MAX ? 0 : (stride <= SEED_SHORT_MAX(m->ix->k) ? 1 : 2);
+    const int gclass = m->ix->k < SEED_K_MIN || m->ix->k > SEED_K_MAX ? 0 : stride <= SEED_SHORT_MAX(m->ix->k) ? 1 : nreads < SEED_SPLIT_READS ? 2 : 3;
     BlockParams *P = m->h_par;
     P->reads = d_reads;
     P->lens = d_lens;

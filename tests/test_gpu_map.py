@@ -612,3 +612,23 @@ def test_gpu_refill_schedules_of_every_planner(cuda_lib, n, k, copies, e):
         _check(out, ref.records(), ref.unmapped)
         st = m.stats()
         assert (st["batches"], st["candidates"]) == (ref.stats["batches"], ref.stats["candidates"])
+
+
+@pytest.mark.parametrize("nreads", [8191, 8192, 9001])
+def test_gpu_uneven_blocks_listed_by_length(cuda_lib, nreads):
+    """Blocks of both seed kernels' reads below and from the size at which they
+    are listed by length first, with one kind missing or nearly so as well."""
+    g = genome(250_000, 71)
+    reads, lens, _, _ = synth.reads(g, nreads, 50, 250, 0.03, seed=72, stride=250)
+    eper = np.array([math.ceil(0.05 * int(L)) for L in lens], np.uint8)
+    _, mix = oracle_index(g)
+    m = cuda_lib.Mapper(cuda_lib.Index.build(g), max_reads=nreads)
+    ref_recs, ref_unm = records_by_e(mix, reads, lens, eper, nthreads=8)
+    _check(m.map(reads, lens, 0, errors_per_read=eper), ref_recs, ref_unm)
+    for cut in (164, 165):  # the longest read of 10 long seeds
+        short = np.minimum(lens, cut).astype(np.uint32)
+        ref = po.map_reads(mix, reads, short, 6, nthreads=8)
+        _check(m.map(reads, short, 6), ref.records(), ref.unmapped)
+    long = np.maximum(lens, 165).astype(np.uint32)
+    ref = po.map_reads(mix, reads, long, 6, nthreads=8)
+    _check(m.map(reads, long, 6), ref.records(), ref.unmapped)
