@@ -62,6 +62,7 @@ enum {
     TOT_PLM, TOT_PLMQ, // the same with more selected seeds
     TOT_PLW, TOT_PLWQ, // and those with long schedules; queue head of k_plan
     TOT_CQ,            // queue head of the candidate stage (items)
+    TOT_HV, TOT_HVQ,   // batches of many kept positions (k_cand_heavy) and their queue head
     TOT_RQC, TOT_RQW,  // queue heads of the records count and write passes (groups of 32 items)
     TOT_UNM,                   // reads without a location
     TOT_SS, TOT_SL,            // short and long reads of a block of both (k_seed_split)
@@ -137,7 +138,7 @@ struct MapBufs {
     // per chunk / batch slot (cap_chunks; batch b of an item sits at slot it_choff + b)
     uint32_t *ch_g, *ch_meta;
     uint32_t *bt_c0, *bt_c1, *bt_e0, *bt_cnt; // cap_chunks + cap_items slots
-    uint32_t *sort_scratch; // SWM_BATCH_POSITIONS words per resident k_cand warp
+    uint4 *heavy; // batches k_cand_heavy sorts: {batch slot, first candidate (cand_ub), kept positions, item}
     // upper-bound candidates (cap_elems)
     uint32_t *cand_ub;
     // dense candidates (cap_cands)
@@ -1817,12 +1818,13 @@ __device__ __forceinline__ uint32_t warp_sort_unique(const uint32_t *buf, uint32
     return u;
 }
 
-// The kept (adjusted) positions of one batch, sorted ascending and unique,
-// written to dst (merge + unique of block_heap_sort, mapper_cpe.c:1999-2089);
-// returns how many. They sit in sc (shared memory) or, when spilled, in the
-// warp's global scratch gs (room for SWM_BATCH_POSITIONS).
-__device__ __forceinline__ uint32_t batch_sort_unique(uint32_t *sc, uint32_t *gs, bool spilled, uint32_t kept,
-                                                      uint32_t *dst) {
+#define CAND_SMEM_KEEP 128 // survivors of a batch held in shared memory (more go to its place of cand_ub)
+#define CAND_WARP_SORT 256 // most of them that the batch's warp sorts; k_cand_heavy the others
+
+// The kept (adjusted) positions of one batch, at most CAND_SMEM_KEEP of them in
+// sc, sorted ascending and unique, written to dst (merge + unique of
+// block_heap_sort, mapper_cpe.c:1999-2089); returns how many.
+__device__ __forceinline__ uint32_t batch_sort_unique(uint32_t *sc, uint32_t kept, uint32_t *dst) {
     const uint32_t lane = lane_id();
     uint32_t u = 0;
     if (kept <= 8) {
@@ -1847,44 +1849,87 @@ __device__ __forceinline__ uint32_t batch_sort_unique(uint32_t *sc, uint32_t *gs
         u = __popc(m);
     } else if (kept <= 64) {
         u = warp_sort_unique<2>(sc, kept, dst);
-    } else if (kept <= 128) {
-        u = warp_sort_unique<4>(spilled ? gs : sc, kept, dst);
-    } else if (kept <= 256) {
-        u = warp_sort_unique<8>(gs, kept, dst);
-    } else { // bitonic sort in the warp's global scratch
-        uint32_t n2 = 512;
-        while (n2 < kept) n2 <<= 1;
-        uint32_t *buf = spilled ? gs : sc;
-        for (uint32_t i = kept + lane; i < n2; i += 32) buf[i] = 0xffffffffu;
-        __syncwarp();
-        for (uint32_t size = 2; size <= n2; size <<= 1) {
-            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                for (uint32_t i = lane; i < n2 / 2; i += 32) {
-                    const uint32_t lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
-                    const bool up = ((lo & size) == 0);
-                    const uint32_t a = buf[lo], d = buf[hi];
-                    if ((a > d) == up) {
-                        buf[lo] = d;
-                        buf[hi] = a;
-                    }
-                }
-                __syncwarp();
-            }
-        }
-        for (uint32_t i0 = 0; i0 < kept; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            const bool keep = i < kept && (i == 0 || buf[i - 1] != buf[i]);
-            const uint32_t m = __ballot_sync(0xffffffffu, keep);
-            if (keep) dst[u + __popc(m & lanemask_lt())] = buf[i];
-            u += __popc(m);
-        }
+    } else if (kept <= CAND_SMEM_KEEP) {
+        u = warp_sort_unique<4>(sc, kept, dst);
+    } else {
+        u = warp_sort_unique<8>(dst, kept, dst); // all loaded before the first is stored
     }
     return u;
 }
 
-#define CAND_MAXCH 128 // chunks (runs) per batch: block_size < 256 allows at most 128
+// A batch that kept more than CAND_SMEM_KEEP positions: they are in its place of
+// cand_ub, unsorted, and k_cand_heavy takes it from here.
+__device__ __forceinline__ void push_heavy(const MapBufs &B, uint32_t slot, uint32_t e0, uint32_t kept, uint32_t item) {
+    if (lane_id() == 0) B.heavy[atomicAdd(&B.tot[TOT_HV], 1u)] = make_uint4(slot, e0, kept, item);
+}
 
-#define CAND_SMEM_KEEP 128 // survivors of a batch held in shared memory (more go to global scratch)
+// Sort and unique the batches of more than CAND_WARP_SORT kept positions, a block
+// each, in shared memory. Bound by the exchange steps' barriers (66 for 2,048).
+// A warp of the candidate kernel that sorted such a batch itself in global
+// memory took some 70 us for it while the rest of a small block was long done:
+// candidate stage of 4,096 reads on 1 Gbp 137 -> 56 us, of 65,536 uneven ones on
+// 3 Gbp 445 -> 311, of 524,288 1,665 -> 1,485. Batches of 129 to 256 stay with the
+// warp (8 registers a lane): the block sort of those too was slower at 524,288
+// reads (1,860). Launches nothing early on a large block: with the scan's and the
+// compaction's blocks let in beside it the verification's were spread unevenly
+// in some runs (3,750 -> 5,050).
+#define HEAVY_THREADS 128
+__global__ void __launch_bounds__(HEAVY_THREADS) k_cand_heavy(MapBufs B, uint64_t cap_chunks, uint64_t cap_elems) {
+    in_order(B);
+    if (B.tot[TOT_FLAGS] != 0 || B.tot[TOT_CHUNKS] > cap_chunks || B.tot[TOT_ELEMS] > cap_elems) return;
+    __shared__ uint32_t v[SWM_BATCH_POSITIONS];
+    __shared__ uint32_t next, wsum[HEAVY_THREADS / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = B.tot[TOT_HV];
+    for (;;) {
+        if (tid == 0) next = atomicAdd(&B.tot[TOT_HVQ], 1u);
+        __syncthreads();
+        if (next >= n) break;
+        const uint4 h = B.heavy[next];
+        const uint32_t kept = h.z;
+        uint32_t *dst = B.cand_ub + h.y;
+        uint32_t n2 = 256;
+        while (n2 < kept) n2 <<= 1;
+        for (uint32_t i = tid; i < n2; i += HEAVY_THREADS) v[i] = i < kept ? dst[i] : 0xffffffffu;
+        __syncthreads();
+        for (uint32_t size = 2; size <= n2; size <<= 1) {
+            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+                for (uint32_t i = tid; i < n2 / 2; i += HEAVY_THREADS) {
+                    const uint32_t lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
+                    const uint32_t a = v[lo], d = v[hi];
+                    if ((a > d) == ((lo & size) == 0)) {
+                        v[lo] = d;
+                        v[hi] = a;
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        uint32_t u = 0;
+        for (uint32_t i0 = 0; i0 < kept; i0 += HEAVY_THREADS) {
+            const uint32_t i = i0 + tid;
+            const bool keep = i < kept && (i == 0 || v[i - 1] != v[i]);
+            const uint32_t m = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) wsum[warp] = __popc(m);
+            __syncthreads();
+            uint32_t at = u, all = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < HEAVY_THREADS / 32; w++) {
+                at += w < warp ? wsum[w] : 0u;
+                all += wsum[w];
+            }
+            if (keep) dst[at + __popc(m & lanemask_lt())] = v[i];
+            u += all;
+            __syncthreads();
+        }
+        if (tid == 0) {
+            B.bt_cnt[h.x] = u;
+            atomicAdd(&B.it_ncand[h.w], u);
+        }
+        __syncthreads(); // `next` is read by all
+    }
+}
+
+#define CAND_MAXCH 128 // chunks (runs) per batch: block_size < 256 allows at most 128
 
 struct CandSmem {
     uint32_t gs[CAND_MAXCH];     // first global index of each chunk minus its start in the batch
@@ -1913,8 +1958,6 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS) k_cand(const
     if (B.tot[TOT_FLAGS] != 0 || B.tot[TOT_CHUNKS] > cap_chunks || B.tot[TOT_ELEMS] > cap_elems) return;
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
     CandSmem &S = sm_all[wib];
-    // a warp's survivors past CAND_SMEM_KEEP go to its slice of global scratch
-    auto gscratch = [&]() { return B.sort_scratch + (uint64_t)(blockIdx.x * CAND_WARPS + wib) * SWM_BATCH_POSITIONS; };
     unsigned long long kept_all = 0; // this warp's kept positions, added to the block's count once
     for (uint32_t g0 = warp_take_items(&B.tot[TOT_CQ]), gi = 0; g0 < nitems;) {
         const uint32_t item = g0 + gi;
@@ -1990,7 +2033,7 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS) k_cand(const
                 const uint32_t E = carry;
                 if (lane == 0) S.start[nchk] = (uint16_t)E;
                 __syncwarp();
-                bool spilled = false; // survivors in S.sc, or in global scratch once they outgrow it
+                bool spilled = false; // survivors in S.sc, or in the batch's place of cand_ub once they outgrow it
                 uint32_t kept = 0, cdone = 0; // cdone: chunks that start before eb
                 for (uint32_t eb = 0; eb < E; eb += 32) {
                     const uint32_t el = eb + lane;
@@ -2017,22 +2060,25 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS) k_cand(const
                     }
                     const uint32_t m = __ballot_sync(0xffffffffu, ok);
                     if (!spilled && kept + __popc(m) > CAND_SMEM_KEEP) {
-                        uint32_t *gs = gscratch();
-                        for (uint32_t i = lane; i < kept; i += 32) gs[i] = S.sc[i];
+                        for (uint32_t i = lane; i < kept; i += 32) B.cand_ub[e0 + i] = S.sc[i];
                         spilled = true;
                         __syncwarp();
                     }
                     if (ok) {
                         const uint32_t at = kept + __popc(m & lanemask_lt());
-                        if (spilled) gscratch()[at] = p;
+                        if (spilled) B.cand_ub[e0 + at] = p;
                         else S.sc[at] = p;
                     }
                     kept += __popc(m);
                 }
                 __syncwarp();
-                const uint32_t u = batch_sort_unique(S.sc, gscratch(), spilled, kept, B.cand_ub + e0);
-                if (lane == 0) B.bt_cnt[sbase + b] = u;
-                total += u;
+                if (kept > CAND_WARP_SORT) {
+                    push_heavy(B, sbase + b, e0, kept, item);
+                } else {
+                    const uint32_t u = batch_sort_unique(S.sc, kept, B.cand_ub + e0);
+                    if (lane == 0) B.bt_cnt[sbase + b] = u;
+                    total += u;
+                }
                 kept_all += kept;
                 __syncwarp();
             }
@@ -2106,7 +2152,6 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS)
     if (B.tot[TOT_FLAGS] != 0 || B.tot[TOT_CHUNKS] > cap_chunks || B.tot[TOT_ELEMS] > cap_elems) return;
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
     CandTabSmem &S = sm_all[wib];
-    auto gscratch = [&]() { return B.sort_scratch + (uint64_t)(blockIdx.x * CAND_WARPS + wib) * SWM_BATCH_POSITIONS; };
     unsigned long long kept_all = 0; // this warp's kept positions, added to the block's count once
     for (uint32_t g0 = warp_take_items(&B.tot[TOT_CQ]), gi = 0; g0 < nitems;) {
         const uint32_t item = g0 + gi;
@@ -2230,22 +2275,25 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS)
                     }
                     const uint32_t m = __ballot_sync(0xffffffffu, ok);
                     if (!spilled && kept + __popc(m) > CAND_SMEM_KEEP) {
-                        uint32_t *gs = gscratch();
-                        for (uint32_t i = lane; i < kept; i += 32) gs[i] = S.sc[i];
+                        for (uint32_t i = lane; i < kept; i += 32) B.cand_ub[e0 + i] = S.sc[i];
                         spilled = true;
                         __syncwarp();
                     }
                     if (ok) {
                         const uint32_t at = kept + __popc(m & lanemask_lt());
-                        if (spilled) gscratch()[at] = p;
+                        if (spilled) B.cand_ub[e0 + at] = p;
                         else S.sc[at] = p;
                     }
                     kept += __popc(m);
                 }
                 __syncwarp();
-                const uint32_t u = batch_sort_unique(S.sc, gscratch(), spilled, kept, B.cand_ub + e0);
-                if (lane == 0) B.bt_cnt[sbase + b] = u;
-                total += u;
+                if (kept > CAND_WARP_SORT) {
+                    push_heavy(B, sbase + b, e0, kept, item);
+                } else {
+                    const uint32_t u = batch_sort_unique(S.sc, kept, B.cand_ub + e0);
+                    if (lane == 0) B.bt_cnt[sbase + b] = u;
+                    total += u;
+                }
                 kept_all += kept;
                 __syncwarp();
             }
@@ -3902,7 +3950,7 @@ static int dmalloc(T **p, uint64_t count) {
 static void free_bufs(MapBufs &B) {
     void *ps[] = {B.par, B.seed_list, B.it_w, B.sel, B.sel_fl, B.sel_key, B.it_perm, B.unm, B.it_nsel, B.it_e, B.it_nch, B.it_nel, B.it_nbat,
                   B.it_choff, B.it_eloff, B.it_nrec, B.it_nw, B.it_nb, B.it_recoff, B.it_woff, B.it_boff, B.it_ncand, B.plan_list, B.plan_more,
-                  B.it_coff, B.ch_g, B.ch_meta, B.bt_c0, B.bt_c1, B.bt_e0, B.bt_cnt, B.sort_scratch, B.cand_ub, B.cc_pos,
+                  B.it_coff, B.ch_g, B.ch_meta, B.bt_c0, B.bt_c1, B.bt_e0, B.bt_cnt, B.heavy, B.cand_ub, B.cc_pos,
                   B.cc_item, B.plan_keys, B.vr_flag, B.vr_loc, B.vr_err, B.vr_mloc, B.vr_tlen, B.vr_cig, B.vr_aoff, B.arena, B.tb_list,
                   B.tb_cp, B.slow_list, B.vt_x, B.vt_st, B.vt_cp,
                   B.out_w, B.out_c, B.rec_woff, B.rec_boff, B.rec_blen, B.tot, B.stat, B.scan_state};
@@ -3954,7 +4002,7 @@ static int alloc_work(swm_mapper *m) {
     int rc = SWM_OK;
     m->gen++; // the captured graph holds the old buffers
     cudaFree(B.ch_g); cudaFree(B.ch_meta); cudaFree(B.plan_keys); cudaFree(B.bt_c0); cudaFree(B.bt_c1); cudaFree(B.bt_e0);
-    cudaFree(B.bt_cnt); cudaFree(B.sort_scratch); cudaFree(B.cand_ub); cudaFree(B.cc_pos);
+    cudaFree(B.bt_cnt); cudaFree(B.heavy); cudaFree(B.cand_ub); cudaFree(B.cc_pos);
     cudaFree(B.cc_item); cudaFree(B.vr_flag); cudaFree(B.vr_loc); cudaFree(B.vr_err); cudaFree(B.vr_mloc);
     cudaFree(B.vr_tlen); cudaFree(B.vr_cig); cudaFree(B.vr_aoff); cudaFree(B.arena); cudaFree(B.out_w);
     cudaFree(B.tb_list); cudaFree(B.tb_cp); cudaFree(B.slow_list); cudaFree(B.vt_x); cudaFree(B.vt_st); cudaFree(B.vt_cp);
@@ -3966,7 +4014,7 @@ static int alloc_work(swm_mapper *m) {
     rc |= dmalloc(&B.bt_c1, m->cap_chunks + m->cap_items);
     rc |= dmalloc(&B.bt_e0, m->cap_chunks + m->cap_items);
     rc |= dmalloc(&B.bt_cnt, m->cap_chunks + m->cap_items);
-    rc |= dmalloc(&B.sort_scratch, (uint64_t)cand_grid(m) * CAND_WARPS * SWM_BATCH_POSITIONS);
+    rc |= dmalloc(&B.heavy, m->cap_elems / CAND_WARP_SORT + 1);
     rc |= dmalloc(&B.cand_ub, m->cap_elems);
     rc |= dmalloc(&B.cc_pos, m->cap_cands);
     rc |= dmalloc(&B.cc_item, m->cap_cands);
@@ -4152,6 +4200,8 @@ static int enqueue_ops(swm_mapper *m, cudaStream_t st, int gclass, int vmode) {
     else
         LAUNCH(k_cand, cand_grid(m), CAND_WARPS * 32, 0, st, false, ix->d_pos, ix->d_ls, B, cch, cel,
                ix->k + SWM_SEED_STEP - 1);
+    LAUNCH(k_cand_heavy, grid_cap(m->cap_elems / CAND_WARP_SORT * HEAVY_THREADS, HEAVY_THREADS, 12), HEAVY_THREADS, 0, st, true,
+           B, cch, cel);
     LAUNCH(k_scan_items<1, false>, scan_grid, 256, 0, st, true, B,
            ScanItems{{B.it_ncand}, {B.it_coff}, {TOT_CANDS}, 2, TOT_SC2, 3});
     LAUNCH(k_compact, grid_cap(ci, 256, 8), 256, 0, st, true, B, cch, cel, cca);

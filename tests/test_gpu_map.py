@@ -614,6 +614,29 @@ def test_gpu_refill_schedules_of_every_planner(cuda_lib, n, k, copies, e):
         assert (st["batches"], st["candidates"]) == (ref.stats["batches"], ref.stats["candidates"])
 
 
+@pytest.mark.parametrize("copies", [31, 33, 64, 65, 128, 129, 255, 257, 700, 2047, 2050])
+def test_gpu_batches_of_many_kept_positions(cuda_lib, copies):
+    """Exact copies of one unit, so that a batch keeps `copies` positions of each
+    of its seeds up to the batch's limit: around the sizes at which another sort
+    takes over."""
+    rng = np.random.default_rng(64)
+    unit, step = rng.choice(np.frombuffer(b"ACGT", np.uint8), 130), 170
+    g = genome(copies * step + 50_000, 65)
+    at = np.arange(copies)[:, None] * step + np.arange(130)[None, :]
+    g[at] = unit
+    reads, lens, _, _ = synth.reads(g, 24, 100, 100, 0.02, seed=66)
+    near = np.stack([unit[i:i + 100] for i in range(0, 30, 5)])
+    reads[:6, :100], lens[:6] = near, 100
+    _, mix = oracle_index(g)
+    ref = po.map_reads(mix, reads, lens, 5, nthreads=8, cap_records=100_000)
+    for table in (False, True):
+        ix = cuda_lib.Index.build(g)
+        assert (ix.candidate_table(table) > 0) == table
+        m = cuda_lib.Mapper(ix, max_reads=24)
+        _check(m.map(reads, lens, 5, records_cap=100_000), ref.records(), ref.unmapped)
+        assert m.stats()["candidates"] == ref.stats["candidates"]
+
+
 @pytest.mark.parametrize("nreads", [8191, 8192, 9001])
 def test_gpu_uneven_blocks_listed_by_length(cuda_lib, nreads):
     """Blocks of both seed kernels' reads below and from the size at which they
