@@ -3748,30 +3748,44 @@ __device__ uint32_t records_seq(const MapBufs &B, uint32_t item, uint64_t cap_re
     return nrec;
 }
 
-// Items with at most this many candidates take the one-thread path of
-// k_records (records_seq); the others the warp path.
-#define RECORDS_LIGHT 16
+#define RECORDS_STEP 512 // flags a warp takes at once, 16 bytes a lane
 
-// Records, groups of 32 consecutive items taken from a queue: items with few
-// candidates one thread each (records_seq, all lanes at once), the others
-// one warp each. Most of those need none of the sequential machinery: while
-// num + 8 <= SWM_MAX_CIGAR and len + 256 <= 16 SWM_MAX_CIGAR the flush tests are false,
-// so when the item's passing candidates (P of them, S bytes of [NM, len,
-// text] before dedup) keep within those bounds, or (write pass) the count
-// pass found at most one record, the item is one record of every passing
-// candidate in order except a traceback hit whose location equals the
-// previous passing candidate's (that previous one was then emitted or had
-// the same location itself). The warp reads 32 verdict flags per load, and
-// only the passing lanes read their location and CIGAR; the rest go through
-// records_seq on lane 0. Count pass: the item's record / word / byte counts;
-// write pass: the records; its last
-// block copies the block's totals and statistics to the host.
+// What a warp of k_records keeps of its group of 32 items.
+struct RecordsSmem {
+    uint16_t list[RECORDS_STEP]; // passing candidates of the step: place in it, bit 15 set for a traceback hit
+    uint32_t cb[32];             // items' first candidates
+    uint32_t n[32], by[32];      // count pass: locations and bytes; write pass: the group's running ones at the item's first
+    uint32_t p[32], s[32];       // count pass: passing candidates and bytes before dedup; write pass: the item's out_w and out_c
+};
+
+// Records, groups of 32 consecutive items taken from a queue. Most items need
+// none of the sequential machinery of records_seq: while num + 8 <= SWM_MAX_CIGAR
+// and len + 256 <= 16 SWM_MAX_CIGAR the flush tests are false, so when the item's
+// passing candidates (P of them, S bytes of [NM, len, text] before dedup) keep
+// within those bounds, or (write pass) the count pass found one record, the item
+// is one record of every passing candidate in order except a traceback hit whose
+// location equals the previous passing candidate's (that previous one was then
+// emitted or had the same location itself). The other items go through
+// records_seq, a lane each.
+//
+// Bound by the round trips of a group (queue, items, flags, locations, texts) and
+// the warps in flight. The group's candidates are consecutive, so the warp reads
+// their flags 512 at a time whatever items they belong to, lists the passing ones
+// and takes 32 of those at once, each looking its item up. Items one after
+// another (32 flags a load), those of at most 16 candidates by a lane each, made
+// every item a round trip of its own: both passes of 524,288 reads on 3 Gbp (52
+// candidates an item) 544 us, so 167; of 524,288 on 100 Mbp 172 and 115; of 4,096
+// on 1 Gbp 80 and 25.
+// Count pass: the items' record / word / byte counts; write pass: the records; its
+// last block copies the block's totals and statistics to the host.
 template <bool WRITE>
 __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks, uint64_t cap_elems,
                                                  uint64_t cap_cands, uint64_t cap_recs, uint64_t cap_words,
                                                  uint64_t cap_bytes, uint32_t *h_tot, unsigned long long *h_stat) {
     in_order();
     if (!WRITE) stamp(B, 6);
+    __shared__ RecordsSmem smem[4];
+    RecordsSmem &S = smem[threadIdx.x >> 5];
     const bool failed = block_failed(B, cap_chunks, cap_elems, cap_cands);
     const uint32_t nitems = B.par->nitems, lane = lane_id();
     const uint8_t *__restrict__ vflag = B.vr_flag;
@@ -3786,111 +3800,147 @@ __global__ void __launch_bounds__(128) k_records(MapBufs B, uint64_t cap_chunks,
         if (item0 >= nitems) break;
         // the group's scalars: lane j holds item item0 + j's
         const uint32_t mine = item0 + lane;
-        uint32_t g_cb = 0, g_nc = 0, g_nrec = 0, g_wb = 0, g_bb = 0, g_rb = 0;
-        bool g_ok = true;
+        uint32_t cb = 0xffffffffu, cend = 0, nrec = 0, nwords = 0, wb = 0, bb = 0;
+        bool one = false; // write pass: one record, with room for it
         if (mine < nitems) {
-            g_cb = B.it_coff[mine];
+            cb = B.it_coff[mine];
             const uint32_t nbat = B.it_nbat[mine];
-            g_nc = nbat ? B.it_ncand[mine] : 0u;
+            cend = cb + (nbat ? B.it_ncand[mine] : 0u);
             batches += nbat;
             if (WRITE) {
-                g_nrec = B.it_nrec[mine];
-                g_wb = B.it_woff[mine];
-                g_bb = B.it_boff[mine];
-                g_rb = B.it_recoff[mine];
-                g_ok = (uint64_t)g_rb + g_nrec <= cap_recs && (uint64_t)g_wb + B.it_nw[mine] <= cap_words &&
-                       (uint64_t)g_bb + B.it_nb[mine] <= cap_bytes;
-            }
-        }
-        // items with few candidates: one lane each, all at once (the warp
-        // path below would spend a pass of 32 lanes on a handful of flags)
-        const bool light = mine < nitems && g_nc <= RECORDS_LIGHT;
-        if (light && !(WRITE && g_nrec == 0))
-            records_seq<WRITE>(B, mine, cap_recs, cap_words, cap_bytes, locs_total);
-        const unsigned heavy = __ballot_sync(0xffffffffu, mine < nitems && !light);
-        for (unsigned hm = heavy; hm; hm &= hm - 1) {
-            const uint32_t j = __ffs(hm) - 1;
-            const uint32_t item = item0 + j;
-            const uint32_t cb = __shfl_sync(0xffffffffu, g_cb, j), nc = __shfl_sync(0xffffffffu, g_nc, j);
-            const uint32_t nrec_c = __shfl_sync(0xffffffffu, g_nrec, j);
-            if (WRITE && nrec_c == 0) continue; // nothing passed (or every location deduped)
-            if (WRITE && nrec_c > 1) {          // flushes: the sequential rules
-                if (lane == 0) records_seq<true>(B, item, cap_recs, cap_words, cap_bytes, locs_total);
-                continue;
-            }
-            const uint32_t wbase = __shfl_sync(0xffffffffu, g_wb, j), bbase = __shfl_sync(0xffffffffu, g_bb, j);
-            const bool ok = __shfl_sync(0xffffffffu, (uint32_t)g_ok, j) != 0;
-            uint32_t num = 0, len = 0, P = 0, S = 0, last = 0;
-            bool has = false;
-            for (uint32_t c0 = cb; c0 < cb + nc; c0 += 32) {
-                const uint32_t c = c0 + lane;
-                const uint8_t f = c < cb + nc ? vflag[c] : (uint8_t)VR_FAIL;
-                const bool pass = f == VR_HAM || f == VR_TB;
-                const unsigned pm = __ballot_sync(0xffffffffu, pass);
-                if (!pm) continue;
-                uint32_t loc = 0, tl = 0;
-                if (pass) {
-                    loc = vloc[c];
-                    tl = vtlen[c];
-                }
-                const unsigned below = pm & lanemask_lt();
-                const uint32_t ploc = __shfl_sync(0xffffffffu, loc, below ? 31 - __clz(below) : lane);
-                const bool dup = f == VR_TB && (below ? ploc == loc : (has && last == loc));
-                const bool keep = pass && !dup;
-                const unsigned km = __ballot_sync(0xffffffffu, keep);
-                const uint32_t by = keep ? 2 + tl : 0u;
-                const uint32_t incl = warp_scan_incl(by);
-                if (WRITE && keep && ok) {
-                    out_w[wbase + 2 + num + __popc(km & lanemask_lt())] = loc;
-                    const uint32_t bcur = bbase + len + incl - by;
-                    const uint4 h = *reinterpret_cast<const uint4 *>(vcig + (uint64_t)c * SWM_CIGAR_SLOT);
-                    const uint32_t hw[4] = {h.x, h.y, h.z, h.w};
-                    if (tl + 2 <= 16) {
-#pragma unroll
-                        for (uint32_t q = 0; q < 16; q++)
-                            if (q < tl + 2) out_c[bcur + q] = (uint8_t)(hw[q >> 2] >> (8 * (q & 3)));
+                nrec = B.it_nrec[mine];
+                if (nrec == 1) {
+                    wb = B.it_woff[mine];
+                    bb = B.it_boff[mine];
+                    nwords = B.it_nw[mine];
+                    const uint32_t rb = B.it_recoff[mine], nb = B.it_nb[mine];
+                    one = (uint64_t)rb + 1 <= cap_recs && (uint64_t)wb + nwords <= cap_words && (uint64_t)bb + nb <= cap_bytes;
+                    if (one) {
+                        out_w[wb] = mine;
+                        out_w[wb + 1] = (nwords - 2) | (1u << 31);
+                        B.rec_woff[rb] = wb;
+                        B.rec_boff[rb] = bb;
+                        B.rec_blen[rb] = nb;
                     } else {
-                        out_c[bcur] = (uint8_t)h.x;
-                        out_c[bcur + 1] = (uint8_t)(h.x >> 8);
-                        const uint8_t *tx = (tl <= SWM_CIGAR_SLOT - 2) ? vcig + (uint64_t)c * SWM_CIGAR_SLOT + 2
-                                                                      : B.arena + B.vr_aoff[c];
-                        for (uint32_t q = 0; q < tl; q++) out_c[bcur + 2 + q] = tx[q];
+                        atomicOr(&B.tot[TOT_FLAGS], OV_RECS);
                     }
-                }
-                num += __popc(km);
-                len += __shfl_sync(0xffffffffu, incl, 31);
-                if (!WRITE) {
-                    P += __popc(pm);
-                    S += __reduce_add_sync(0xffffffffu, pass ? 2 + tl : 0u);
-                }
-                last = __shfl_sync(0xffffffffu, loc, 31 - __clz(pm));
-                has = true;
-            }
-            if (!WRITE) {
-                if (P + 8 <= SWM_MAX_CIGAR && S + 16 * 16 <= SWM_MAX_CIGAR * 16) {
-                    if (lane == 0) {
-                        B.it_nrec[item] = num ? 1u : 0u;
-                        B.it_nw[item] = num ? 2 + num : 0u;
-                        B.it_nb[item] = len;
-                    }
-                } else if (lane == 0) {
-                    records_seq<false>(B, item, cap_recs, cap_words, cap_bytes, locs_total);
-                }
-            } else {
-                const uint32_t rb = __shfl_sync(0xffffffffu, g_rb, j);
-                if (!ok && lane == 0) atomicOr(&B.tot[TOT_FLAGS], OV_RECS);
-                if (lane == 0 && num) {
-                    if (ok) {
-                        out_w[wbase] = item;
-                        out_w[wbase + 1] = num | (1u << 31);
-                        B.rec_woff[rb] = wbase;
-                        B.rec_boff[rb] = bbase;
-                        B.rec_blen[rb] = len;
-                    }
-                    locs_total += num;
+                    locs_total += nwords - 2;
                 }
             }
         }
+        const unsigned ones = __ballot_sync(0xffffffffu, one);
+        S.cb[lane] = cb;
+        S.n[lane] = S.by[lane] = 0;
+        S.p[lane] = WRITE ? wb + 2 : 0u;
+        S.s[lane] = WRITE ? bb : 0u;
+        const uint32_t first = __shfl_sync(0xffffffffu, cb, 0);
+        uint32_t end = __reduce_max_sync(0xffffffffu, cend);
+        if (WRITE && !ones) end = first;
+        uint32_t last = 0, last_j = 32;  // the passing candidate before: its location and item
+        uint32_t run_n = 0, run_by = 0;  // write pass: the group's locations and bytes so far
+        const uint32_t s0 = first & ~15u;
+        uint4 next = make_uint4(0, 0, 0, 0);
+        if (s0 + 16 * lane < end) next = *reinterpret_cast<const uint4 *>(vflag + s0 + 16 * lane);
+        for (uint32_t s = s0; s < end; s += RECORDS_STEP) {
+            const uint4 w = next;
+            const uint32_t c0 = s + 16 * lane;
+            if ((uint64_t)c0 + RECORDS_STEP < end) next = *reinterpret_cast<const uint4 *>(vflag + c0 + RECORDS_STEP);
+            const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+            uint32_t pass = 0, tb = 0; // bit i: flag i
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                // a byte of 1 or 2, and of 2, as one bit each, the four gathered by a multiply
+                const uint32_t t = __vcmpeq4(ww[q], 0x02020202u) & 0x01010101u;
+                const uint32_t h = __vcmpeq4(ww[q], 0x01010101u) & 0x01010101u;
+                tb |= ((t * 0x01020408u) >> 24) << (4 * q);
+                pass |= (((t | h) * 0x01020408u) >> 24) << (4 * q);
+            }
+            if (c0 < first) pass &= 0xffffffffu << min(first - c0, 31u);
+            if (c0 + 16 > end) pass &= c0 < end ? (1u << (end - c0)) - 1u : 0u;
+            const uint32_t np = __popc(pass), incl = warp_scan_incl(np), total = __shfl_sync(0xffffffffu, incl, 31);
+            if (!total) continue;
+            uint32_t at = incl - np;
+            for (; pass; pass &= pass - 1) {
+                const uint32_t bit = __ffs(pass) - 1;
+                S.list[at++] = (uint16_t)(16 * lane + bit | ((tb >> bit & 1u) << 15));
+            }
+            __syncwarp();
+            for (uint32_t i0 = 0; i0 < total; i0 += 32) {
+                const bool valid = i0 + lane < total;
+                const uint32_t e = S.list[valid ? i0 + lane : i0], c = s + (e & 0x7fffu);
+                const uint32_t loc = vloc[c], tl = vtlen[c];
+                uint4 h = make_uint4(0, 0, 0, 0);
+                if (WRITE && valid) h = *reinterpret_cast<const uint4 *>(vcig + (uint64_t)c * SWM_CIGAR_SLOT);
+                uint32_t j = 0; // the last item to start at or before c: those of none start where the next does
+#pragma unroll
+                for (uint32_t half = 16; half; half >>= 1)
+                    if (S.cb[j + half] <= c) j += half;
+                uint32_t ploc = __shfl_up_sync(0xffffffffu, loc, 1), pj = __shfl_up_sync(0xffffffffu, j, 1);
+                if (lane == 0) {
+                    ploc = last;
+                    pj = last_j;
+                }
+                const bool keep = valid && !((e >> 15) && pj == j && ploc == loc); // 475-477
+                if (!WRITE) {
+                    if (valid) {
+                        atomicAdd(&S.p[j], 1u);
+                        atomicAdd(&S.s[j], 2 + tl);
+                    }
+                    if (keep) {
+                        atomicAdd(&S.n[j], 1u);
+                        atomicAdd(&S.by[j], 2 + tl);
+                    }
+                } else {
+                    const uint32_t km = __ballot_sync(0xffffffffu, keep), by = keep ? 2 + tl : 0u;
+                    const uint32_t bincl = warp_scan_incl(by);
+                    const uint32_t rn = run_n + __popc(km & lanemask_lt()), rby = run_by + bincl - by;
+                    if (valid && pj != j) { // the item's first
+                        S.n[j] = rn;
+                        S.by[j] = rby;
+                    }
+                    __syncwarp();
+                    if (keep && (ones >> j & 1u)) {
+                        out_w[S.p[j] + rn - S.n[j]] = loc;
+                        // [NM, len, text]: the slot's first 16 bytes in one load
+                        uint8_t *dst = out_c + (S.s[j] + rby - S.by[j]);
+                        const uint32_t hw[4] = {h.x, h.y, h.z, h.w};
+                        if (tl + 2 <= 16) {
+#pragma unroll
+                            for (uint32_t q = 0; q < 16; q++)
+                                if (q < tl + 2) dst[q] = (uint8_t)(hw[q >> 2] >> (8 * (q & 3)));
+                        } else {
+                            dst[0] = (uint8_t)h.x;
+                            dst[1] = (uint8_t)(h.x >> 8);
+                            const uint8_t *tx = (tl <= SWM_CIGAR_SLOT - 2) ? vcig + (uint64_t)c * SWM_CIGAR_SLOT + 2
+                                                                          : B.arena + B.vr_aoff[c];
+                            for (uint32_t q = 0; q < tl; q++) dst[2 + q] = tx[q];
+                        }
+                    }
+                    run_n += __popc(km);
+                    run_by += __shfl_sync(0xffffffffu, bincl, 31);
+                }
+                const uint32_t end_lane = min(31u, total - i0 - 1);
+                last = __shfl_sync(0xffffffffu, loc, end_lane);
+                last_j = __shfl_sync(0xffffffffu, j, end_lane);
+            }
+            __syncwarp(); // the list is read
+        }
+        __syncwarp();
+        if (mine < nitems) {
+            if (!WRITE) {
+                if (S.p[lane] + 8 <= SWM_MAX_CIGAR && S.s[lane] + 16 * 16 <= SWM_MAX_CIGAR * 16) {
+                    const uint32_t num = S.n[lane];
+                    B.it_nrec[mine] = num ? 1u : 0u;
+                    B.it_nw[mine] = num ? 2 + num : 0u;
+                    B.it_nb[mine] = S.by[lane];
+                } else {
+                    records_seq<false>(B, mine, cap_recs, cap_words, cap_bytes, locs_total);
+                }
+            } else if (nrec > 1) { // flushes: the sequential rules
+                records_seq<true>(B, mine, cap_recs, cap_words, cap_bytes, locs_total);
+            }
+        }
+        __syncwarp();
     }
     if (!WRITE) {
         warp_add_u64(&B.stat[ST_BATCHES], batches);
@@ -4018,7 +4068,7 @@ static int alloc_work(swm_mapper *m) {
     rc |= dmalloc(&B.cand_ub, m->cap_elems);
     rc |= dmalloc(&B.cc_pos, m->cap_cands);
     rc |= dmalloc(&B.cc_item, m->cap_cands);
-    rc |= dmalloc(&B.vr_flag, m->cap_cands);
+    rc |= dmalloc(&B.vr_flag, m->cap_cands + 16); // read 16 at a time
     rc |= dmalloc(&B.vr_loc, m->cap_cands);
     rc |= dmalloc(&B.vr_err, m->cap_cands);
     rc |= dmalloc(&B.vr_mloc, m->cap_cands);

@@ -637,6 +637,35 @@ def test_gpu_batches_of_many_kept_positions(cuda_lib, copies):
         assert m.stats()["candidates"] == ref.stats["candidates"]
 
 
+@pytest.mark.parametrize("nreads", [1, 15, 16, 17, 40])
+@pytest.mark.parametrize("copies", [1, 200, 247, 248, 249, 600])
+def test_gpu_records_around_the_flush_bounds(cuda_lib, copies, nreads):
+    """Reads of a unit of `copies` copies, every fourth of them mutated past the
+    error bound and some by an indel, between reads that map once or not at all:
+    items of one record, of several (256 locations at most each) and of none in
+    groups of 32 items, whole and partial ones, with more than 512 candidates."""
+    rng = np.random.default_rng(67)
+    unit, step = rng.choice(np.frombuffer(b"ACGT", np.uint8), 130), 170
+    total = copies + copies // 3
+    g = genome(total * step + 60_000, 68)
+    for i in range(total):
+        u = unit.copy()
+        if i % 4 == 3:  # 100 bases of it are 20 and more substitutions off, seeds still match
+            at = rng.choice(np.arange(45, 130), 40, replace=False)
+            u[at] = rng.choice(np.frombuffer(b"ACGT", np.uint8), 40)
+        elif i % 4 == 1:
+            u = np.delete(u, 60 + i % 3)
+        g[i * step:i * step + u.size] = u
+    reads, lens, _, _ = synth.reads(g[-50_000:], nreads, 100, 100, 0.03, seed=69)
+    for r in range(0, nreads, 3):
+        reads[r, :100], lens[r] = unit[r % 30:r % 30 + 100], 100
+    reads[1::5] = rng.choice(np.frombuffer(b"ACGT", np.uint8), reads[1::5].shape)
+    _, mix = oracle_index(g)
+    ref = po.map_reads(mix, reads, lens, 5, nthreads=8, cap_records=100_000)
+    m = cuda_lib.Mapper(cuda_lib.Index.build(g), max_reads=nreads)
+    _check(m.map(reads, lens, 5, records_cap=100_000), ref.records(), ref.unmapped)
+
+
 @pytest.mark.parametrize("nreads", [8191, 8192, 9001])
 def test_gpu_uneven_blocks_listed_by_length(cuda_lib, nreads):
     """Blocks of both seed kernels' reads below and from the size at which they
