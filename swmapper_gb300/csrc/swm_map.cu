@@ -2303,12 +2303,55 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS)
     if (lane == 0 && kept_all) atomicAdd(&B.stat[ST_KEPT], kept_all);
 }
 
-// Dense candidate list: item by item, batch by batch, in verification order.
-#define COMPACT_HEAVY 16 // candidates above which an item is copied by its whole warp
+#define COMPACT_BATCHES 128 // batches a warp of k_compact lists at once
 
+struct CompactSmem {
+    uint32_t st[COMPACT_BATCHES];  // first place of the batch in the dense list
+    uint32_t src[COMPACT_BATCHES]; // what to add to a place for its place in cand_ub
+    uint8_t it[COMPACT_BATCHES];   // the batch's item in the group
+    uint32_t b0[32];               // batches of the group before the item's
+};
+
+// The places beg .. end - 1 of the dense list, of the listed batches: a lane each,
+// four in flight. HALF: half the batches listed, a power of two.
+template <uint32_t HALF>
+__device__ __forceinline__ void compact_copy(const MapBufs &B, const CompactSmem &S, uint32_t item0, uint32_t beg,
+                                             uint32_t end) {
+    const uint32_t *__restrict__ ub = B.cand_ub;
+    for (uint32_t i0 = beg; i0 < end; i0 += 128) {
+        uint32_t pos[4], k[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t i = i0 + 32 * u + lane_id();
+            k[u] = 0; // the last batch to start at or before i
+#pragma unroll
+            for (uint32_t half = HALF; half; half >>= 1)
+                if (S.st[k[u] + half] <= i) k[u] += half;
+            if (i < end) pos[u] = ub[S.src[k[u]] + i];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t i = i0 + 32 * u + lane_id();
+            if (i < end) {
+                B.cc_pos[i] = pos[u];
+                B.cc_item[i] = item0 + S.it[k[u]];
+            }
+        }
+    }
+}
+
+// Dense candidate list: item by item, batch by batch, in verification order. The
+// places of a group of 32 items follow each other, so a warp lists the group's
+// batches (first place and where from) and takes its places 128 at a time, whatever
+// items they belong to. Bound by the round trips of a group and the warps in
+// flight; items and their batches one after another, a round trip each,
+// was 294 us for 524,288 reads on 3 Gbp (52 candidates an item), so 180; for 65,536
+// uneven ones 97 and 51; for 4,096 on 1 Gbp 25 and 13.
 __global__ void __launch_bounds__(256) k_compact(MapBufs B, uint64_t cap_chunks, uint64_t cap_elems,
                                                  uint64_t cap_cands) {
     in_order(B);
+    __shared__ CompactSmem smem[8];
+    CompactSmem &S = smem[threadIdx.x >> 5];
     const uint32_t nitems = B.par->nitems;
     if (B.tot[TOT_FLAGS] != 0 || B.tot[TOT_CHUNKS] > cap_chunks || B.tot[TOT_ELEMS] > cap_elems) return;
     const uint32_t lane = lane_id();
@@ -2316,11 +2359,7 @@ __global__ void __launch_bounds__(256) k_compact(MapBufs B, uint64_t cap_chunks,
     for (uint32_t item0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); item0 < nitems;
          item0 += gridDim.x * blockDim.x) {
         const uint32_t item = item0 + lane;
-        // one thread per item: its scalars in one round trip, then its few
-        // candidates batch by batch; items with many candidates are left to
-        // the whole warp below
         uint32_t nb = 0, o0 = 0, nc = 0, sbase = 0, eloff = 0;
-        bool heavy = false;
         if (item < nitems) {
             nb = B.it_nbat[item];
             o0 = B.it_coff[item];
@@ -2331,38 +2370,55 @@ __global__ void __launch_bounds__(256) k_compact(MapBufs B, uint64_t cap_chunks,
                 atomicOr(&B.tot[TOT_FLAGS], OV_CANDS);
                 nb = 0;
             }
-            heavy = nb && nc > COMPACT_HEAVY;
-            if (nb && !heavy) {
-                uint32_t o = o0;
-                for (uint32_t b = 0; b < nb; b++) {
-                    const uint32_t n = nb > 1 ? B.bt_cnt[sbase + b] : nc;
-                    const uint32_t e0 = nb > 1 ? B.bt_e0[sbase + b] : eloff;
-                    for (uint32_t j = 0; j < n; j++) {
-                        B.cc_pos[o + j] = B.cand_ub[e0 + j];
-                        B.cc_item[o + j] = item;
-                    }
-                    o += n;
+            if (nc == 0) nb = 0;
+        }
+        const uint32_t act = __ballot_sync(0xffffffffu, nb != 0);
+        if (!act) continue;
+        uint32_t run = __shfl_sync(0xffffffffu, o0, __ffs(act) - 1);
+        if (!__any_sync(0xffffffffu, nb > 1)) { // a batch each: its size and place are the item's
+            const uint32_t r = __popc(act & lanemask_lt());
+            if (lane >= __popc(act)) S.st[lane] = 0xffffffffu;
+            __syncwarp();
+            if (nb) {
+                S.st[r] = o0;
+                S.src[r] = eloff - o0;
+                S.it[r] = (uint8_t)lane;
+            }
+            __syncwarp();
+            compact_copy<16>(B, S, item0, run, __reduce_max_sync(0xffffffffu, nb ? o0 + nc : 0u));
+        } else {
+            const uint32_t incl = warp_scan_incl(nb), all = __shfl_sync(0xffffffffu, incl, 31);
+            S.b0[lane] = incl - nb;
+            __syncwarp();
+            for (uint32_t t0 = 0; t0 < all; t0 += COMPACT_BATCHES) {
+                uint32_t cnt[COMPACT_BATCHES / 32], e0[COMPACT_BATCHES / 32], j[COMPACT_BATCHES / 32];
+#pragma unroll
+                for (int q = 0; q < COMPACT_BATCHES / 32; q++) {
+                    const uint32_t t = t0 + 32 * q + lane;
+                    j[q] = 0;
+#pragma unroll
+                    for (uint32_t half = 16; half; half >>= 1)
+                        if (S.b0[j[q] + half] <= t) j[q] += half;
+                    const uint32_t slot = __shfl_sync(0xffffffffu, sbase, j[q]) + t - S.b0[j[q]];
+                    const uint32_t el = __shfl_sync(0xffffffffu, eloff, j[q]), b = __shfl_sync(0xffffffffu, nb, j[q]);
+                    cnt[q] = t < all ? B.bt_cnt[slot] : 0u;
+                    e0[q] = t < all && b > 1 ? B.bt_e0[slot] : el; // a single batch starts where its item does
                 }
+                const uint32_t beg = run;
+#pragma unroll
+                for (int q = 0; q < COMPACT_BATCHES / 32; q++) {
+                    const uint32_t ci = warp_scan_incl(cnt[q]), at = run + ci - cnt[q];
+                    S.st[32 * q + lane] = t0 + 32 * q + lane < all ? at : 0xffffffffu;
+                    S.src[32 * q + lane] = e0[q] - at;
+                    S.it[32 * q + lane] = (uint8_t)j[q];
+                    run += __shfl_sync(0xffffffffu, ci, 31);
+                }
+                __syncwarp();
+                compact_copy<COMPACT_BATCHES / 2>(B, S, item0, beg, run);
+                __syncwarp();
             }
         }
-        uint32_t hm = __ballot_sync(0xffffffffu, heavy);
-        while (hm) { // the warp copies each heavy item of the group, lanes over its candidates
-            const uint32_t src = __ffs(hm) - 1;
-            hm &= hm - 1;
-            const uint32_t hnb = __shfl_sync(0xffffffffu, nb, src);
-            const uint32_t hnc = __shfl_sync(0xffffffffu, nc, src), hsb = __shfl_sync(0xffffffffu, sbase, src);
-            const uint32_t hel = __shfl_sync(0xffffffffu, eloff, src);
-            uint32_t o = __shfl_sync(0xffffffffu, o0, src);
-            for (uint32_t b = 0; b < hnb; b++) {
-                const uint32_t n = hnb > 1 ? B.bt_cnt[hsb + b] : hnc;
-                const uint32_t e0 = hnb > 1 ? B.bt_e0[hsb + b] : hel;
-                for (uint32_t j = lane; j < n; j += 32) {
-                    B.cc_pos[o + j] = B.cand_ub[e0 + j];
-                    B.cc_item[o + j] = item0 + src;
-                }
-                o += n;
-            }
-        }
+        __syncwarp();
     }
 }
 

@@ -666,6 +666,27 @@ def test_gpu_records_around_the_flush_bounds(cuda_lib, copies, nreads):
     _check(m.map(reads, lens, 5, records_cap=100_000), ref.records(), ref.unmapped)
 
 
+@pytest.mark.parametrize("e,rmin,rmax", [(2, 60, 100), (5, 150, 250), (8, 200, 250)])
+def test_gpu_dense_list_of_items_of_many_batches(cuda_lib, e, rmin, rmax):
+    """Groups of 32 items that mix items of no, one and many batches, with more
+    batches in a group than a warp lists at once, in whole and partial groups."""
+    rng = np.random.default_rng(73)
+    unit, step, copies = rng.choice(np.frombuffer(b"ACGT", np.uint8), 250), 260, 1500
+    g = genome(copies * step + 60_000, 74)
+    at = np.arange(copies)[:, None] * step + np.arange(250)[None, :]
+    mut = rng.random((copies, 250)) < 0.01
+    g[at] = np.where(mut, rng.choice(np.frombuffer(b"ACGT", np.uint8), (copies, 250)), unit)
+    reads, lens, _, _ = synth.reads(g, 53, rmin, rmax, 0.01, seed=75, stride=250)
+    reads[::4] = rng.choice(np.frombuffer(b"ACGT", np.uint8), reads[::4].shape)
+    mix = po.MapIndex(po.build_index(g))
+    ref = po.map_reads(mix, reads, lens, e, nthreads=8, cap_records=200_000)
+    m = cuda_lib.Mapper(cuda_lib.Index.build(g), max_reads=53)
+    _check(m.map(reads, lens, e, records_cap=200_000), ref.records(), ref.unmapped)
+    st = m.stats()
+    assert (st["batches"], st["candidates"]) == (ref.stats["batches"], ref.stats["candidates"])
+    assert st["batches"] > 53
+
+
 @pytest.mark.parametrize("nreads", [8191, 8192, 9001])
 def test_gpu_uneven_blocks_listed_by_length(cuda_lib, nreads):
     """Blocks of both seed kernels' reads below and from the size at which they
