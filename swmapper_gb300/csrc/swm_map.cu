@@ -71,21 +71,19 @@ enum {
     TOT_N
 };
 
-// Next CAND_TAKE items of a warp in the candidate stage (head *q): items differ
-// by a factor of a hundred in work (kept positions, batches), so warps take
-// them from a queue in small groups instead of a fixed stride.
-#define CAND_TAKE 4
-__device__ __forceinline__ uint32_t warp_take_items(uint32_t *q) {
-    uint32_t b = 0;
-    if ((threadIdx.x & 31) == 0) b = atomicAdd(q, (uint32_t)CAND_TAKE);
-    return __shfl_sync(0xffffffffu, b, 0);
-}
+// Items a warp of the candidate stage takes from the queue at once: they differ by
+// a factor of a hundred in work (kept positions, batches), so small groups instead
+// of a fixed stride. Large blocks take 8: after some histories of allocations in
+// the process the requests to the queue head are slow, and 524,288 reads on 3 Gbp
+// took 1,480 or 1,780 us with 4, 1,500 either way with 8 (1,530 with 16; on
+// 100 Mbp 541, 545 and 567).
+#define CAND_TAKE(nitems) ((nitems) >= 1u << 18 ? 8u : 4u)
 
-// Next 32 work units of a warp from a device work queue (head *q): every lane
+// Next units (32) of a warp from a device work queue (head *q): every lane
 // gets the same base; the warp is done when it reaches n.
-__device__ __forceinline__ uint32_t warp_take(uint32_t *q) {
+__device__ __forceinline__ uint32_t warp_take(uint32_t *q, uint32_t units = 32) {
     uint32_t b = 0;
-    if ((threadIdx.x & 31) == 0) b = atomicAdd(q, 32u);
+    if ((threadIdx.x & 31) == 0) b = atomicAdd(q, units);
     return __shfl_sync(0xffffffffu, b, 0);
 }
 
@@ -1959,11 +1957,12 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS) k_cand(const
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
     CandSmem &S = sm_all[wib];
     unsigned long long kept_all = 0; // this warp's kept positions, added to the block's count once
-    for (uint32_t g0 = warp_take_items(&B.tot[TOT_CQ]), gi = 0; g0 < nitems;) {
+    const uint32_t take = CAND_TAKE(nitems);
+    for (uint32_t g0 = warp_take(&B.tot[TOT_CQ], take), gi = 0; g0 < nitems;) {
         const uint32_t item = g0 + gi;
-        if (++gi == CAND_TAKE || item + 1 >= nitems) {
+        if (++gi == take || item + 1 >= nitems) {
             gi = 0;
-            g0 = warp_take_items(&B.tot[TOT_CQ]);
+            g0 = warp_take(&B.tot[TOT_CQ], take);
         }
         if (item >= nitems) break;
         const uint32_t nb = B.it_nbat[item];
@@ -2153,11 +2152,12 @@ __global__ void __launch_bounds__(CAND_WARPS * 32, CAND_MIN_BLOCKS)
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
     CandTabSmem &S = sm_all[wib];
     unsigned long long kept_all = 0; // this warp's kept positions, added to the block's count once
-    for (uint32_t g0 = warp_take_items(&B.tot[TOT_CQ]), gi = 0; g0 < nitems;) {
+    const uint32_t take = CAND_TAKE(nitems);
+    for (uint32_t g0 = warp_take(&B.tot[TOT_CQ], take), gi = 0; g0 < nitems;) {
         const uint32_t item = g0 + gi;
-        if (++gi == CAND_TAKE || item + 1 >= nitems) {
+        if (++gi == take || item + 1 >= nitems) {
             gi = 0;
-            g0 = warp_take_items(&B.tot[TOT_CQ]);
+            g0 = warp_take(&B.tot[TOT_CQ], take);
         }
         if (item >= nitems) break;
         const uint32_t nb = B.it_nbat[item];
@@ -2807,6 +2807,7 @@ __global__ void __launch_bounds__(128, VERIFY_BLOCKS_PER_SM)
     const uint64_t nc_all = B.tot[TOT_CANDS];
     const uint32_t n = (uint32_t)(nc_all < cap_cands ? nc_all : cap_cands);
     const uint32_t lane = lane_id();
+    const uint32_t *__restrict__ lens = B.par->lens;
     // per-lane counts fit 32 bits: a lane runs at most ceil(cap_cands / lanes of
     // the grid) candidates of at most 254 x 31 cells
     uint32_t cells = 0, nsteps = 0;
@@ -2825,13 +2826,25 @@ __global__ void __launch_bounds__(128, VERIFY_BLOCKS_PER_SM)
     // is taken, so the ring never overwrites a slot not yet handed out.
     __shared__ uint4 ring_s[4][64]; // 128 threads: 4 warps
     uint4 *ring = ring_s[threadIdx.x >> 5];
+    // candidates a warp takes from the queue at once (four ranges while every warp
+    // takes at least 16 times): requests to the one queue head are what a large
+    // block's warps wait for otherwise, by as much as the process's history of
+    // allocations has it -- 524,288 reads on 3 Gbp 3,750 us after one and 5,240 after
+    // another with single ranges, 3,775 after either with four.
+    const uint32_t take = n / (16 * 128) >= gridDim.x * (blockDim.x >> 5) ? 128 : 32;
+    uint32_t range = 0, range_end = 0;
     uint32_t rh = 0, rt = 0; // slots handed out / staged (counts; slot = count & 63)
     for (;;) {
         const unsigned need = __ballot_sync(0xffffffffu, !act);
         if (need) {
             const uint32_t k = __popc(need), r = __popc(need & lanemask_lt());
             while (rt - rh < k && !drained) {
-                const uint32_t t = warp_take(&B.tot[TOT_VQ]);
+                if (range == range_end) {
+                    range = warp_take(&B.tot[TOT_VQ], take);
+                    range_end = range + take;
+                }
+                const uint32_t t = range;
+                range += 32;
                 if (t >= n) {
                     drained = true;
                     break;
@@ -2841,7 +2854,7 @@ __global__ void __launch_bounds__(128, VERIFY_BLOCKS_PER_SM)
                 uint4 rec = make_uint4(0u, 0u, 0u, 0u);
                 if (cj < n) {
                     const uint32_t item = B.cc_item[cj], p = B.cc_pos[cj];
-                    const uint32_t L = B.par->lens[item >> 1], e = B.it_e[item];
+                    const uint32_t L = lens[item >> 1], e = B.it_e[item];
                     uint32_t rl;
                     const uint32_t w0 = window_start(p, L, e, ref_length, &rl);
                     const int lh = (int)rl - (int)L; // last_high: cells 0 .. lh of the final scan
