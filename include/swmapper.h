@@ -100,10 +100,11 @@ int swm_hash_offset_noalloc(const uint32_t *d_hash_count, uint32_t *d_hash_offse
  * index arrays; the files are unchanged). For k = 12 the first mapper made on
  * an index whose buckets average 8 or more entries (a genome of about 540 Mbp
  * or more) builds a candidate table when the device has room for it: the
- * entries of every bucket grouped, for each seed shift, by the 6 flank bits
- * long_seeds_filter compares (mapper_cpe.c:2090-2123), behind a directly
- * indexed table of 2^32 + 1 offsets (about 17 GiB, plus 16 bytes per index
- * entry). The candidate stage then reads only the entries the filter keeps
+ * entries of every bucket grouped by the 6 flank bits long_seeds_filter
+ * compares for each seed shift (mapper_cpe.c:2090-2123), a 12-mer with its flank
+ * bits of one shift being a 15-mer: groups in the order of 15-mer and shift,
+ * behind a directly indexed table of 2^32 + 1 offsets (about 17 GiB, plus 16
+ * bytes per index entry). The candidate stage then reads only the entries the filter keeps
  * instead of every entry of the fetched buckets; results are identical
  * either way. enable = 0 drops the table and keeps it from being built again
  * (mappers fall back to filtering every entry; call it with no block in

@@ -8,24 +8,28 @@
 //
 //   k_seed12   thread / item   read encodings, seed lookups, long-seed order,
 //   (k_seed)                   flank codes            (mapper_cpe.c:1246-1401,
-//                                                      2451-2499)
-//   scan       chunk and element offsets per item
-//   k_plan*    lane or warp /  the fetch schedule: 32-position chunks,
-//              item            heap-ordered refills, batch boundaries
-//                                                     (mapper_cpe.c:2124-2419)
+//                                                      2451-2499); k_seed for k
+//                              outside 10 .. 14
+//   k_scan_items               chunk and element offsets per item (one pass,
+//                              decoupled look-back)
+//   k_plan_list, k_plan*       the fetch schedule: 32-position chunks,
+//              lane or warp /  heap-ordered refills, batch boundaries
+//              item                                   (mapper_cpe.c:2124-2419)
 //   k_cand /   warp / item     gather + position adjust + flank filter (or
 //   k_cand_table               the candidate table's survivors) + per-batch
-//                              sort-unique            (mapper_cpe.c:1893-2123)
-//   scan       candidate offsets
-//   k_compact  thread or warp  dense candidate list
-//              / item
+//   + k_cand_heavy  block /    sort-unique; large batches
+//              batch                                  (mapper_cpe.c:1893-2123)
+//   k_scan_items               candidate offsets
+//   k_compact  warp / 32 items dense candidate list
 //   k_verify_stream   lane /   window, banded Myers 16 bases at a time with a
 //   + k_verify_finish  cand    stop bound; last bases, final scan, Hamming
 //   (or k_verify, two passes)  check               (mapper_cpe.c:229-660,
 //                                                      1403-1435,1509-1586)
-//   k_traceback thread / cand  traceback + CIGAR text (align_reads, mapper_cpe.c:229-517)
-//   k_records  thread or warp  groups of 8, record flushes, dedup, primary
-//              / item          flag (count pass, scan, write pass)
+//   k_traceback thread / cand  checkpoints, traceback + CIGAR text (align_reads,
+//                              mapper_cpe.c:229-517)
+//   k_records  warp /          groups of 8, record flushes, dedup, primary
+//              32 items        flag (count pass, scan that also lists the
+//                              unmapped reads, write pass)
 //                                                     (mapper_cpe.c:1437-1507,
 //                                                      1753-1860)
 //
@@ -3309,9 +3313,9 @@ __global__ void __launch_bounds__(128, 8) k_verify_finish(const uint32_t *__rest
 // and D0 contains it, so a step whose bases agree is always an M step: runs
 // of agreeing bases along the diagonal are taken 32 at a time from the bit
 // planes. Only the other steps (errors, or walks outside the band) need D0 /
-// HP, which are recomputed from the (VP, VN) checkpoint k_verify left at the
-// start of their 32-base block. The run-length route stays in shared memory;
-// a walk with more than TB_ROUTE runs is handed to k_traceback_slow.
+// HP, which are recomputed from the (VP, VN) checkpoint left at the
+// start of their 16-base half block. The run-length route stays in shared memory;
+// a walk with more than TB_ROUTE runs is left to traceback_slow.
 #define TB_THREADS 64
 #define TB_ROUTE 48
 
