@@ -2349,8 +2349,9 @@ __device__ __forceinline__ void compact_copy(const MapBufs &B, const CompactSmem
 // batches (first place and where from) and takes its places 128 at a time, whatever
 // items they belong to. Bound by the round trips of a group and the warps in
 // flight; items and their batches one after another, a round trip each,
-// was 294 us for 524,288 reads on 3 Gbp (52 candidates an item), so 180; for 65,536
-// uneven ones 97 and 51; for 4,096 on 1 Gbp 25 and 13.
+// was 294 us for 524,288 reads on 3 Gbp (52 candidates an item), so 200; for 65,536
+// uneven ones 97 and 52; for 4,096 on 1 Gbp 25 and 13. A grid of the resident 6
+// blocks an SM instead of 8 was equal, 32 registers for 8 slower (212).
 __global__ void __launch_bounds__(256) k_compact(MapBufs B, uint64_t cap_chunks, uint64_t cap_elems,
                                                  uint64_t cap_cands) {
     in_order(B);
